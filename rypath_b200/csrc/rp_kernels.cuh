@@ -604,7 +604,8 @@ __global__ void __launch_bounds__(Block, 512 / Block) k_nee(const __grid_constan
                         const u32 block = 133 + cnt - 2;
                         const float u0 = sample_uniform(p, draw_word0(s, p, ident.x, ident.y, ident.z, index, block));
                         // sample_li (shaders/packet_transport.h:470-553)
-                        const Selected choice = light_sample(s, cp.position, cp.shading_normal, u0);
+                        float selected_pmf = 0; // light_pmf of the selected light
+                        const Selected choice = light_sample<true>(s, cp.position, cp.shading_normal, u0, selected_pmf);
                         float u1 = 0, u2 = 0;
                         const bool env_image = Img && s.img.env_image != kNone && choice.light == s.environment_light;
                         if (choice.pmf > 0 && (choice.light < s.emitter_count || env_image)) {
@@ -613,7 +614,7 @@ __global__ void __launch_bounds__(Block, 512 / Block) k_nee(const __grid_constan
                             u2 = sample_uniform(p, w.z);
                         }
                         V4 lbeta = v4(0);
-                        float spdf = 0;
+                        float spdf = 0, geometry_pdf = 0; // geometry_pdf: light_geometry_pdf of the sampled point
                         bool li_ok = true, delta_light = false;
                         SurfacePoint lp;
                         lp.position = lp.error = lp.geometric_normal = lp.shading_normal = v3(0, 0, 0);
@@ -626,6 +627,7 @@ __global__ void __launch_bounds__(Block, 512 / Block) k_nee(const __grid_constan
                                 if (!light_geometry_sample(s, sel, cp.position, cp.shading_normal, u1, u2, lp, spdf)) {
                                     li_ok = false;
                                 } else {
+                                    geometry_pdf = spdf;
                                     spdf *= choice.pmf;
                                     const V3 dl = lp.position - cp.position;
                                     const float d2 = dot(dl, dl);
@@ -696,12 +698,12 @@ __global__ void __launch_bounds__(Block, 512 / Block) k_nee(const __grid_constan
                                     V4 contribution = value;
                                     bool weight_ok = true;
                                     if (!delta_light) {
-                                        const float sel_pmf = light_pmf(s, cp.position, cp.shading_normal, sel);
+                                        const float sel_pmf =
+                                            selected_pmf >= 0 ? selected_pmf : light_pmf(s, cp.position, cp.shading_normal, sel);
                                         const float lpdf =
                                             env_image ? environment_image_pdf(s.img, direction, true) * sel_pmf
-                                            : nonzero3(lp.geometric_normal)
-                                                ? sel_pmf * light_geometry_pdf(s, sel, cp.position, cp.shading_normal, lp)
-                                                : 0.0f;
+                                            : nonzero3(lp.geometric_normal) ? sel_pmf * geometry_pdf
+                                                                            : 0.0f;
                                         bool ok;
                                         const V4 bsdf_pdf = represented_pdf<F == 3 ? 0 : F>(
                                             cbsdf, cp.shading_normal, cp.position, latest.position, env_image,

@@ -877,25 +877,49 @@ RP_DEV bool prepare_roughness(float u, float v, bool remap, bool force_smooth, G
     }
     return true;
 }
-// shaders/conductor.h:120-138
-RP_DEV Eval conductor_evaluate(float eta, float k, const Ggx &g, V3 wo, V3 wi) {
-    if (!finite3(wo) || !finite3(wi))
-        return {0, 0, false};
-    if (g.smooth || wo.z == 0 || wi.z == 0 || ((wo.z > 0) != (wi.z > 0)))
-        return {0, 0, true};
+// shaders/conductor.h:120-138, split into the part that every wavelength of a hero packet
+// shares (half vector, masking, distribution, density) and the lane's Fresnel.  Evaluated per
+// lane as a whole, the shared part (18 divisions and 4 square roots) ran four times.
+struct ConductorShared {
+    float cosine, d, denominator, pdf; // |wo . m|, distribution, value's divisor, density
+    bool zero, valid, finite;          // no reflection; the half vector exists; lambda terms and density
+};
+RP_DEV ConductorShared conductor_shared(const Ggx &g, V3 wo, V3 wi) {
+    ConductorShared c{0, 0, 0, 0, false, true, true};
+    if (!finite3(wo) || !finite3(wi)) {
+        c.valid = false;
+        return c;
+    }
+    if (g.smooth || wo.z == 0 || wi.z == 0 || ((wo.z > 0) != (wi.z > 0))) {
+        c.zero = true;
+        return c;
+    }
     V3 m;
-    if (!unit(wo + wi, m))
+    if (!unit(wo + wi, m)) {
+        c.valid = false;
+        return c;
+    }
+    c.cosine = fabsf(dot(wo, m));
+    const float lo = ggx_lambda(g.alpha_x, g.alpha_y, wo), li = ggx_lambda(g.alpha_x, g.alpha_y, wi);
+    c.d = ggx_distribution(g.alpha_x, g.alpha_y, m);
+    c.denominator = 4 * fabsf(wo.z) * fabsf(wi.z) * (1 + lo + li);
+    c.pdf = c.d / (4 * fabsf(wo.z) * (1 + lo));
+    c.finite = isfinite(lo) && isfinite(li) && isfinite(c.d) && isfinite(c.pdf) && c.pdf >= 0;
+    return c;
+}
+RP_DEV Eval conductor_lane(const ConductorShared &c, float eta, float k) {
+    if (!c.valid)
         return {0, 0, false};
+    if (c.zero)
+        return {0, 0, true};
     float f;
-    if (!conductor_fresnel(fabsf(dot(wo, m)), eta, k, f))
+    if (!conductor_fresnel(c.cosine, eta, k, f))
         return {0, 0, false};
-    const float lo = ggx_lambda(g.alpha_x, g.alpha_y, wo), li = ggx_lambda(g.alpha_x, g.alpha_y, wi),
-                d = ggx_distribution(g.alpha_x, g.alpha_y, m);
-    const float value = d * f / (4 * fabsf(wo.z) * fabsf(wi.z) * (1 + lo + li));
-    const float pdf = d / (4 * fabsf(wo.z) * (1 + lo));
-    const bool valid = isfinite(lo) && isfinite(li) && isfinite(d) && isfinite(value) && isfinite(pdf) &&
-                       value >= 0 && pdf >= 0;
-    return {value, pdf, valid};
+    const float value = c.d * f / c.denominator;
+    return {value, c.pdf, c.finite && isfinite(value) && value >= 0};
+}
+RP_DEV Eval conductor_evaluate(float eta, float k, const Ggx &g, V3 wo, V3 wi) {
+    return conductor_lane(conductor_shared(g, wo, wi), eta, k);
 }
 // Visible-normal sampling: shaders/conductor.h:157-185, dielectric.h:160-188
 RP_DEV bool ggx_visible_normal(float ax, float ay, V3 wo, float ux, float uy, V3 &m) {
@@ -1005,11 +1029,21 @@ RP_DEV bool dielectric_optics(float cosine, float eta, float &F, float &etap, fl
     F = .5f * (rp * rp + rs * rs);
     return isfinite(ct) && isfinite(F) && F >= 0 && F <= 1;
 }
-// shaders/dielectric.h:76-126
-RP_DEV Eval dielectric_evaluate(float eta, const Ggx &g, V3 wo, V3 wi) {
+// The masking terms that every lane of a rough dielectric shares (its half vector and
+// distribution depend on the lane's eta).
+struct DielectricShared {
+    float lo, li;
+};
+RP_DEV DielectricShared dielectric_shared(const Ggx &g, V3 wo, V3 wi) {
+    if (g.smooth || wo.z == 0 || wi.z == 0)
+        return {0, 0};
+    return {ggx_lambda(g.alpha_x, g.alpha_y, wo), ggx_lambda(g.alpha_x, g.alpha_y, wi)};
+}
+// shaders/dielectric.h:76-126; smooth: no rough lobe (a smooth surface, or eta 1)
+RP_DEV Eval dielectric_lane(const DielectricShared &sh, float eta, const Ggx &g, bool smooth, V3 wo, V3 wi) {
     if (!finite3(wo) || !finite3(wi))
         return {0, 0, false};
-    if (g.smooth || wo.z == 0 || wi.z == 0)
+    if (smooth || wo.z == 0 || wi.z == 0)
         return {0, 0, true};
     const bool reflection = (wo.z > 0) == (wi.z > 0);
     const bool entering = wo.z > 0;
@@ -1028,7 +1062,7 @@ RP_DEV Eval dielectric_evaluate(float eta, const Ggx &g, V3 wo, V3 wi) {
     bool tir;
     if (!dielectric_optics(co, eta, F, ep, ct, tir))
         return {0, 0, false};
-    const float lo = ggx_lambda(g.alpha_x, g.alpha_y, wo), li = ggx_lambda(g.alpha_x, g.alpha_y, wi);
+    const float lo = sh.lo, li = sh.li;
     const float d = ggx_distribution(g.alpha_x, g.alpha_y, m);
     if (!isfinite(lo) || !isfinite(li) || !isfinite(d))
         return {0, 0, false};
@@ -1049,10 +1083,41 @@ RP_DEV Eval dielectric_evaluate(float eta, const Ggx &g, V3 wo, V3 wi) {
             isfinite(lo) && isfinite(li) && isfinite(d) && isfinite(value) && isfinite(pdf) && value >= 0 &&
                 pdf >= 0};
 }
+RP_DEV Eval dielectric_evaluate(float eta, const Ggx &g, V3 wo, V3 wi) {
+    return dielectric_lane(dielectric_shared(g, wo, wi), eta, g, g.smooth, wo, wi);
+}
 // shaders/dielectric.h:129-133
 RP_DEV float refraction_coefficient(float eta, float co, float ct) {
     const float c = fabsf(co);
     return co < 0 ? ((eta - 1) * (eta + 1)) / (eta * c + ct) : (((1 - eta) * (1 + eta)) / eta) / (c + eta * ct);
+}
+// The reflected or refracted direction about microfacet m (co = wo . m; ct, tir from
+// dielectric_optics); false for a refraction under total internal reflection.
+RP_DEV bool dielectric_direction(float eta, V3 wo, V3 m, float co, float ct, bool tir, bool reflection, V3 &wi) {
+    if (reflection) {
+        wi = -wo + 2 * co * m;
+        return true;
+    }
+    if (tir)
+        return false;
+    const float coefficient = eta == 1 ? 0 : refraction_coefficient(eta, co, ct);
+    wi = (co < 0 ? (-eta) * wo : (-wo) / eta) + coefficient * (co < 0 ? -m : m);
+    return true;
+}
+// dielectric_sample of a smooth surface on a chosen side, given its optics
+RP_DEV BSample smooth_dielectric(float eta, V3 wo, V3 m, float co, float F, float ct, bool tir, bool reflection) {
+    BSample s{{0, 0, 0}, 0, 0, true, false, true};
+    if (!dielectric_direction(eta, wo, m, co, ct, tir, reflection, s.wi) || !finite3(s.wi)) {
+        s.valid = false;
+        return s;
+    }
+    if (s.wi.z == 0 || (((s.wi.z > 0) == (wo.z > 0)) != reflection))
+        return s;
+    s.pdf = reflection ? F : 1 - F;
+    s.weight = reflection ? 1 : (co < 0 ? eta * eta : 1 / (eta * eta));
+    s.valid = isfinite(s.pdf) && s.pdf > 0 && isfinite(s.weight) && s.weight > 0;
+    s.accepted = s.valid;
+    return s;
 }
 // shaders/dielectric.h:134-227
 RP_DEV BSample dielectric_sample(float eta, const Ggx &g, V3 wo, float uc, float ux, float uy, float &sampled_eta) {
@@ -1078,27 +1143,16 @@ RP_DEV BSample dielectric_sample(float eta, const Ggx &g, V3 wo, float uc, float
         return s;
     }
     const bool reflection = uc < F;
-    if (reflection)
-        s.wi = -wo + 2 * co * m;
-    else {
-        if (tir) {
+    if (g.smooth) {
+        s = smooth_dielectric(eta, wo, m, co, F, ct, tir, reflection);
+    } else {
+        if (!dielectric_direction(eta, wo, m, co, ct, tir, reflection, s.wi) || !finite3(s.wi)) {
             s.valid = false;
             return s;
         }
-        const float coefficient = eta == 1 ? 0 : refraction_coefficient(eta, co, ct);
-        s.wi = (co < 0 ? (-eta) * wo : (-wo) / eta) + coefficient * (co < 0 ? -m : m);
-    }
-    if (!finite3(s.wi)) {
-        s.valid = false;
-        return s;
-    }
-    if (s.wi.z == 0 || (((s.wi.z > 0) == (wo.z > 0)) != reflection))
-        return s;
-    const float scale = reflection ? 1 : (co < 0 ? eta * eta : 1 / (eta * eta));
-    if (g.smooth) {
-        s.pdf = reflection ? F : 1 - F;
-        s.weight = scale;
-    } else {
+        if (s.wi.z == 0 || (((s.wi.z > 0) == (wo.z > 0)) != reflection))
+            return s;
+        const float scale = reflection ? 1 : (co < 0 ? eta * eta : 1 / (eta * eta));
         const float lo = ggx_lambda(g.alpha_x, g.alpha_y, wo), li = ggx_lambda(g.alpha_x, g.alpha_y, s.wi);
         const float d = ggx_distribution(g.alpha_x, g.alpha_y, m);
         if (!isfinite(lo) || !isfinite(li) || !isfinite(d)) {
@@ -1114,10 +1168,10 @@ RP_DEV BSample dielectric_sample(float eta, const Ggx &g, V3 wo, float uc, float
             s.pdf = d * fabsf(co) * ct * (1 - F) / (fabsf(wo.z) * (1 + lo) * den * den);
         }
         s.weight = scale * (1 + lo) / (1 + lo + li);
-        s.valid = isfinite(lo) && isfinite(li) && isfinite(d);
+        s.valid = isfinite(lo) && isfinite(li) && isfinite(d) && isfinite(s.pdf) && s.pdf > 0 && isfinite(s.weight) &&
+                  s.weight > 0;
+        s.accepted = s.valid;
     }
-    s.valid = s.valid && isfinite(s.pdf) && s.pdf > 0 && isfinite(s.weight) && s.weight > 0;
-    s.accepted = s.valid;
     if (s.accepted && !reflection)
         sampled_eta = ep;
     return s;
@@ -1146,18 +1200,6 @@ RP_DEV bool hero_connectible(const HeroBsdf &p) {
 }
 // One wavelength of a family-K BSDF; a dielectric lane with eta == 1 is smooth, as
 // rypath_dielectric::prepare makes it (shaders/dielectric.h:19).
-template <int K> RP_DEV Eval lane_evaluate_k(const HeroBsdf &p, int k, V3 wo, V3 wi) {
-    if constexpr (K == 0) {
-        return diffuse_evaluate(p.param[k], wo, wi);
-    } else if constexpr (K == 1) {
-        return conductor_evaluate(p.param[k], p.k[k], p.g, wo, wi);
-    } else {
-        Ggx g = p.g;
-        if (p.param[k] == 1)
-            g.smooth = true;
-        return dielectric_evaluate(p.param[k], g, wo, wi);
-    }
-}
 template <int K> RP_DEV BSample lane_sample_k(const HeroBsdf &p, int k, V3 wo, float uc, float ux, float uy, float &eta) {
     eta = 1;
     if constexpr (K == 0) {
@@ -1171,14 +1213,17 @@ template <int K> RP_DEV BSample lane_sample_k(const HeroBsdf &p, int k, V3 wo, f
         return dielectric_sample(p.param[k], g, wo, uc, ux, uy, eta);
     }
 }
-RP_DEV Eval lane_evaluate(const HeroBsdf &p, int k, V3 wo, V3 wi) {
-    return p.kind == 0 ? lane_evaluate_k<0>(p, k, wo, wi)
-                       : (p.kind == 1 ? lane_evaluate_k<1>(p, k, wo, wi) : lane_evaluate_k<2>(p, k, wo, wi));
-}
 RP_DEV BSample lane_sample(const HeroBsdf &p, int k, V3 wo, float uc, float ux, float uy, float &eta) {
     return p.kind == 0 ? lane_sample_k<0>(p, k, wo, uc, ux, uy, eta)
                        : (p.kind == 1 ? lane_sample_k<1>(p, k, wo, uc, ux, uy, eta)
                                       : lane_sample_k<2>(p, k, wo, uc, ux, uy, eta));
+}
+RP_DEV Eval lane_evaluate(const HeroBsdf &p, int k, V3 wo, V3 wi) {
+    if (p.kind == 0)
+        return diffuse_evaluate(p.param[k], wo, wi);
+    if (p.kind == 1)
+        return conductor_evaluate(p.param[k], p.k[k], p.g, wo, wi);
+    return dielectric_lane(dielectric_shared(p.g, wo, wi), p.param[k], p.g, p.g.smooth || p.param[k] == 1, wo, wi);
 }
 struct HeroEval {
     V4 f, pdf;
@@ -1191,11 +1236,23 @@ template <int K> __device__ __noinline__ HeroEval hero_evaluate_k(const HeroBsdf
     if (!(p.active_mask & 1u) || (p.active_mask & ~15u) || !finite3(wo) || !finite3(wi))
         return out;
     out.valid = true;
+    ConductorShared cs;
+    DielectricShared ds;
+    if constexpr (K == 1)
+        cs = conductor_shared(p.g, wo, wi);
+    if constexpr (K == 2)
+        ds = dielectric_shared(p.g, wo, wi);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         if (!(p.active_mask & (1u << k)))
             continue;
-        const Eval e = lane_evaluate_k<K>(p, k, wo, wi);
+        Eval e;
+        if constexpr (K == 0)
+            e = diffuse_evaluate(p.param[k], wo, wi);
+        else if constexpr (K == 1)
+            e = conductor_lane(cs, p.param[k], p.k[k]);
+        else
+            e = dielectric_lane(ds, p.param[k], p.g, p.g.smooth || p.param[k] == 1, wo, wi);
         out.f.v[k] = e.f;
         out.pdf.v[k] = e.pdf;
         out.valid = out.valid && e.valid;
@@ -1242,17 +1299,16 @@ RP_DEV bool dirac_lane(const HeroBsdf &p, int k, V3 wo, V3 wi, float ux, float u
         const float probability = transmission ? 1 - F : F;
         if (probability == 0)
             return true;
-        float sampled_eta;
-        Ggx g = p.g;
-        g.smooth = true;
-        const BSample c = dielectric_sample(p.param[k], g, wo, transmission ? F : 0.f, ux, uy, sampled_eta);
+        // the smooth lobe sampled at this lane's eta, whose optics are known (dielectric_sample
+        // at uc = F or 0 takes the same side)
+        const BSample c = smooth_dielectric(p.param[k], wo, v3(0, 0, 1), wo.z, F, ct, tir, !transmission);
         if (!c.valid)
             return false;
         if (!(c.pdf > 0) || !eq3(c.wi, wi))
             return true;
         pdf = c.pdf;
         mass = c.weight * pdf;
-        eta = sampled_eta;
+        eta = c.accepted && transmission ? ep : 1;
         return isfinite(mass) && mass >= 0;
     }
     return true;

@@ -497,26 +497,34 @@ struct Selected {
     u32 light;
     float pmf;
 };
-// :43-95
-__device__ __noinline__ Selected light_sample(const DeviceScene &s, V3 position, V3 normal, float u) {
+// Levels of the light tree whose branch ratios a light sample keeps for its own density.
+constexpr u32 kRatioLevels = 16;
+// :43-95.  Density: `density` is light_pmf of the selected light, from the importances that the
+// descent computed (light_pmf multiplies the same ratios from the leaf up; a leaf deeper than
+// kRatioLevels leaves it to light_pmf, density -1).
+template <bool Density>
+__device__ __noinline__ Selected light_sample(const DeviceScene &s, V3 position, V3 normal, float u, float &density) {
     const u32 count = s.light_count;
     if (!count)
         return {kNone, 0};
     u = fminf(fmaxf(u, 0.f), kOneMinusEps);
     if (s.light_sampler == 2) {
         const u32 id = min(u32(u * count), count - 1);
+        density = 1.f / count;
         return {id, 1.f / count};
     }
     if (s.light_sampler == 1) {
         const float v = u * count;
         const u32 i = min(u32(v), count - 1);
         const u32 id = v - i < s.light_alias[i].threshold ? i : s.light_alias[i].alias;
+        density = s.light_alias[id].pmf;
         return {id, s.light_alias[id].pmf};
     }
     const u32 ninf = s.infinite_count, nodes = s.light_node_count;
     const float infinite = float(ninf) / float(ninf + (nodes ? 1 : 0));
     if (u < infinite) {
         const u32 i = min(u32((u / infinite) * ninf), ninf - 1);
+        density = 1.f / float(ninf + (nodes ? 1 : 0));
         return {s.infinite_lights[i], 1.f / float(ninf + (nodes ? 1 : 0))};
     }
     if (!nodes)
@@ -525,11 +533,18 @@ __device__ __noinline__ Selected light_sample(const DeviceScene &s, V3 position,
     float pmf = 1 - infinite;
     u32 i = 0;
     float reached = 0; // importance of node i, once a parent has computed it
+    float ratio[Density ? kRatioLevels : 1];
     for (u32 steps = 0; steps < nodes; ++steps) {
         const DLightBounds &node = s.light_nodes[i];
         if (node.light != kNone) {
             if ((steps == 0 ? light_importance(node, position, normal) : reached) <= 0)
                 return {kNone, 0};
+            if (Density) {
+                density = steps <= kRatioLevels ? 1.f - infinite : -1.f;
+                if (steps <= kRatioLevels)
+                    for (u32 k = steps; k-- > 0;)
+                        density *= ratio[k];
+            }
             return {node.light, pmf};
         }
         const float a = light_importance(s.light_nodes[i + 1], position, normal),
@@ -537,7 +552,10 @@ __device__ __noinline__ Selected light_sample(const DeviceScene &s, V3 position,
         if (!(sum > 0))
             return {kNone, 0};
         const float q = a / sum;
-        if (u < q) {
+        const bool first = u < q;
+        if (Density && steps < kRatioLevels)
+            ratio[steps] = first ? q : b / sum;
+        if (first) {
             pmf *= q;
             u = fminf(u / q, kOneMinusEps);
             i++;
@@ -550,6 +568,10 @@ __device__ __noinline__ Selected light_sample(const DeviceScene &s, V3 position,
         }
     }
     return {kNone, 0};
+}
+RP_DEV Selected light_sample(const DeviceScene &s, V3 position, V3 normal, float u) {
+    float density;
+    return light_sample<false>(s, position, normal, u, density);
 }
 // :96-126
 __device__ __noinline__ float light_pmf(const DeviceScene &s, V3 position, V3 normal, u32 id) {
@@ -595,11 +617,6 @@ RP_DEV float sph_angle(V3 a, V3 b) {
 RP_DEV float sph_triangle_area(V3 a, V3 b, V3 c) {
     return fabsf(2 * atan2f(dot(a, cross(b, c)), 1 + dot(a, b) + dot(a, c) + dot(b, c)));
 }
-RP_DEV float triangle_solid_angle(V3 p0, V3 p1, V3 p2, V3 r) {
-    if (!nonzero_len(p0 - r) || !nonzero_len(p1 - r) || !nonzero_len(p2 - r))
-        return 0;
-    return sph_triangle_area(unitv(p0 - r), unitv(p1 - r), unitv(p2 - r));
-}
 struct W4 {
     float a, b, c, d;
 };
@@ -613,28 +630,49 @@ RP_DEV float linear_sample(float u, float a, float b) {
         return 0;
     return fminf(kOneMinusEps, u * (a + b) / (a + sqrtf((1 - u) * a * a + u * b * b)));
 }
-RP_DEV float bilinear_pdf(float ux, float uy, W4 weights) {
+// w: normalised weights
+RP_DEV float bilinear_pdf(float ux, float uy, W4 w) {
     if (ux < 0 || ux > 1 || uy < 0 || uy > 1)
         return 0;
-    const W4 w = normalized_weights(weights);
     return 4 * ((1 - ux) * (1 - uy) * w.a + ux * (1 - uy) * w.b + (1 - ux) * uy * w.c + ux * uy * w.d) /
            (w.a + w.b + w.c + w.d);
 }
+// An emitting triangle seen from a reference point: its corners, the unit vectors to them and
+// the solid angle (0 when a corner is the point itself).  Sampling a point, its density and
+// the density's inverse mapping are all functions of these, so they are computed once per
+// light sample instead of by each (27 normalisations of three divisions before, 3 now).
+struct SeenTriangle {
+    V3 p[3], a, b, c;
+    float area;
+};
+// :86-90 (triangle_solid_angle)
+RP_DEV void see_triangle(SeenTriangle &t, V3 r) {
+    const V3 da = t.p[0] - r, db = t.p[1] - r, dc = t.p[2] - r;
+    t.area = 0;
+    t.a = t.b = t.c = v3(0, 0, 0);
+    if (!nonzero_len(da) || !nonzero_len(db) || !nonzero_len(dc))
+        return;
+    t.a = unitv(da);
+    t.b = unitv(db);
+    t.c = unitv(dc);
+    t.area = sph_triangle_area(t.a, t.b, t.c);
+}
+RP_DEV bool spherical_range(float area) { return area >= 3e-4f && area <= 6.22f; }
 // :116-121
-RP_DEV W4 triangle_cosines(V3 a, V3 b, V3 c, V3 r, V3 n) {
-    const float wa = fmaxf(.01f, fabsf(dot(n, unitv(a - r))));
-    const float wb = fmaxf(.01f, fabsf(dot(n, unitv(b - r))));
-    const float wc = fmaxf(.01f, fabsf(dot(n, unitv(c - r))));
+RP_DEV W4 triangle_cosines(const SeenTriangle &t, V3 n) {
+    const float wa = fmaxf(.01f, fabsf(dot(n, t.a)));
+    const float wb = fmaxf(.01f, fabsf(dot(n, t.b)));
+    const float wc = fmaxf(.01f, fabsf(dot(n, t.c)));
     return {wb, wb, wa, wc};
 }
 // :128-172 (PBRT SampleSphericalTriangle, rationalised)
-RP_DEV bool sph_triangle_sample(V3 p0, V3 p1, V3 p2, V3 r, float ux, float uy, float &b1o, float &b2o) {
-    const V3 a = unitv(p0 - r), b = unitv(p1 - r), c = unitv(p2 - r);
+RP_DEV bool sph_triangle_sample(const SeenTriangle &tri, V3 r, float ux, float uy, float &b1o, float &b2o) {
+    const V3 a = tri.a, b = tri.b, c = tri.c;
     const V3 nab = cross(a, b), nca = cross(c, a);
     if (!nonzero_len(nab) || !nonzero_len(nca))
         return false;
     const float alpha = sph_angle(unitv(nab), -unitv(nca));
-    const float area = sph_triangle_area(a, b, c);
+    const float area = tri.area;
     const float ca = cosf(alpha), sa = sinf(alpha);
     const float subarea = ux * area;
     const float sh = sinf(subarea / 2), st = sinf(subarea), ct_area = cosf(subarea);
@@ -658,11 +696,11 @@ RP_DEV bool sph_triangle_sample(V3 p0, V3 p1, V3 p2, V3 r, float ux, float uy, f
     if (!nonzero_len(tangent))
         return false;
     const V3 direction = ct * b + safe_sqrt(omct * (2 - omct)) * unitv(tangent);
-    const V3 e1 = p1 - p0, e2 = p2 - p0, s1 = cross(direction, e2);
+    const V3 e1 = tri.p[1] - tri.p[0], e2 = tri.p[2] - tri.p[0], s1 = cross(direction, e2);
     const float denom = dot(s1, e1);
     if (denom == 0)
         return false;
-    const V3 sv = r - p0;
+    const V3 sv = r - tri.p[0];
     float b1 = clamp01(dot(sv, s1) / denom), b2 = clamp01(dot(direction, cross(sv, e1)) / denom);
     if (b1 + b2 > 1) {
         const float sum = b1 + b2;
@@ -674,13 +712,12 @@ RP_DEV bool sph_triangle_sample(V3 p0, V3 p1, V3 p2, V3 r, float ux, float uy, f
     return isfinite(b1) && isfinite(b2);
 }
 // :174-182
-RP_DEV void sph_triangle_inverse(V3 p0, V3 p1, V3 p2, V3 r, V3 dir, float &u0, float &u1) {
-    const V3 a = unitv(p0 - r), b = unitv(p1 - r), c = unitv(p2 - r);
-    V3 cp = unitv(cross(cross(b, dir), cross(c, a)));
-    if (dot(cp, a + c) < 0)
+RP_DEV void sph_triangle_inverse(const SeenTriangle &t, V3 dir, float &u0, float &u1) {
+    V3 cp = unitv(cross(cross(t.b, dir), cross(t.c, t.a)));
+    if (dot(cp, t.a + t.c) < 0)
         cp = -cp;
-    u0 = clamp01(sph_triangle_area(a, b, cp) / sph_triangle_area(a, b, c));
-    u1 = clamp01(dot(dir - b, dir - b) / dot(cp - b, cp - b));
+    u0 = clamp01(sph_triangle_area(t.a, t.b, cp) / t.area);
+    u1 = clamp01(dot(dir - t.b, dir - t.b) / dot(cp - t.b, cp - t.b));
 }
 // shaders/light_geometry_sampling.h:16-29
 RP_DEV void emitter_corners(const DeviceScene &s, u32 emitter, V3 p[3]) {
@@ -699,43 +736,53 @@ RP_DEV float area_solid_angle_pdf(float area_density, V3 reference, const Surfac
     const float cosine = fabsf(dot(point.geometric_normal, delta * (1.0f / sqrtf(d2))));
     return cosine > 0 ? area_density * d2 / cosine : 0;
 }
-// shaders/light_geometry_sampling.h:116-153 (triangles)
-__device__ __noinline__ float light_geometry_pdf(const DeviceScene &s, u32 emitter, V3 reference, V3 normal, const SurfacePoint &point) {
+// The solid-angle density of `point` on a seen triangle; `weights`: its normalised cosines
+// where the reference has a normal.
+RP_DEV float seen_pdf(const SeenTriangle &t, V3 reference, bool weighted, W4 weights, const SurfacePoint &point) {
     const V3 delta = point.position - reference;
     if (!(dot(delta, delta) > 0) || !(point.inverse_area_pdf > 0))
         return 0;
-    V3 p[3];
-    emitter_corners(s, emitter, p);
-    const float area = triangle_solid_angle(p[0], p[1], p[2], reference);
-    if (area >= 3e-4f && area <= 6.22f) {
+    if (spherical_range(t.area)) {
         float u0, u1;
-        sph_triangle_inverse(p[0], p[1], p[2], reference, normalize3(delta), u0, u1);
-        return (dot(normal, normal) > 0 ? bilinear_pdf(u0, u1, triangle_cosines(p[0], p[1], p[2], reference, normal))
-                                        : 1.f) /
-               area;
+        sph_triangle_inverse(t, normalize3(delta), u0, u1);
+        return (weighted ? bilinear_pdf(u0, u1, weights) : 1.f) / t.area;
     }
     return area_solid_angle_pdf(1 / point.inverse_area_pdf, reference, point);
 }
-// shaders/light_geometry_sampling.h:155-209 (triangles)
+// shaders/light_geometry_sampling.h:116-153 (triangles)
+__device__ __noinline__ float light_geometry_pdf(const DeviceScene &s, u32 emitter, V3 reference, V3 normal, const SurfacePoint &point) {
+    SeenTriangle t;
+    emitter_corners(s, emitter, t.p);
+    see_triangle(t, reference);
+    const bool weighted = dot(normal, normal) > 0;
+    W4 w{1, 1, 1, 1};
+    if (weighted && spherical_range(t.area))
+        w = normalized_weights(triangle_cosines(t, normal));
+    return seen_pdf(t, reference, weighted, w, point);
+}
+// shaders/light_geometry_sampling.h:155-209 (triangles).  `pdf` is light_geometry_pdf of the
+// sampled point.
 __device__ __noinline__ bool light_geometry_sample(const DeviceScene &s, u32 emitter, V3 reference, V3 normal, float ux, float uy,
                                   SurfacePoint &point, float &pdf) {
     if (!isfinite(ux) || !isfinite(uy) || ux < 0 || uy < 0 || ux > 1 || uy > 1)
         return false;
     ux = fminf(ux, kOneMinusEps);
     uy = fminf(uy, kOneMinusEps);
-    V3 p[3];
-    emitter_corners(s, emitter, p);
+    SeenTriangle t;
+    emitter_corners(s, emitter, t.p);
+    see_triangle(t, reference);
+    const bool weighted = dot(normal, normal) > 0;
+    W4 w{1, 1, 1, 1};
     float b1, b2;
-    const float area = triangle_solid_angle(p[0], p[1], p[2], reference);
-    if (area >= 3e-4f && area <= 6.22f) {
-        if (dot(normal, normal) > 0) {
-            const W4 w = normalized_weights(triangle_cosines(p[0], p[1], p[2], reference, normal));
+    if (spherical_range(t.area)) {
+        if (weighted) {
+            w = normalized_weights(triangle_cosines(t, normal));
             const float y = linear_sample(uy, w.a + w.b, w.c + w.d);
             const float x = linear_sample(ux, (1 - y) * w.a + y * w.c, (1 - y) * w.b + y * w.d);
             ux = x;
             uy = y;
         }
-        if (!sph_triangle_sample(p[0], p[1], p[2], reference, ux, uy, b1, b2))
+        if (!sph_triangle_sample(t, reference, ux, uy, b1, b2))
             return false;
     } else {
         const float root = sqrtf(ux);
@@ -745,7 +792,7 @@ __device__ __noinline__ bool light_geometry_sample(const DeviceScene &s, u32 emi
     if (!isfinite(b1) || !isfinite(b2) ||
         !triangle_surface_point(s, s.emitter_instance[emitter], s.emitter_local[emitter], b1, b2, false, point))
         return false;
-    pdf = light_geometry_pdf(s, emitter, reference, normal, point);
+    pdf = seen_pdf(t, reference, weighted, w, point);
     return isfinite(pdf) && pdf >= 0;
 }
 
