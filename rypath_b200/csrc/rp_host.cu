@@ -773,6 +773,24 @@ template <class T> T *dupload(std::vector<void *> &owned, const T *src, size_t c
     return p;
 }
 
+// The range of knots [begin, begin + count) when they increase strictly and each lies within a
+// quarter of a step of even spacing, so that a wavelength's segment can be guessed
+// (KnotRange); scale 0 otherwise.
+KnotRange uniform_knots(const rp_scene_desc *d, u32 begin, u32 count) {
+    const KnotRange none{0, 0, 0};
+    if (!d->knots || count < 2 || begin > d->knot_count || count > d->knot_count - begin)
+        return none;
+    const float2 *k = reinterpret_cast<const float2 *>(d->knots) + begin;
+    const double first = k[0].x, step = (double(k[count - 1].x) - first) / (count - 1);
+    if (!std::isfinite(first) || !std::isfinite(step) || !(step > 0))
+        return none;
+    for (u32 i = 0; i < count; ++i)
+        if (!(std::fabs(double(k[i].x) - (first + i * step)) <= 0.25 * step) || (i && !(k[i].x > k[i - 1].x)))
+            return none;
+    const float scale = float(1 / step), span = k[count - 1].x - k[0].x;
+    return std::isfinite(scale) && scale > 0 && std::isfinite(span) ? KnotRange{k[0].x, k[count - 1].x, scale} : none;
+}
+
 // Upload a description's images in their wire layout; an environment image also gets its
 // importance tables and its light power (mean RGB illuminant power times its scale; -1 when
 // there is no environment image).
@@ -935,10 +953,10 @@ struct rp_scene {
     // on `stream`; `forked` and `joined` order the two (timing disabled)
     cudaStream_t side = nullptr;
     cudaEvent_t forked = nullptr, joined = nullptr;
-    // Owen prefix table of the draw blocks (attach_owen_prefix), built for one seed
-    unsigned short *owen_prefix = nullptr;
-    u32 owen_capacity = 0, owen_blocks = 0, owen_seed = 0;
-    bool owen_built = false;
+    // tables of the draw blocks (attach_draw_tables), built for one seed
+    unsigned char *draw_tables = nullptr;
+    u32 draw_capacity = 0, draw_blocks = 0, draw_seed = 0;
+    bool draw_built = false;
     // the shade kernels of BSDF families 1-3 run on their own streams beside family 0's
     cudaStream_t family[3] = {nullptr, nullptr, nullptr};
     cudaEvent_t family_done[3] = {nullptr, nullptr, nullptr};
@@ -1001,8 +1019,8 @@ struct rp_scene {
             cudaFreeAsync(scalar_records, stream);
         if (slot_storage)
             cudaFreeAsync(slot_storage, stream);
-        if (owen_prefix)
-            cudaFreeAsync(owen_prefix, stream);
+        if (draw_tables)
+            cudaFreeAsync(draw_tables, stream);
         if (adjoint_storage)
             cudaFreeAsync(adjoint_storage, stream);
         if (film_stage)
@@ -1435,37 +1453,52 @@ void launch_shade(rp_scene *s, const WaveParams &p, const PathPool &pool, int in
     launch_shade_img<Adjoint, true>(s, p, pool, in, grid, smem);
 }
 
-// Sobol sampler with Owen randomisation: attaches the table of the first kOwenPrefixBits
-// scrambling rounds of the continuation and light-sample draw blocks (one block per vertex up to
-// the maximum depth), building it on the scene stream when the seed or depth changed.  Every
-// word drawn through it equals the fully computed word.
-void attach_owen_prefix(rp_scene *s, WaveParams &p) {
+// Sobol sampler with Owen randomisation: attaches the tables of the draw blocks of the scene's
+// transport, building them on the scene stream when the seed or depth changed.  Hero: the
+// continuation and light-sample blocks [4, 4 + n) and [133, 133 + n), one of each per vertex up
+// to the maximum depth; scalar: blocks [1, 1 + n), two per vertex.  Every word drawn through
+// them equals the fully computed word.
+void attach_draw_tables(rp_scene *s, WaveParams &p) {
     p.owen_prefix = nullptr;
-    p.owen_blocks = 0;
+    p.draw_bytes = nullptr;
+    p.draw_hash = nullptr;
+    p.draw_first = p.draw_blocks = 0;
     if (p.sampler != RP_SAMPLER_SOBOL || p.randomization != RP_RANDOMIZE_OWEN)
         return;
-    const u32 blocks = std::min<u32>(std::max<u32>(s->ds.max_depth, 1), 129);
-    if (s->owen_capacity < blocks) {
-        if (s->owen_prefix)
-            cudaFreeAsync(s->owen_prefix, s->stream);
-        s->owen_prefix = nullptr;
-        s->owen_capacity = 0;
-        s->owen_built = false;
-        RP_CHECK(cudaMallocAsync(reinterpret_cast<void **>(&s->owen_prefix),
-                                 size_t(2) * blocks * 4 * kOwenPrefixEntries * sizeof(unsigned short), s->stream));
-        s->owen_capacity = blocks;
+    const bool hero = s->transport == RP_TRANSPORT_HERO;
+    const u32 depth = std::max<u32>(s->ds.max_depth, 1);
+    const u32 blocks = hero ? std::min<u32>(depth, 129) : 2 * std::min<u32>(depth, 127);
+    const u32 tables = hero ? 2 * blocks : blocks, first = hero ? 4 : 1;
+    const size_t products = size_t(tables) * kIndexBytes * 256 * sizeof(uint4);
+    const size_t prefixes = size_t(tables) * 4 * kOwenPrefixEntries * sizeof(unsigned short);
+    if (s->draw_capacity < tables) {
+        if (s->draw_tables)
+            cudaFreeAsync(s->draw_tables, s->stream);
+        s->draw_tables = nullptr;
+        s->draw_capacity = 0;
+        s->draw_built = false;
+        RP_CHECK(cudaMallocAsync(reinterpret_cast<void **>(&s->draw_tables), products + prefixes + tables * 4 * sizeof(u32),
+                                 s->stream));
+        s->draw_capacity = tables;
     }
-    if (!s->owen_built || s->owen_seed != p.seed_low || s->owen_blocks != blocks) {
-        const u32 total = 2 * blocks * 4 * kOwenPrefixEntries;
-        k_owen_prefix<<<grid_for(s->sm_count, total, 256, 8), 256, 0, s->stream>>>(s->owen_prefix, blocks, p.seed_low);
+    uint4 *bytes = reinterpret_cast<uint4 *>(s->draw_tables);
+    unsigned short *prefix = reinterpret_cast<unsigned short *>(s->draw_tables + products);
+    u32 *hash = reinterpret_cast<u32 *>(s->draw_tables + products + prefixes);
+    if (!s->draw_built || s->draw_seed != p.seed_low || s->draw_blocks != blocks) {
+        const u32 total = tables * 4 * kOwenPrefixEntries;
+        k_draw_tables<<<grid_for(s->sm_count, total, 256, 8), 256, 0, s->stream>>>(s->ds.sobol, prefix, bytes, hash, first,
+                                                                                   blocks, tables, p.seed_low);
         RP_CHECK(cudaGetLastError());
         ++s->launches;
-        s->owen_seed = p.seed_low;
-        s->owen_blocks = blocks;
-        s->owen_built = true;
+        s->draw_seed = p.seed_low;
+        s->draw_blocks = blocks;
+        s->draw_built = true;
     }
-    p.owen_prefix = s->owen_prefix;
-    p.owen_blocks = blocks;
+    p.owen_prefix = prefix;
+    p.draw_bytes = bytes;
+    p.draw_hash = hash;
+    p.draw_first = first;
+    p.draw_blocks = blocks;
 }
 
 // One wave: raygen, then max_depth + 1 events of trace -> shade -> shadow.
@@ -1479,7 +1512,7 @@ void attach_owen_prefix(rp_scene *s, WaveParams &p) {
 // order's.
 void run_wave(rp_scene *s, const WaveParams &request_params, size_t adjoint_smem = 0) {
     WaveParams p = request_params;
-    attach_owen_prefix(s, p);
+    attach_draw_tables(s, p);
     s->ensure_pool(p.lanes);
     PathPool &pool = s->pool;
     pool.lane_closest = s->counting ? s->lane_closest : nullptr;
@@ -1581,7 +1614,9 @@ constexpr int kScalarTripsPerCheck = 8;
 
 // One wave of the scalar transport, one record per lane in s->scalar_records: camera rays,
 // then walk / step trips over the slots until every lane's record is written.
-void run_scalar_wave(rp_scene *s, const WaveParams &p, u32 boundary_limit) {
+void run_scalar_wave(rp_scene *s, const WaveParams &request_params, u32 boundary_limit) {
+    WaveParams p = request_params;
+    attach_draw_tables(s, p);
     s->ensure_scalar(p.lanes);
     if (!s->step_blocks) {
         int per_sm = 0;
@@ -2140,7 +2175,9 @@ rp_status rp_cuda_scene_create(const rp_scene_desc *d, int device, rp_scene **ou
                        m.u_roughness, m.v_roughness, m.remap_roughness,    m.first_material,  m.second_material,
                        m.mix_amount,  m.image_texture, {m.coefficients[0], m.coefficients[1], m.coefficients[2]},
                        {m.reflectance[0], m.reflectance[1], m.reflectance[2], m.reflectance[3], m.reflectance[4],
-                        m.reflectance[5], m.reflectance[6], m.reflectance[7]}};
+                        m.reflectance[5], m.reflectance[6], m.reflectance[7]},
+                       uniform_knots(d, m.knot_begin, m.knot_count), uniform_knots(d, m.eta_begin, m.eta_count),
+                       uniform_knots(d, m.k_begin, m.k_count)};
         }
         ds.materials = dupload(own, mats.data(), mats.size(), stm);
         ds.material_count = d->material_count;
@@ -3109,7 +3146,7 @@ float run_batch(rp_scene *s, const BatchPlan &plan, const BatchBuffers &buf, con
                 const rp_batch_config &c, FilmPixel *film, size_t waves) {
     s->ensure_pool(c.wave_lanes);
     WaveParams p = batch_params(r);
-    attach_owen_prefix(s, p);
+    attach_draw_tables(s, p);
     const FilmClamp clamp = film_clamp(r.exposure, r.max_component_value);
     const Batch b = buf.batch(plan);
     RP_CHECK(cudaMemsetAsync(buf.cursor, 0, 8, s->stream));

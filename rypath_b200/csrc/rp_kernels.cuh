@@ -344,7 +344,12 @@ __global__ void __launch_bounds__(Block, 512 / Block) k_shade(const __grid_const
                             status = 1;
                             break;
                         }
-                        const uint4 draws = draw_words(s, p, ident.x, ident.y, ident.z, index, 4 + cnt - 2);
+                        // only a dielectric reads the lobe word, a smooth one only that of the
+                        // three, and the first event no roulette word
+                        const bool survival = roulette && cnt > 2;
+                        const u32 set = F == 2 ? (cbsdf.g.smooth ? (survival ? kDrawXW : kDrawX) : kDrawAll)
+                                               : (survival ? kDrawYZW : kDrawYZ);
+                        const uint4 draws = draw_words(s, p, ident.x, ident.y, ident.z, index, 4 + cnt - 2, set);
                         swo = to_local(cframe, cwo);
                         cbsdf.active_mask = active_mask;
                         direct_density = density;
@@ -602,14 +607,14 @@ __global__ void __launch_bounds__(Block, 512 / Block) k_nee(const __grid_constan
                         // point on an area light, are drawn only when an area light was selected
                         // (the same words either way)
                         const u32 block = 133 + cnt - 2;
-                        const float u0 = sample_uniform(p, draw_word0(s, p, ident.x, ident.y, ident.z, index, block));
+                        const float u0 = sample_uniform(p, draw_words(s, p, ident.x, ident.y, ident.z, index, block, kDrawX).x);
                         // sample_li (shaders/packet_transport.h:470-553)
                         float selected_pmf = 0; // light_pmf of the selected light
                         const Selected choice = light_sample<true>(s, cp.position, cp.shading_normal, u0, selected_pmf);
                         float u1 = 0, u2 = 0;
                         const bool env_image = Img && s.img.env_image != kNone && choice.light == s.environment_light;
                         if (choice.pmf > 0 && (choice.light < s.emitter_count || env_image)) {
-                            const uint4 w = draw_words(s, p, ident.x, ident.y, ident.z, index, block);
+                            const uint4 w = draw_words(s, p, ident.x, ident.y, ident.z, index, block, kDrawYZ);
                             u1 = sample_uniform(p, w.y);
                             u2 = sample_uniform(p, w.z);
                         }
@@ -972,14 +977,29 @@ __global__ void k_count_failures(PathPool pool, u32 lanes) {
     }
 }
 // Every sample of a wave reduced per pixel in canonical (absolute sample, pixel) order.
-// Owen prefix table (owen_prefix_rounds of every prefix) of the draw blocks [4, 4 + blocks)
-// and [133, 133 + blocks), four dimensions each.
-__global__ void k_owen_prefix(unsigned short *table, u32 blocks, u32 seed) {
-    const u32 total = 2 * blocks * 4 * kOwenPrefixEntries;
-    for (u32 e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
-        const u32 slot = e / (4 * kOwenPrefixEntries), k = (e / kOwenPrefixEntries) & 3u, prefix = e % kOwenPrefixEntries;
-        const u32 block = slot < blocks ? 4 + slot : 133 + (slot - blocks);
-        table[e] = (unsigned short)owen_prefix_rounds(prefix, sobol_dimension_hash(4 * block + k, seed));
+// The DrawTables of the draw blocks [first, first + blocks), then [133, ...), `tables` in all.
+__global__ void k_draw_tables(SobolTables sobol, unsigned short *prefix, uint4 *bytes, u32 *hash, u32 first, u32 blocks,
+                              u32 tables, u32 seed) {
+    const u32 prefixes = tables * 4 * kOwenPrefixEntries, products = tables * kIndexBytes * 256;
+    const u32 stride = gridDim.x * blockDim.x, begin = blockIdx.x * blockDim.x + threadIdx.x;
+    for (u32 e = begin; e < prefixes; e += stride) {
+        const u32 slot = e / (4 * kOwenPrefixEntries), k = (e / kOwenPrefixEntries) & 3u;
+        const u32 block = slot < blocks ? first + slot : 133 + (slot - blocks);
+        const u32 h = sobol_dimension_hash(4 * block + k, seed);
+        prefix[e] = (unsigned short)owen_prefix_rounds(e % kOwenPrefixEntries, h);
+        if (e % kOwenPrefixEntries == 0)
+            hash[4 * slot + k] = h;
+    }
+    for (u32 e = begin; e < products; e += stride) {
+        const u32 slot = e / (kIndexBytes * 256), byte = (e >> 8) % kIndexBytes, value = e & 0xffu;
+        const u32 block = slot < blocks ? first + slot : 133 + (slot - blocks);
+        u32 v[4] = {0, 0, 0, 0};
+        for (u32 bit = 0; bit < 8 && 8 * byte + bit < kSobolMatrix; ++bit)
+            if (value >> bit & 1u)
+                for (u32 k = 0; k < 4; ++k)
+                    if (4 * block + k < 1024u)
+                        v[k] ^= __ldg(sobol.directions + (4 * block + k) * kSobolMatrix + 8 * byte + bit);
+        bytes[e] = make_uint4(v[0], v[1], v[2], v[3]);
     }
 }
 

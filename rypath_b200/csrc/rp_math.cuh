@@ -170,81 +170,102 @@ RP_DEV u32 owen_prefix_rounds(u32 prefix, u32 hash) {
             value ^= u32(1) << (31 - bit);
     return value >> (32 - kOwenPrefixBits);
 }
-// Four consecutive dimensions [dimension, dimension + 4) of one Sobol index, each equal to
-// sobol_word of its dimension.  `prefix` (optional, Owen only): the four dimensions' tables of
-// owen_prefix_rounds, kOwenPrefixEntries entries each.  The four generator products share the walk over the index
-// bits, and the four Owen bit loops run in lockstep: each loop is a chain of dependent 64-bit
-// hashes, so four independent chains keep the pipelines busy where one would stall on each
-// hash.
-RP_DEV uint4 sobol_words4(const SobolTables &t, u64 index, u32 dimension, u32 mode, u32 seed,
-                          const unsigned short *prefix = nullptr) {
-    const u32 *col = t.directions + dimension * kSobolMatrix;
-    u32 v[4] = {0, 0, 0, 0};
-    u32 lo = u32(index), hi = u32(index >> 32);
-    while (lo) {
-        const int b = __ffs(lo) - 1;
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            v[k] ^= __ldg(col + k * kSobolMatrix + b);
-        lo &= lo - 1;
-    }
-    while (hi) {
-        const int b = __ffs(hi) - 1;
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            v[k] ^= __ldg(col + k * kSobolMatrix + 32 + b);
-        hi &= hi - 1;
-    }
-    if (mode == 0)
-        return make_uint4(v[0], v[1], v[2], v[3]);
-    u32 h[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-        h[k] = sobol_dimension_hash(dimension + k, seed);
-    if (mode != 3) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            v[k] = scramble_word(v[k], mode, h[k]);
-        return make_uint4(v[0], v[1], v[2], v[3]);
-    }
-    // Owen (the mode-3 loop of scramble_word), four words at once
-    u32 first = 1;
-    if (prefix) {
-        constexpr u32 low = 32 - kOwenPrefixBits;
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            v[k] = (v[k] & ((u32(1) << low) - 1)) | (u32(__ldg(prefix + k * kOwenPrefixEntries + (v[k] >> low))) << low);
-        first = kOwenPrefixBits;
-    } else {
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            v[k] ^= (h[k] & 1) << 31;
-    }
-#pragma unroll 1
-    for (u32 bit = first; bit < 32; ++bit) {
-        const u32 mask = ~u32(0) << (32 - bit), flip = u32(1) << (31 - bit);
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (u32(mix_bits((v[k] & mask) ^ h[k])) & (u32(1) << bit))
-                v[k] ^= flip;
-    }
-    return make_uint4(v[0], v[1], v[2], v[3]);
+// Tables of one draw block (the four dimensions [d, d + 4) of one seed, k_draw_tables): their
+// dimension hashes, owen_prefix_rounds of every prefix, and the generator products of every
+// byte of the index -- the four dimensions' words side by side, so that a product is one
+// 16-byte load for each byte of the index instead of a walk over its set bits.
+constexpr u32 kIndexBytes = 7; // 52 generator columns
+struct DrawTable {
+    const unsigned short *prefix; // [4][kOwenPrefixEntries]
+    const uint4 *bytes;           // [kIndexBytes][256]
+    const u32 *hash;              // [4]
+};
+RP_DEV u32 word_of(const uint4 &v, int k) { return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w; }
+// mix_bits after its first step, whose shift by 31 of a 32-bit value only carries its top bit
+// into bit 0: constant over the rounds of a word, so sobol_words folds it into the hash.
+RP_DEV u32 mix_bits_tail(u32 z) {
+    u64 v = u64(z) * 0x7fb5d329728ea185ull;
+    v ^= v >> 27;
+    v *= 0x81dadef4bc2dd44dull;
+    return u32(v ^ (v >> 33));
 }
-// sobol_word of one dimension; with Owen randomisation and that dimension's table of
-// owen_prefix_rounds (`prefix`, optional), the table replaces the first kOwenPrefixBits rounds.
-RP_DEV u32 sobol_word_prefixed(const SobolTables &t, u64 index, u32 dimension, u32 mode, u32 seed,
-                               const unsigned short *prefix) {
-    if (mode != 3 || !prefix)
-        return sobol_word(t, index, dimension, mode, seed);
-    constexpr u32 low = 32 - kOwenPrefixBits;
-    u32 v = sobol_raw(t, index, dimension);
-    const u32 h = sobol_dimension_hash(dimension, seed);
-    v = (v & ((u32(1) << low) - 1)) | (u32(__ldg(prefix + (v >> low))) << low);
+// Words K... of the four consecutive dimensions [dimension, dimension + 4) of one Sobol index,
+// each equal to sobol_word of its dimension; out[k] of the other words is left alone.  `table`
+// (optional, Owen only): the block's tables.  The Owen bit loops run in lockstep: each loop is
+// a chain of dependent 64-bit hashes, so independent chains keep the pipelines busy where one
+// would stall on each hash.  Coarse: the caller reads only the top kOwenPrefixBits bits of
+// that word, which a table gives without any round.
+template <int Coarse, int... K>
+RP_DEV void sobol_words(const SobolTables &t, u64 index, u32 dimension, u32 mode, u32 seed, const DrawTable &table,
+                        u32 (&out)[4]) {
+    constexpr int N = sizeof...(K);
+    constexpr int dim[N] = {K...};
+    u32 v[N] = {}, h[N];
+    const bool tabled = table.prefix != nullptr;
+    if (tabled) {
+        const uint4 *e = table.bytes;
 #pragma unroll 1
-    for (u32 bit = kOwenPrefixBits; bit < 32; ++bit)
-        if (u32(mix_bits((v & (~u32(0) << (32 - bit))) ^ h)) & (u32(1) << bit))
-            v ^= u32(1) << (31 - bit);
-    return v;
+        for (u32 byte = 0; index && byte < kIndexBytes; ++byte, index >>= 8, e += 256) {
+            const uint4 w = __ldg(e + (u32(index) & 0xffu));
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+                v[k] ^= word_of(w, dim[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < N; ++k)
+            h[k] = __ldg(table.hash + dim[k]);
+    } else {
+        const u32 *col = t.directions + dimension * kSobolMatrix;
+#pragma unroll 1
+        for (; index; index &= index - 1) {
+            const int b = __ffsll((long long)index) - 1;
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+                v[k] ^= __ldg(col + dim[k] * kSobolMatrix + b);
+        }
+        if (mode != 0) {
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+                h[k] = sobol_dimension_hash(dimension + dim[k], seed);
+        }
+    }
+    if (mode == 3) {
+        // Owen (the mode-3 loop of scramble_word), all words at once
+        u32 first = 1;
+        if (tabled) {
+            constexpr u32 low = 32 - kOwenPrefixBits;
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+                v[k] = (v[k] & ((u32(1) << low) - 1)) |
+                       (u32(__ldg(table.prefix + dim[k] * kOwenPrefixEntries + (v[k] >> low))) << low);
+            first = kOwenPrefixBits;
+        } else {
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+                v[k] ^= (h[k] & 1) << 31;
+        }
+#pragma unroll
+        for (int k = 0; k < N; ++k)
+            h[k] ^= (v[k] ^ h[k]) >> 31; // mix_bits' first step
+#pragma unroll 1
+        for (u32 bit = first; bit < 32; ++bit) {
+            const u32 mask = ~u32(0) << (32 - bit), flip = u32(1) << (31 - bit);
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                if (dim[k] == Coarse && tabled)
+                    continue;
+                if (mix_bits_tail((v[k] & mask) ^ h[k]) & (u32(1) << bit))
+                    v[k] ^= flip;
+            }
+        }
+    } else if (mode != 0) {
+#pragma unroll
+        for (int k = 0; k < N; ++k)
+            v[k] = scramble_word(v[k], mode, h[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+        out[dim[k]] = v[k];
 }
 // src/sobol_shared.h:143-154
 RP_DEV float sobol_uniform(u32 v) {
@@ -1374,8 +1395,8 @@ template <int K> RP_DEV HeroSample hero_sample_k(const HeroBsdf &p, V3 wo, float
 }
 
 // ------------------------------------------------------------------ spectra and geometry helpers
-// shaders/render.metal:548-574
-RP_DEV float pbrt_reflectance(const float2 *k, u32 count, float w) {
+// shaders/render.metal:548-574; out of line: evenly spaced knots do not reach it
+__device__ __noinline__ float pbrt_reflectance(const float2 *k, u32 count, float w) {
     if (w < k[0].x || w > k[count - 1].x)
         return 0.0f;
     u32 lo = 0, hi = count - 1;
@@ -1414,18 +1435,81 @@ RP_DEV u32 dense_index(float w) {
     const u32 nm = u32(w);
     return nm + u32(w - float(nm) >= 0.5f) - 360u;
 }
+// Knots of a sampled spectrum that are close to evenly spaced (uniform_knots, checked on the
+// host; scale 0: not): the segment of a wavelength is guessed from its position, and taken
+// when its knots hold the wavelength -- the segment that the search finds, the knots being
+// strictly increasing.  The search is a chain of seven dependent loads for 32 knots.
+struct KnotRange {
+    float first, last, scale; // segments per unit
+};
+// Four wavelengths' values at once (their loads overlap): pbrt_reflectance of each, or with
+// `extend` the end values outside the knots (optical_value).
+RP_DEV void knot_values4(const float2 *k, u32 count, const KnotRange &r, bool extend, V4 w, float (&out)[4]) {
+    if (r.scale > 0) {
+        float2 a[4], b[4];
+        bool held = true;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float x = fminf(fmaxf(w.v[i], r.first), r.last);
+            const u32 g = min(u32((x - r.first) * r.scale), count - 2);
+            a[i] = __ldg(k + g);
+            b[i] = __ldg(k + g + 1);
+            held = held && a[i].x <= x && (x < b[i].x || g == count - 2);
+        }
+        if (held) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float span = b[i].x - a[i].x;
+                const float t = (w.v[i] - a[i].x) / span;
+                const float inside = a[i].y + (b[i].y - a[i].y) * t;
+                out[i] = w.v[i] < r.first  ? (extend ? a[i].y : 0.0f)
+                         : w.v[i] > r.last ? (extend ? b[i].y : 0.0f)
+                                           : inside;
+            }
+            return;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        out[i] = extend && w.v[i] < k[0].x ? k[0].y
+                 : extend && w.v[i] > k[count - 1].x ? k[count - 1].y
+                                                     : pbrt_reflectance(k, count, w.v[i]);
+}
+// One wavelength of knot_values4
+RP_DEV float knot_value(const float2 *k, u32 count, const KnotRange &r, bool extend, float w) {
+    if (r.scale > 0) {
+        const float x = fminf(fmaxf(w, r.first), r.last);
+        const u32 g = min(u32((x - r.first) * r.scale), count - 2);
+        const float2 a = __ldg(k + g), b = __ldg(k + g + 1);
+        if (a.x <= x && (x < b.x || g == count - 2)) {
+            if (w < r.first)
+                return extend ? a.y : 0.0f;
+            if (w > r.last)
+                return extend ? b.y : 0.0f;
+            const float t = (w - a.x) / (b.x - a.x);
+            return a.y + (b.y - a.y) * t;
+        }
+    }
+    if (extend && w < k[0].x)
+        return k[0].y;
+    if (extend && w > k[count - 1].x)
+        return k[count - 1].y;
+    return pbrt_reflectance(k, count, w);
+}
 // shaders/render.metal:1978-1990
-RP_DEV float optical_value(const float2 *knots, u32 begin, u32 count, u32 total, bool extend, float w) {
+RP_DEV float optical_value(const float2 *knots, u32 begin, u32 count, u32 total, const KnotRange &r, bool extend, float w) {
     if (count < 2 || begin > total || count > total - begin)
         return __int_as_float(0x7fffffff);
-    const float2 *c = knots + begin;
-    if (extend) {
-        if (w < c[0].x)
-            return c[0].y;
-        if (w > c[count - 1].x)
-            return c[count - 1].y;
+    return knot_value(knots + begin, count, r, extend, w);
+}
+// optical_value of four wavelengths
+RP_DEV void optical_values4(const float2 *knots, u32 begin, u32 count, u32 total, const KnotRange &r, bool extend, V4 w,
+                            float (&out)[4]) {
+    if (count < 2 || begin > total || count > total - begin) {
+        out[0] = out[1] = out[2] = out[3] = __int_as_float(0x7fffffff);
+        return;
     }
-    return pbrt_reflectance(c, count, w);
+    knot_values4(knots + begin, count, r, extend, w, out);
 }
 // shaders/render.metal:849-852
 RP_DEV float gamma_bound(float n) {

@@ -37,6 +37,7 @@ struct DMaterial {
     u32 image_texture; // image reflectance (kind 3)
     float coefficients[3]; // RGB sigmoid reflectance (kind 2)
     float reflectance[8];  // demo-model sampled reflectance at the demo knots
+    KnotRange knot_range, eta_range, k_range;
 };
 struct DPositional {
     float position[3];

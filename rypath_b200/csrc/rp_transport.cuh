@@ -82,20 +82,25 @@ struct WaveParams {
     u32 lanes;
     u32 log_spp;        // ZSobol: log2 of the total sample budget
     u32 boundary_limit; // pass-through crossings allowed between two vertices
-    // Sobol sampler with Owen randomisation: the first kOwenPrefixBits scrambling rounds of the
-    // draw blocks [4, 4 + owen_blocks) and [133, 133 + owen_blocks), tabulated (null: none)
+    // Sobol sampler with Owen randomisation: tables (DrawTable) of the draw blocks [draw_first,
+    // draw_first + draw_blocks) and, for the hero transport (draw_first 4), [133, 133 +
+    // draw_blocks); null: none
     const unsigned short *owen_prefix;
-    u32 owen_blocks;
+    const uint4 *draw_bytes;
+    const u32 *draw_hash;
+    u32 draw_first, draw_blocks;
 };
-// Table of one draw block's four dimensions in the Owen prefix table (null if not tabulated).
-RP_DEV const unsigned short *owen_prefix_table(const WaveParams &p, u32 block) {
-    if (!p.owen_prefix || p.randomization != 3)
-        return nullptr;
-    if (block - 4u < p.owen_blocks)
-        return p.owen_prefix + size_t(block - 4u) * 4 * kOwenPrefixEntries;
-    if (block - 133u < p.owen_blocks)
-        return p.owen_prefix + size_t(p.owen_blocks + block - 133u) * 4 * kOwenPrefixEntries;
-    return nullptr;
+// Tables of one draw block (null prefix if not tabulated).
+RP_DEV DrawTable draw_table(const WaveParams &p, u32 block) {
+    if (p.owen_prefix && p.randomization == 3) {
+        u32 slot = block - p.draw_first;
+        if (slot >= p.draw_blocks)
+            slot = p.draw_first == 4u && block - 133u < p.draw_blocks ? p.draw_blocks + block - 133u : ~0u;
+        if (slot != ~0u)
+            return {p.owen_prefix + size_t(slot) * 4 * kOwenPrefixEntries, p.draw_bytes + size_t(slot) * kIndexBytes * 256,
+                    p.draw_hash + 4 * slot};
+    }
+    return {nullptr, nullptr, nullptr};
 }
 
 // shaders/render.metal:113-122
@@ -111,31 +116,54 @@ RP_DEV u32 zdraw(const DeviceScene &s, const WaveParams &p, u64 index, u32 dimen
     return zsobol_word(s.sobol, index, dimension, axis, pair, p.m, p.log_spp, p.randomization, p.seed_low);
 }
 
+// Words of a draw block that an event reads (x 1, y 2, z 4, w 8): the sets its callers use.
+// A word costs a radical inverse or up to 31 rounds of hashes, so those that the event does
+// not read are not computed; they are zero.
+enum : u32 { kDrawX = 1, kDrawXY = 3, kDrawYZ = 6, kDrawXYZ = 7, kDrawXW = 9, kDrawYZW = 14, kDrawAll = 15 };
+// kDrawXY and kDrawXYZ with this bit: of z only the top two bits are read (a decision against
+// 0xc0000000 of the Sobol samplers).
+constexpr u32 kDrawCoarseZ = 16;
+
 // shaders/render.metal:154-179 (independent and Sobol samplers); out of line, one copy per kernel
 __device__ __noinline__ uint4 draw_words(const DeviceScene &s, const WaveParams &p, u32 pixel, u32 slo, u32 shi,
-                                         u64 index, u32 block) {
+                                         u64 index, u32 block, u32 set = kDrawAll) {
     if (p.sampler == 0)
         return philox(make_uint4(pixel, slo, shi, block), p.seed_low, p.seed_high);
     const u32 d = 4 * block;
-    if (p.sampler == 2)
-        return make_uint4(float_bits(qmc_radical(s.primes, d, index, p.randomization, p.seed_low)),
-                          float_bits(qmc_radical(s.primes, d + 1, index, p.randomization, p.seed_low)),
-                          float_bits(qmc_radical(s.primes, d + 2, index, p.randomization, p.seed_low)),
-                          float_bits(qmc_radical(s.primes, d + 3, index, p.randomization, p.seed_low)));
-    if (p.sampler == 3) {
+    u32 v[4] = {0, 0, 0, 0};
+    if (p.sampler == 1) {
+        const DrawTable table = draw_table(p, block);
+        const u32 mode = p.randomization, seed = p.seed_low;
+        if (set == kDrawX)
+            sobol_words<-1, 0>(s.sobol, index, d, mode, seed, table, v);
+        else if (set == kDrawXY)
+            sobol_words<-1, 0, 1>(s.sobol, index, d, mode, seed, table, v);
+        else if (set == kDrawYZ)
+            sobol_words<-1, 1, 2>(s.sobol, index, d, mode, seed, table, v);
+        else if (set == kDrawXW)
+            sobol_words<-1, 0, 3>(s.sobol, index, d, mode, seed, table, v);
+        else if (set == (kDrawXYZ | kDrawCoarseZ))
+            sobol_words<2, 0, 1, 2>(s.sobol, index, d, mode, seed, table, v);
+        else if (set == kDrawXYZ)
+            sobol_words<-1, 0, 1, 2>(s.sobol, index, d, mode, seed, table, v);
+        else if (set == kDrawYZW)
+            sobol_words<-1, 1, 2, 3>(s.sobol, index, d, mode, seed, table, v);
+        else
+            sobol_words<-1, 0, 1, 2, 3>(s.sobol, index, d, mode, seed, table, v);
+    } else if (p.sampler == 2) {
+#pragma unroll 1
+        for (u32 k = 0; k < 4; ++k)
+            if (set >> k & 1u)
+                v[k] = float_bits(qmc_radical(s.primes, d + k, index, p.randomization, p.seed_low));
+    } else {
         const bool even = (block & 1) == 0;
-        return make_uint4(zdraw(s, p, index, d, 0, true), zdraw(s, p, index, d, 1, true),
-                          zdraw(s, p, index, d + 2, 0, even), zdraw(s, p, index, even ? d + 2 : d + 3, even ? 1 : 0, even));
+#pragma unroll 1
+        for (u32 k = 0; k < 4; ++k)
+            if (set >> k & 1u)
+                v[k] = k < 2 ? zdraw(s, p, index, d, k, true)
+                             : zdraw(s, p, index, k == 2 || even ? d + 2 : d + 3, k == 3 && even ? 1 : 0, even);
     }
-    return sobol_words4(s.sobol, index, 4 * block, p.randomization, p.seed_low, owen_prefix_table(p, block));
-}
-
-// The first word of draw_words (the block's first dimension) alone.
-__device__ __noinline__ u32 draw_word0(const DeviceScene &s, const WaveParams &p, u32 pixel, u32 slo, u32 shi,
-                                       u64 index, u32 block) {
-    if (p.sampler == 1)
-        return sobol_word_prefixed(s.sobol, index, 4 * block, p.randomization, p.seed_low, owen_prefix_table(p, block));
-    return draw_words(s, p, pixel, slo, shi, index, block).x;
+    return make_uint4(v[0], v[1], v[2], v[3]);
 }
 
 struct BeginSample {
@@ -471,27 +499,33 @@ RP_DEV float sigmoid_reflectance(const float *c, float w) {
     return 0.5f + 0.5f * copysignf(1.0f / sqrtf(1.0f + inverse * inverse), p);
 }
 // shaders/packet_walk.h:22-57 (sampled / constant / blackbody / RGB / image reflectance; image:
-// the reconstruction of the hit's filtered RGB)
-RP_DEV bool material_reflectance(const DeviceScene &s, const DMaterial &m, float w, const RgbPolynomial *image,
-                                 float &rho) {
-    if (m.scattering != 0) {
-        rho = 1;
-    } else if (m.kind == 3 && image && m.image_texture < s.img.texture_count) {
-        rho = rgb_polynomial_at(*image, w);
+// the reconstruction of the hit's filtered RGB) at four wavelengths
+__device__ __noinline__ float material_blackbody(float factor, float w) { return blackbody_reflectance(factor, w); }
+RP_DEV bool material_reflectance4(const DeviceScene &s, const DMaterial &m, V4 w, const RgbPolynomial *image,
+                                  float (&rho)[4]) {
+    if (m.kind == 3 && image && m.image_texture < s.img.texture_count) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            rho[k] = rgb_polynomial_at(*image, w.v[k]);
     } else if (m.kind == 0 && m.knot_count >= 2 && m.knot_begin <= s.knot_count &&
                m.knot_count <= s.knot_count - m.knot_begin) {
-        rho = pbrt_reflectance(s.knots + m.knot_begin, m.knot_count, w);
+        knot_values4(s.knots + m.knot_begin, m.knot_count, m.knot_range, false, w, rho);
     } else if (m.kind == 1) {
-        rho = m.scalar_value;
+        rho[0] = rho[1] = rho[2] = rho[3] = m.scalar_value;
     } else if (m.kind == 4) {
-        rho = blackbody_reflectance(m.scalar_value, w);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            rho[k] = material_blackbody(m.scalar_value, w.v[k]);
     } else if (m.kind == 2) {
-        rho = sigmoid_reflectance(m.coefficients, w);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            rho[k] = sigmoid_reflectance(m.coefficients, w.v[k]);
     } else
         return false;
-    return isfinite(rho) && rho >= 0 && rho <= 1;
+    return true;
 }
-// shaders/hero_current_bsdf.h:72-101 with prepare_scattering (shaders/render.metal:2079-2160)
+// shaders/hero_current_bsdf.h:72-101 with prepare_scattering (shaders/render.metal:2079-2160).
+// The four wavelengths are evaluated together, active or not, so that their loads overlap.
 template <int K>
 RP_DEV bool prepare_bsdf(const DeviceScene &s, const DMaterial &m, V4 lambda, u32 mask, HeroBsdf &out,
                          const RgbPolynomial *image = nullptr) {
@@ -513,32 +547,40 @@ RP_DEV bool prepare_bsdf(const DeviceScene &s, const DMaterial &m, V4 lambda, u3
             return false;
         prepare_roughness(u, v, m.remap != 0, false, out.g);
     }
+    if constexpr (K == 0) {
+        float rho[4];
+        if (!material_reflectance4(s, m, lambda, image, rho))
+            return (mask & 15u) == 0;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        if (!(mask & (1u << k)))
-            continue;
-        float rho;
-        if (!material_reflectance(s, m, lambda.v[k], image, rho))
-            return false;
-        if constexpr (K == 0) {
-            out.param[k] = rho;
-            continue;
-        }
-        const float eta = optical_value(s.knots, m.eta_begin, m.eta_count, s.knot_count, (m.optical_extensions & 1u) != 0,
-                                        lambda.v[k]);
-        const float kk = optical_value(s.knots, m.k_begin, m.k_count, s.knot_count, (m.optical_extensions & 2u) != 0,
-                                       lambda.v[k]);
-        if constexpr (K == 1) {
-            // shaders/conductor.h:22-25
-            if (!isfinite(eta) || !isfinite(kk) || eta < 0 || kk < 0 || (eta == 0 && kk == 0))
-                return false;
-            out.param[k] = eta;
-            out.k[k] = kk;
-        } else {
-            // shaders/dielectric.h:15-18
-            if (!isfinite(eta) || eta < 0)
-                return false;
-            out.param[k] = eta == 0 ? 1 : eta;
+        for (int k = 0; k < 4; ++k)
+            if (mask & (1u << k)) {
+                if (!isfinite(rho[k]) || !(rho[k] >= 0 && rho[k] <= 1))
+                    return false;
+                out.param[k] = rho[k];
+            }
+    } else {
+        float eta[4], kk[4];
+        optical_values4(s.knots, m.eta_begin, m.eta_count, s.knot_count, m.eta_range, (m.optical_extensions & 1u) != 0,
+                        lambda, eta);
+        if constexpr (K == 1)
+            optical_values4(s.knots, m.k_begin, m.k_count, s.knot_count, m.k_range, (m.optical_extensions & 2u) != 0,
+                            lambda, kk);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (!(mask & (1u << k)))
+                continue;
+            if constexpr (K == 1) {
+                // shaders/conductor.h:22-25
+                if (!isfinite(eta[k]) || !isfinite(kk[k]) || eta[k] < 0 || kk[k] < 0 || (eta[k] == 0 && kk[k] == 0))
+                    return false;
+                out.param[k] = eta[k];
+                out.k[k] = kk[k];
+            } else {
+                // shaders/dielectric.h:15-18
+                if (!isfinite(eta[k]) || eta[k] < 0)
+                    return false;
+                out.param[k] = eta[k] == 0 ? 1 : eta[k];
+            }
         }
     }
     return true;

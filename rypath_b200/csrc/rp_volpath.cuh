@@ -628,10 +628,10 @@ __device__ __noinline__ bool prepare_scalar_bsdf(const DeviceScene &s, const DMa
     const float u = m.u_roughness, v = m.v_roughness;
     if (!isfinite(u) || !isfinite(v) || u < 0 || v < 0)
         return false;
-    float eta = optical_value(s.knots, m.eta_begin, m.eta_count, s.knot_count, (m.optical_extensions & 1u) != 0, w);
+    float eta = optical_value(s.knots, m.eta_begin, m.eta_count, s.knot_count, m.eta_range, (m.optical_extensions & 1u) != 0, w);
     b.k = 0;
     if (m.scattering == 1) {
-        b.k = optical_value(s.knots, m.k_begin, m.k_count, s.knot_count, (m.optical_extensions & 2u) != 0, w);
+        b.k = optical_value(s.knots, m.k_begin, m.k_count, s.knot_count, m.k_range, (m.optical_extensions & 2u) != 0, w);
         if (!isfinite(eta) || !isfinite(b.k) || eta < 0 || b.k < 0 || (eta == 0 && b.k == 0))
             return false;
     } else {
@@ -910,7 +910,7 @@ RP_DEV int shade_event(const DeviceScene &s, const WaveParams &p, const ScalarPa
         rho = demo_reflectance(surface.reflectance, path.wavelength);
     } else if (surface.kind == 0 && surface.knot_count >= 2 && surface.knot_begin <= s.knot_count &&
                surface.knot_count <= s.knot_count - surface.knot_begin) {
-        rho = pbrt_reflectance(s.knots + surface.knot_begin, surface.knot_count, path.wavelength);
+        rho = knot_value(s.knots + surface.knot_begin, surface.knot_count, surface.knot_range, false, path.wavelength);
     } else if (surface.kind == 1) {
         rho = surface.scalar_value;
     } else if (surface.kind == 4) {
@@ -981,8 +981,10 @@ RP_DEV int shade_event(const DeviceScene &s, const WaveParams &p, const ScalarPa
         path.status = S_ARITHMETIC;
         return kEventFinished;
     }
-    const uint4 light_words = draw_words(s, p, path.pixel, path.slo, path.shi, path.index, 2 + 2 * bounce);
-    const uint4 bsdf_words = draw_words(s, p, path.pixel, path.slo, path.shi, path.index, 1 + 2 * bounce);
+    const uint4 light_words = draw_words(s, p, path.pixel, path.slo, path.shi, path.index, 2 + 2 * bounce, kDrawXYZ);
+    // the third word decides the roulette, from the third scattering on
+    const uint4 bsdf_words = draw_words(s, p, path.pixel, path.slo, path.shi, path.index, 1 + 2 * bounce,
+                                        path.scatterings >= 2 ? kDrawXYZ | kDrawCoarseZ : kDrawXY);
     // light sample: the demo model's sky sampled uniformly over the sphere with the
     // cosine-ratio weight (:709-781); PBRT scenes' lights with power-heuristic MIS (:783-835).
     // Dirac surfaces take no light sample.
