@@ -970,6 +970,7 @@ struct rp_scene {
     BuildTmp tmp{};
     u32 tree_levels = 0;     // most internal nodes on a root-to-leaf path of the LBVH
     u32 wide_levels = 0;     // levels of the compressed 8-wide traversal tree
+    u32 family_mask = 0;     // BSDF families of the scene's materials
     bool resolve = false;    // hero scene with pass-through or mix-root instances
     bool dielectrics = false; // a dielectric material: the QMC samplers' depth limit
     bool scalar_full = false; // conductors, dielectrics or procedural primitives: the full scalar step kernel
@@ -1382,75 +1383,85 @@ void launch_trace(const rp_scene *s, const PathPool &pool, int in, unsigned grid
         launch_trace_stack<Count, Block, kStackDepth>(s, pool, in, grid, st, limit);
 }
 template <bool Count, int Block, bool Adjoint, int Stack>
-void launch_shadow_stack(const rp_scene *s, const PathPool &pool, unsigned grid, size_t smem, cudaStream_t st,
+void launch_shadow_stack(const rp_scene *s, const PathPool &pool, int in, unsigned grid, size_t smem, cudaStream_t st,
                          u32 limit) {
     if (s->resolve)
-        k_shadow<Count, Block, Adjoint, Stack, true><<<grid, Block, smem, st>>>(s->ds, pool, limit);
+        k_shadow<Count, Block, Adjoint, Stack, true><<<grid, Block, smem, st>>>(s->ds, pool, in, limit);
     else
-        k_shadow<Count, Block, Adjoint, Stack, false><<<grid, Block, smem, st>>>(s->ds, pool, limit);
+        k_shadow<Count, Block, Adjoint, Stack, false><<<grid, Block, smem, st>>>(s->ds, pool, in, limit);
 }
 template <bool Count, int Block, bool Adjoint>
-void launch_shadow(const rp_scene *s, const PathPool &pool, unsigned grid, size_t smem, cudaStream_t st, u32 limit) {
+void launch_shadow(const rp_scene *s, const PathPool &pool, int in, unsigned grid, size_t smem, cudaStream_t st, u32 limit) {
     if (s->wide_levels <= u32(kShortStack))
-        launch_shadow_stack<Count, Block, Adjoint, kShortStack>(s, pool, grid, smem, st, limit);
+        launch_shadow_stack<Count, Block, Adjoint, kShortStack>(s, pool, in, grid, smem, st, limit);
     else
-        launch_shadow_stack<Count, Block, Adjoint, kStackDepth>(s, pool, grid, smem, st, limit);
+        launch_shadow_stack<Count, Block, Adjoint, kStackDepth>(s, pool, in, grid, smem, st, limit);
 }
 
-// The four shade kernels of one event (one per BSDF family), run side by side: family 0 on
-// the scene stream, families 1-3 on their own streams, joined back before the shadow walks.
-// Each reads only its own bin and appends to the path and shadow queues with atomics, so the
-// queue order may differ from a serial launch but no path's result does (every later kernel
-// reads a path by its id, and the film reduces by lane).
-template <bool Adjoint, bool Img>
-void launch_shade_img(rp_scene *s, const WaveParams &p, const PathPool &pool, int in, unsigned grid, size_t smem) {
+// The shade kernels of one event, one per BSDF family that the scene's materials have and the
+// escape kernel, run side by side: the first on the scene stream, the others on streams of
+// their own, joined back before the shadow walks.  Each reads only its own bin and appends to
+// the path and shadow queues with atomics, so the queue order may differ from a serial launch
+// but no path's result does (every later kernel reads a path by its id, and the film reduces
+// by lane).  A scene of one family keeps its escape kernel on the scene stream, before the
+// others: it is short, and a fork and a join cost more than it.
+constexpr int kShadeBlock = 256;
+template <int F, int Block, bool Adjoint, bool Img>
+void launch_family(rp_scene *s, const WaveParams &p, const PathPool &pool, int in, unsigned grid, size_t smem,
+                   cudaStream_t st) {
+    // counting runs time each family kernel alone: all run one after another on the scene
+    // stream, so each one's events bracket its own work (side by side they share the SMs)
+    if (s->counting)
+        s->mark_family(F, st);
+    k_shade<F, Block, Adjoint, Img><<<grid, Block, smem, st>>>(s->ds, p, pool, in);
+    if constexpr (F != 3)
+        k_nee<F, Block, Img><<<grid, Block, 0, st>>>(s->ds, p, pool, in);
+    if (s->counting)
+        s->done_family(st);
+}
+template <int Block, bool Adjoint, bool Img>
+void launch_families(rp_scene *s, const WaveParams &p, const PathPool &pool, int in, unsigned grid, size_t smem) {
+    const u32 mask = s->family_mask;
+    const bool fork = !s->counting && (mask & (mask - 1)) != 0;
+    if (!fork) {
+        launch_family<3, Block, Adjoint, Img>(s, p, pool, in, grid, smem, s->stream);
+        if (mask & 1u)
+            launch_family<0, Block, Adjoint, Img>(s, p, pool, in, grid, smem, s->stream);
+        if (mask & 2u)
+            launch_family<1, Block, Adjoint, Img>(s, p, pool, in, grid, smem, s->stream);
+        if (mask & 4u)
+            launch_family<2, Block, Adjoint, Img>(s, p, pool, in, grid, smem, s->stream);
+        return;
+    }
+    const bool used[3] = {(mask & 2u) != 0, (mask & 4u) != 0, true};
     RP_CHECK(cudaEventRecord(s->forked, s->stream));
     for (int k = 0; k < 3; ++k)
-        RP_CHECK(cudaStreamWaitEvent(s->family[k], s->forked, 0));
-    // counting runs time each family kernel alone: the four run one after another on the scene
-    // stream, so each one's events bracket its own work (side by side they share the SMs)
-    const bool timed = s->counting;
-    cudaStream_t on[4] = {s->stream, s->family[0], s->family[1], s->family[2]};
-    if (timed)
-        on[1] = on[2] = on[3] = s->stream;
-    if (timed)
-        s->mark_family(0, on[0]);
-    k_shade<0, 128, Adjoint, Img><<<grid, 128, smem, on[0]>>>(s->ds, p, pool, in);
-    k_nee<0, 128, Img><<<grid, 128, 0, on[0]>>>(s->ds, p, pool);
-    if (timed) {
-        s->done_family(on[0]);
-        s->mark_family(1, on[1]);
-    }
-    k_shade<1, 128, Adjoint, Img><<<grid, 128, smem, on[1]>>>(s->ds, p, pool, in);
-    k_nee<1, 128, Img><<<grid, 128, 0, on[1]>>>(s->ds, p, pool);
-    if (timed) {
-        s->done_family(on[1]);
-        s->mark_family(2, on[2]);
-    }
-    k_shade<2, 128, Adjoint, Img><<<grid, 128, smem, on[2]>>>(s->ds, p, pool, in);
-    k_nee<2, 128, Img><<<grid, 128, 0, on[2]>>>(s->ds, p, pool);
-    if (timed) {
-        s->done_family(on[2]);
-        s->mark_family(3, on[3]);
-    }
-    k_shade<3, 128, Adjoint, Img><<<grid, 128, smem, on[3]>>>(s->ds, p, pool, in);
-    if (timed)
-        s->done_family(on[3]);
-    for (int k = 0; k < 3; ++k) {
-        RP_CHECK(cudaEventRecord(s->family_done[k], s->family[k]));
-        RP_CHECK(cudaStreamWaitEvent(s->stream, s->family_done[k], 0));
-    }
+        if (used[k])
+            RP_CHECK(cudaStreamWaitEvent(s->family[k], s->forked, 0));
+    if (mask & 1u)
+        launch_family<0, Block, Adjoint, Img>(s, p, pool, in, grid, smem, s->stream);
+    if (mask & 2u)
+        launch_family<1, Block, Adjoint, Img>(s, p, pool, in, grid, smem, s->family[0]);
+    if (mask & 4u)
+        launch_family<2, Block, Adjoint, Img>(s, p, pool, in, grid, smem, s->family[1]);
+    launch_family<3, Block, Adjoint, Img>(s, p, pool, in, grid, smem, s->family[2]);
+    for (int k = 0; k < 3; ++k)
+        if (used[k]) {
+            RP_CHECK(cudaEventRecord(s->family_done[k], s->family[k]));
+            RP_CHECK(cudaStreamWaitEvent(s->stream, s->family_done[k], 0));
+        }
 }
+u32 family_kernels(const rp_scene *s) { return 2 * u32(__builtin_popcount(s->family_mask)) + 1; }
 // The plain shade kernels for scenes without images (the adjoint keeps the full ones).
-template <bool Adjoint>
+template <int Block, bool Adjoint>
 void launch_shade(rp_scene *s, const WaveParams &p, const PathPool &pool, int in, unsigned grid, size_t smem) {
     if constexpr (!Adjoint) {
         if (!s->ds.img.textured && s->ds.img.env_image == kNone) {
-            launch_shade_img<false, false>(s, p, pool, in, grid, smem);
+            launch_families<Block, false, false>(s, p, pool, in, grid, smem);
             return;
         }
     }
-    launch_shade_img<Adjoint, true>(s, p, pool, in, grid, smem);
+    launch_families<Block, Adjoint, true>(s, p, pool, in, grid, smem);
 }
 
 // Sobol sampler with Owen randomisation: attaches the tables of the draw blocks of the scene's
@@ -1519,16 +1530,14 @@ void run_wave(rp_scene *s, const WaveParams &request_params, size_t adjoint_smem
     pool.lane_shadow = s->counting ? s->lane_shadow : nullptr;
     const int sms = s->sm_count;
     s->mark(3);
-    RP_CHECK(cudaMemsetAsync(pool.counters, 0, 16 * sizeof(u32), s->stream));
+    RP_CHECK(cudaMemsetAsync(pool.counters, 0, 64 * sizeof(u32), s->stream));
     k_raygen<<<grid_for(sms, p.lanes, 256, 16), 256, 0, s->stream>>>(s->ds, p, pool);
-    RP_CHECK(cudaMemcpyAsync(pool.counters, &p.lanes, sizeof(u32), cudaMemcpyHostToDevice, s->stream));
     s->done();
     int in = 0;
     const u32 events = s->ds.max_depth + 1;
     bool shadow_pending = false;
     for (u32 e = 0; e < events; ++e) {
         s->mark(0);
-        RP_CHECK(cudaMemsetAsync(pool.counters + 4, 0, 4 * sizeof(u32), s->stream));
         const unsigned trace_grid = grid_for(sms, p.lanes, kTraceBlock, 12);
         if (s->counting)
             launch_trace<true, kTraceBlock>(s, pool, in, trace_grid, s->stream, p.boundary_limit);
@@ -1539,26 +1548,23 @@ void run_wave(rp_scene *s, const WaveParams &request_params, size_t adjoint_smem
             RP_CHECK(cudaStreamWaitEvent(s->stream, s->joined, 0));
             shadow_pending = false;
         }
-        s->mark(2, 7);
-        RP_CHECK(cudaMemsetAsync(pool.counters + (in ^ 1), 0, sizeof(u32), s->stream));
-        RP_CHECK(cudaMemsetAsync(pool.counters + 2, 0, sizeof(u32), s->stream));
-        RP_CHECK(cudaMemsetAsync(pool.counters + 8, 0, 3 * sizeof(u32), s->stream));
+        s->mark(2, int(family_kernels(s)));
         const size_t smem = adjoint_smem;
-        const unsigned shade_grid = grid_for(sms, p.lanes, 128, 16);
+        const unsigned shade_grid = grid_for(sms, p.lanes, kShadeBlock, 2048 / kShadeBlock);
         if (pool.hist)
-            launch_shade<true>(s, p, pool, in, shade_grid, smem);
+            launch_shade<kShadeBlock, true>(s, p, pool, in, shade_grid, smem);
         else
-            launch_shade<false>(s, p, pool, in, shade_grid, 0);
+            launch_shade<kShadeBlock, false>(s, p, pool, in, shade_grid, 0);
         s->done();
         RP_CHECK(cudaEventRecord(s->forked, s->stream));
         RP_CHECK(cudaStreamWaitEvent(s->side, s->forked, 0));
         s->mark(1, 1, s->side);
         if (pool.hist)
-            launch_shadow<false, kTraceBlock, true>(s, pool, trace_grid, smem, s->side, p.boundary_limit);
+            launch_shadow<false, kTraceBlock, true>(s, pool, in, trace_grid, smem, s->side, p.boundary_limit);
         else if (s->counting)
-            launch_shadow<true, kTraceBlock, false>(s, pool, trace_grid, 0, s->side, p.boundary_limit);
+            launch_shadow<true, kTraceBlock, false>(s, pool, in, trace_grid, 0, s->side, p.boundary_limit);
         else
-            launch_shadow<false, kTraceBlock, false>(s, pool, trace_grid, 0, s->side, p.boundary_limit);
+            launch_shadow<false, kTraceBlock, false>(s, pool, in, trace_grid, 0, s->side, p.boundary_limit);
         s->done(s->side);
         RP_CHECK(cudaEventRecord(s->joined, s->side));
         shadow_pending = true;
@@ -2179,6 +2185,9 @@ rp_status rp_cuda_scene_create(const rp_scene_desc *d, int device, rp_scene **ou
                        uniform_knots(d, m.knot_begin, m.knot_count), uniform_knots(d, m.eta_begin, m.eta_count),
                        uniform_knots(d, m.k_begin, m.k_count)};
         }
+        for (const DMaterial &m : mats)
+            if (m.scattering < 3)
+                s->family_mask |= 1u << m.scattering;
         ds.materials = dupload(own, mats.data(), mats.size(), stm);
         ds.material_count = d->material_count;
         const u32 all_prims = next_prim + patch_prims + analytic_prims;
@@ -3041,7 +3050,7 @@ void batch_wave_kernels(rp_scene *s, const WaveParams &p, const Batch &b, u32 wa
     PathPool &pool = s->pool;
     const int sms = s->sm_count;
     cudaStream_t st = s->stream;
-    RP_CHECK(cudaMemsetAsync(pool.counters, 0, 16 * sizeof(u32), st));
+    RP_CHECK(cudaMemsetAsync(pool.counters, 0, 64 * sizeof(u32), st));
     k_raygen_views<<<grid_for(sms, wave_lanes, 256, 16), 256, 0, st>>>(s->ds, p, b, pool);
     const int trace_grid = grid_for(sms, wave_lanes, TB, int(blocks_per_sm * 128 / TB));
     const int shade_grid = grid_for(sms, wave_lanes, SB, int(blocks_per_sm * 128 / SB));
@@ -3051,32 +3060,15 @@ void batch_wave_kernels(rp_scene *s, const WaveParams &p, const Batch &b, u32 wa
     int in = 0;
     bool shadow_pending = false;
     for (u32 e = 0; e <= s->ds.max_depth; ++e) {
-        RP_CHECK(cudaMemsetAsync(pool.counters + 4, 0, 4 * sizeof(u32), st));
         launch_trace<false, TB>(s, pool, in, trace_grid, st, p.boundary_limit);
         if (shadow_pending) {
             RP_CHECK(cudaStreamWaitEvent(st, s->joined, 0));
             shadow_pending = false;
         }
-        RP_CHECK(cudaMemsetAsync(pool.counters + (in ^ 1), 0, sizeof(u32), st));
-        RP_CHECK(cudaMemsetAsync(pool.counters + 2, 0, sizeof(u32), st));
-        RP_CHECK(cudaMemsetAsync(pool.counters + 8, 0, 3 * sizeof(u32), st));
-        RP_CHECK(cudaEventRecord(s->forked, st));
-        for (int k = 0; k < 3; ++k)
-            RP_CHECK(cudaStreamWaitEvent(s->family[k], s->forked, 0));
-        k_shade<0, SB><<<shade_grid, SB, 0, st>>>(s->ds, p, pool, in);
-        k_nee<0, SB><<<shade_grid, SB, 0, st>>>(s->ds, p, pool);
-        k_shade<1, SB><<<shade_grid, SB, 0, s->family[0]>>>(s->ds, p, pool, in);
-        k_nee<1, SB><<<shade_grid, SB, 0, s->family[0]>>>(s->ds, p, pool);
-        k_shade<2, SB><<<shade_grid, SB, 0, s->family[1]>>>(s->ds, p, pool, in);
-        k_nee<2, SB><<<shade_grid, SB, 0, s->family[1]>>>(s->ds, p, pool);
-        k_shade<3, SB><<<shade_grid, SB, 0, s->family[2]>>>(s->ds, p, pool, in);
-        for (int k = 0; k < 3; ++k) {
-            RP_CHECK(cudaEventRecord(s->family_done[k], s->family[k]));
-            RP_CHECK(cudaStreamWaitEvent(st, s->family_done[k], 0));
-        }
+        launch_shade<SB, false>(s, p, pool, in, shade_grid, 0);
         RP_CHECK(cudaEventRecord(s->forked, st));
         RP_CHECK(cudaStreamWaitEvent(s->side, s->forked, 0));
-        launch_shadow<false, TB, false>(s, pool, trace_grid, 0, s->side, p.boundary_limit);
+        launch_shadow<false, TB, false>(s, pool, in, trace_grid, 0, s->side, p.boundary_limit);
         RP_CHECK(cudaEventRecord(s->joined, s->side));
         shadow_pending = true;
         in ^= 1;
@@ -3949,8 +3941,6 @@ PathPool static_pool(unsigned char *base, u32 lanes, unsigned long long *stats) 
     return q;
 }
 
-__global__ void k_static_set_lanes(u32 *counter, u32 lanes) { *counter = lanes; }
-
 } // namespace
 
 extern "C" {
@@ -3996,23 +3986,24 @@ rp_status rp_cuda_sample_device_static(rp_scene *s, const rp_request *request, r
         // counters start at zero on every call; every other array is written before it is read
         RP_CHECK(cudaMemsetAsync(pool.counters, 0, 256, st));
         k_raygen<<<grid_for(sms, p.lanes, 256, 16), 256, 0, st>>>(s->ds, p, pool);
-        k_static_set_lanes<<<1, 1, 0, st>>>(pool.counters, p.lanes);
         int in = 0;
         for (u32 ev = 0; ev < s->ds.max_depth + 1; ++ev) {
-            RP_CHECK(cudaMemsetAsync(pool.counters + 4, 0, 4 * sizeof(u32), st));
             launch_trace<false, kTraceBlock>(s, pool, in, grid_for(sms, p.lanes, kTraceBlock, 12), st, p.boundary_limit);
-            RP_CHECK(cudaMemsetAsync(pool.counters + (in ^ 1), 0, sizeof(u32), st));
-            RP_CHECK(cudaMemsetAsync(pool.counters + 2, 0, sizeof(u32), st));
-            RP_CHECK(cudaMemsetAsync(pool.counters + 8, 0, 3 * sizeof(u32), st));
             const unsigned shade_grid = grid_for(sms, p.lanes, 128, 16);
-            k_shade<0><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in);
-            k_nee<0><<<shade_grid, 128, 0, st>>>(s->ds, p, pool);
-            k_shade<1><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in);
-            k_nee<1><<<shade_grid, 128, 0, st>>>(s->ds, p, pool);
-            k_shade<2><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in);
-            k_nee<2><<<shade_grid, 128, 0, st>>>(s->ds, p, pool);
             k_shade<3><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in);
-            launch_shadow<false, kTraceBlock, false>(s, pool, grid_for(sms, p.lanes, kTraceBlock, 12), 0, st, p.boundary_limit);
+            if (s->family_mask & 1u) {
+                k_shade<0><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in);
+                k_nee<0><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in);
+            }
+            if (s->family_mask & 2u) {
+                k_shade<1><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in);
+                k_nee<1><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in);
+            }
+            if (s->family_mask & 4u) {
+                k_shade<2><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in);
+                k_nee<2><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in);
+            }
+            launch_shadow<false, kTraceBlock, false>(s, pool, in, grid_for(sms, p.lanes, kTraceBlock, 12), 0, st, p.boundary_limit);
             in ^= 1;
         }
         k_results<<<grid_for(sms, p.lanes, 256, 16), 256, 0, st>>>(pool, p.lanes, s->ds.filter_weight,

@@ -58,6 +58,8 @@ RP_DEV void raygen_lane(const DeviceScene &s, const RasterCam &cam, const WavePa
 }
 __global__ void k_raygen(const __grid_constant__ DeviceScene s, const __grid_constant__ WaveParams p, PathPool pool) {
     const RasterCam cam{s.origin, s.forward, s.right, s.up};
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        pool.counters[0] = p.lanes;
     for (u32 lane = blockIdx.x * blockDim.x + threadIdx.x; lane < p.lanes; lane += gridDim.x * blockDim.x)
         raygen_lane(s, cam, p, lane, lane, pool);
 }
@@ -140,12 +142,15 @@ __device__ __noinline__ u32 resolve_hit(const DeviceScene &s, const PathPool &po
 // shade stage runs one specialised kernel per family ("material-sorted shading").
 // Stack: traversal stack entries per thread (kShortStack for shallow trees, whose walks then
 // fit eight 128-thread blocks per SM).
-// Resolve: the scene has pass-through or mix-root instances (resolve_hit).
+// Resolve: the scene has pass-through, mix-root or procedural instances (resolve_hit).
 template <bool Count, int Block = kTraceBlock, int Stack = kStackDepth, bool Resolve = false>
 __global__ void __launch_bounds__(Block, Stack <= kShortStack ? 1024 / Block : 1)
     k_trace(const __grid_constant__ DeviceScene s, PathPool pool, int in, u32 boundary_limit) {
     __shared__ uint2 stack[Stack * Block];
     const u32 count = pool.counters[in];
+    u32 *event = pool.event(in);
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        pool.counters[in ^ 1] = 0;
     const u32 *queue = pool.queue[in];
     u32 nodes = 0, tris = 0, rays = 0;
     const u32 stride = gridDim.x * blockDim.x;
@@ -161,8 +166,8 @@ __global__ void __launch_bounds__(Block, Stack <= kShortStack ? 1024 / Block : 1
                 const u32 walks_before = rays;
                 Hit h;
                 const bool ok = walk_closest<Count, Stack, Resolve>(s, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z),
-                                                           __int_as_float(0x7f800000), h, stack + threadIdx.x, Block,
-                                                           nodes, tris);
+                                                                    __int_as_float(0x7f800000), h, stack + threadIdx.x,
+                                                                    Block, nodes, tris);
                 ++rays;
                 u32 prim = ok ? h.prim : kHitInvalid;
                 family = (!ok || h.prim == kNone) ? 3u : u32(__ldg(s.tri_family + h.prim));
@@ -178,7 +183,7 @@ __global__ void __launch_bounds__(Block, Stack <= kShortStack ? 1024 / Block : 1
         const int leader = __ffs(peers) - 1;
         u32 base = 0;
         if (lane == leader && family < 4)
-            base = atomicAdd(pool.counters + 4 + family, __popc(peers));
+            base = atomicAdd(event + kBinCount + family, __popc(peers));
         base = __shfl_sync(0xffffffffu, base, leader);
         if (family < 4)
             pool.bins[size_t(family) * pool.bin_capacity + base + __popc(peers & ((1u << lane) - 1))] = path;
@@ -190,8 +195,370 @@ __global__ void __launch_bounds__(Block, Stack <= kShortStack ? 1024 / Block : 1
     }
 }
 
-// One hero event after its closest hit (shaders/packet_pt_event_body.inc:11-461), for the paths
-// whose hit is of BSDF family F (3: no surface -- environment or a failed query).
+// The warps of a block meet between two phases of a long straight run of code, so that a line of
+// instructions fetched for one serves them all: the shade kernels run five thousand
+// instructions an event once each, and their warps, left to drift apart, spend a third to half
+// of their cycles waiting for instructions.
+template <bool Sync> RP_DEV void phase() {
+    if (Sync)
+        __syncthreads();
+}
+// One hero event of path `path` after its closest hit (shaders/packet_pt_event_body.inc:11-461),
+// a hit of BSDF family F (3: no surface -- environment or a failed query).  keep: the path
+// goes on; nee: its event left a light-sample request.  Sync: the whole block calls this
+// (`active` clear where it has no path), and its warps meet between the phases of the event.
+template <int F, bool Adjoint, bool Img, bool Sync>
+RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool &pool, bool active, u32 path, float *sgrad,
+                       bool &keep, bool &nee) {
+    const u32 capacity = s.max_depth + 2;
+    uint4 ident = pool.ident[path];
+    u32 flags = ident.w;
+    active = active && !(flags & F_COMPLETE);
+    {
+        uint4 cursor = pool.cursor[path];
+        const u64 index = (u64(cursor.y) << 32) | cursor.x;
+        u32 cnt = cursor.z;
+        const V4 lambda = from_float4(pool.lambda[path]);
+        V4 beta = from_float4(pool.beta[path]);
+        V4 radiance = from_float4(pool.radiance[path]);
+        Density density = load_density(pool.dens_f[path], pool.dens_e[path]);
+        const Density previous_density = load_density(pool.prev_f[path], pool.prev_e[path]);
+        Density hero_previous = previous_density;
+        V4 eta_scale = from_float4(pool.eta_scale[path]);
+        bool roulette = (flags & F_ROULETTE) != 0;
+        u32 active_mask = flags & F_MASK;
+        const float4 ro4 = pool.ray_o[path], rd4 = pool.ray_d[path];
+        V3 ro = v3(ro4.x, ro4.y, ro4.z), rd = v3(rd4.x, rd4.y, rd4.z);
+        const float4 hit = pool.hit[path];
+        u32 status = get_status(flags);
+        Density direct_density = density;
+        V4 direct_beta = beta;
+        bool direct_allowed = true;
+        const u32 old_count = cnt;
+        bool terminated = true;
+        // current vertex
+        u32 ctype = kSurface, cinst = kNone, clocal = 0, clight = kNone, cmat = kNone;
+        SurfacePoint cp;
+        cp.position = cp.error = cp.geometric_normal = cp.shading_normal = v3(0, 0, 0);
+        cp.inverse_area_pdf = 0;
+        Frame cframe;
+        HeroBsdf cbsdf;
+        cbsdf.kind = 0;
+        cbsdf.active_mask = active_mask;
+        cbsdf.g = {0, 0, true};
+        V4 cbeta = beta;
+        V3 cwo = v3(0, 0, 0), swo = v3(0, 0, 0);
+        bool cdelta = false, connectible = false;
+        bool go = false; // the event goes on to its next phase
+        if (active) do {
+            if (cnt >= capacity || !nonzero4(beta))
+                break;
+            if (!finite3(ro) || !finite3(rd) || !finite_nonnegative4(beta)) {
+                status = 2;
+                break;
+            }
+            const u32 prim = __float_as_uint(hit.w);
+            if (prim >= kHitArithmetic && prim != kNone) {
+                status = prim == kHitInvalid ? 3u : prim == kHitExhausted ? 4u : 2u;
+                break;
+            }
+            if (prim == kNone) {
+                ctype = kEnvironment;
+                clight = s.environment_light;
+                cp.position = ro + rd;
+                cp.geometric_normal = -rd;
+                cp.shading_normal = -rd;
+                cwo = -rd;
+                cbeta = beta;
+                connectible = true;
+                ++cnt;
+                break;
+            }
+            if constexpr (F == 3) {
+                status = 3; // a surface hit never reaches the no-surface bin
+                break;
+            } else {
+                const float t = hit.x, b1 = hit.y, b2 = hit.z;
+                if (!isfinite(t) || t < 0 || !isfinite(b1) || !isfinite(b2) || prim >= s.prim_count) {
+                    status = 3;
+                    break;
+                }
+                cinst = s.tri_instance[prim];
+                clocal = s.tri_local[prim];
+                const DInstance &instance = s.instances[cinst];
+                if (instance.material >= s.material_count) {
+                    status = 3;
+                    break;
+                }
+                // a mix root's hit was resolved by the closest-hit kernel
+                cmat = (instance.resolve & kMixRoot) ? pool.material[path] : instance.material;
+                ctype = kSurface;
+                clight = instance.emission == kNone ? kNone : instance.emitter_begin + clocal;
+                cwo = -rd;
+                if (!hit_surface_point(s, prim, cinst, clocal, b1, b2, cp)) {
+                    status = 2;
+                    break;
+                }
+                const DMaterial material = s.materials[cmat];
+                // an image reflectance reads its texture at the hit's footprint
+                // (shaders/packet_pt_event_body.inc:147-163, packet_walk.h:39-49)
+                RgbPolynomial image_rgb;
+                bool image = false;
+                if constexpr (F == 0) {
+                    if (Img && s.img.textured && material.kind == 3 && material.image_texture < s.img.texture_count) {
+                        F2 st, dstdx, dstdy;
+                        if (!texture_context(s, p, ident.x, ident.y, ident.z, cinst, clocal, b1, b2,
+                                             cp.geometric_normal, rd, cnt - 1, st, dstdx, dstdy)) {
+                            status = 2;
+                            break;
+                        }
+                        image_rgb = rgb_polynomial(
+                            s.img.rgb_table, image_reflectance_rgb(s.img, material.image_texture, st, dstdx, dstdy));
+                        image = true;
+                    }
+                }
+                if (!shading_frame(cp.shading_normal, cframe) ||
+                    !prepare_bsdf<F>(s, material, lambda, active_mask, cbsdf, image ? &image_rgb : nullptr)) {
+                    status = 2;
+                    break;
+                }
+                V3 ray_position, ray_error;
+                ray_point(ro, rd, t, cp.curved, ray_position, ray_error);
+                cp.error = cp.error + (vabs(cp.position - ray_position) + ray_error);
+                if (!finite3(cp.error)) {
+                    status = 2;
+                    break;
+                }
+                cbeta = beta;
+                connectible = hero_connectible(cbsdf);
+                ++cnt;
+                if (cnt == capacity)
+                    break;
+                if (cnt - 2 >= p.emergency_limit) {
+                    status = 1;
+                    break;
+                }
+                go = true;
+            }
+        } while (false);
+        if constexpr (F != 3) {
+            phase<Sync>();
+            uint4 draws;
+            if (go) {
+                // only a dielectric reads the lobe word, a smooth one only that of the
+                // three, and the first event no roulette word
+                const bool survival = roulette && cnt > 2;
+                const u32 set = F == 2 ? (cbsdf.g.smooth ? (survival ? kDrawXW : kDrawX) : kDrawAll)
+                                       : (survival ? kDrawYZW : kDrawYZ);
+                draws = draw_words(s, p, ident.x, ident.y, ident.z, index, 4 + cnt - 2, set);
+                swo = to_local(cframe, cwo);
+                cbsdf.active_mask = active_mask;
+                direct_density = density;
+                direct_allowed = hero_continue(beta, eta_scale, roulette, cnt - 1, sample_uniform(p, draws.w));
+                direct_beta = beta;
+                connectible = hero_connectible(cbsdf);
+                go = direct_allowed;
+            }
+            phase<Sync>();
+            if (go) do {
+                const HeroSample proposed = hero_sample_k<F>(cbsdf, swo, sample_uniform(p, draws.x),
+                                                        sample_uniform(p, draws.y), sample_uniform(p, draws.z));
+                bool cont_valid = proposed.valid;
+                if (proposed.valid && proposed.accepted) {
+                    hero_previous = direct_density;
+                    const Update adv = advance(direct_density, beta, proposed.numerator, proposed.pdf);
+                    cont_valid = adv.valid;
+                    if (adv.valid) {
+                        beta = adv.beta;
+                        density = adv.density;
+                    }
+                    hero_account_eta(eta_scale, roulette, proposed.eta, proposed.transmission);
+                    active_mask = 1;
+    #pragma unroll
+                    for (int k = 1; k < 4; ++k)
+                        if (density.lane[k].fraction > 0 || (fbits(beta.v[k]) & 0x7fffffffu))
+                            active_mask |= 1u << k;
+                }
+                if (!cont_valid) {
+                    status = 2;
+                    break;
+                }
+                if (!proposed.accepted)
+                    break;
+                V3 wi = to_world(cframe, proposed.wi);
+                if (!unit_vector(wi, wi)) {
+                    status = 2;
+                    break;
+                }
+                if (!finite_nonnegative4(beta)) {
+                    status = 2;
+                    break;
+                }
+                if (proposed.delta)
+                    cdelta = true;
+                const V3 origin = offset_point(cp.position, cp.error, cp.geometric_normal, wi);
+                if (!finite3(origin)) {
+                    status = 2;
+                    break;
+                }
+                ro = origin;
+                rd = wi;
+                terminated = false;
+            } while (false);
+        }
+        phase<Sync>();
+        bool complete = terminated || status != 0 || cnt >= capacity || !nonzero4(beta);
+        // latest vertex (the previous event's) for MIS
+        const float4 lp4 = pool.latest_p[path], ln4 = pool.latest_n[path];
+        Latest latest;
+        latest.type = (flags >> F_LTYPE_SHIFT) & 3u;
+        latest.kind = (flags >> F_LKIND_SHIFT) & 3u;
+        latest.mask = (flags >> F_LMASK_SHIFT) & 15u;
+        latest.delta = (flags & F_LDELTA) != 0;
+        latest.smooth = (flags & F_LSMOOTH) != 0;
+        latest.position = v3(lp4.x, lp4.y, lp4.z);
+        latest.shading_normal = v3(ln4.x, ln4.y, ln4.z);
+        latest.alpha_x = lp4.w;
+        latest.alpha_y = ln4.w;
+        if (cnt != old_count && status == 0) {
+            // hero_endpoint (shaders/hero_pt_helpers.h:157-184)
+            V4 rad = v4(0);
+            bool emission_ok = true;
+            if (ctype == kEnvironment) {
+                if (Img && s.img.env_image != kNone) {
+                    rad = environment_image_radiance4(s.img, rd, lambda);
+                } else if (s.environment != kNone) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        rad.v[k] = spectrum(s, s.environment, lambda.v[k]);
+                }
+                emission_ok = finite_nonnegative4(rad);
+            } else {
+                const V3 delta = latest.position - cp.position;
+                const DInstance &instance = s.instances[cinst];
+                if (!zero3(delta) && instance.emission != kNone) {
+                    const V3 dir = normalize3(delta);
+                    if (s.emission_two_sided[instance.emission] || dot(cp.geometric_normal, dir) > 0) {
+                        const u32 off = instance.emission * 471u;
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            rad.v[k] = cp.inverse_area_pdf == 0 ? 0.f : spectrum(s, off, lambda.v[k]);
+                        emission_ok = finite_nonnegative4(rad);
+                    }
+                }
+            }
+            V4 endpoint = v4(0);
+            if (!emission_ok) {
+                status = 2;
+            } else {
+                const V4 value = mul4(cbeta, rad);
+                if (cnt <= 2 || latest.delta || !nonzero4(value)) {
+                    endpoint = value;
+                } else {
+                    latest.param = from_float4(pool.latest_param[path]);
+                    latest.k = from_float4(pool.latest_k[path]);
+                    const float4 pre = pool.preceding[path];
+                    bool ok;
+                    const V4 bsdf_pdf = represented_pdf<-1>(latest_bsdf(latest), latest.shading_normal, latest.position,
+                                                        v3(pre.x, pre.y, pre.z), ctype == kEnvironment,
+                                                        ctype == kEnvironment ? rd : cp.position, ok);
+                    // hero_history_light_pdf / direct_pdf (shaders/packet_transport.h:740-758)
+                    float lpdf = 0;
+                    const float selection = light_pmf(s, latest.position, latest.shading_normal, clight);
+                    if (ctype == kEnvironment) {
+                        // the constant environment has no unidirectional proposal;
+                        // the image's is its compensated table
+                        lpdf = (Img && s.img.env_image != kNone) ? environment_image_pdf(s.img, rd, true) * selection
+                                                        : 0.0f * selection;
+                    } else {
+                        const V3 dl = cp.position - latest.position;
+                        if (dot(dl, dl) > 0 && nonzero3(cp.geometric_normal) && clight < s.emitter_count)
+                            lpdf = selection * light_geometry_pdf(s, clight, latest.position,
+                                                                  latest.shading_normal, cp);
+                    }
+                    if (!ok || !hero_weight(previous_density, value, ok ? bsdf_pdf : v4(__int_as_float(0x7fffffff)),
+                                            v4(lpdf), endpoint))
+                        status = 2;
+                }
+            }
+            radiance = add4(radiance, endpoint);
+            if (Adjoint) {
+                // replay: the emission's gradient over the vertices before this one,
+                // then this diffuse vertex joins the history of what follows it
+                uint4 h = pool.hist[path];
+                if (status == 0 && nonzero4(endpoint))
+                    adjoint_accumulate(s, pool, sgrad, h, lambda, endpoint, pool.adj_w[path]);
+                if (F == 0 && ctype == kSurface && status == 0) {
+                    const u32 m = cmat;
+                    if (__ldg(pool.adj_slot + m) != kNone) {
+                        h = history_push(h, m);
+                        pool.hist[path] = h;
+                    }
+                }
+            }
+            // hero_direct (shaders/hero_pt_helpers.h:185-221) runs in the light-sample kernel
+            // (k_nee), from the request this event leaves (write_nee_request); its failures fail the
+            // path there.
+            nee = F != 3 && status == 0 && cnt < capacity && direct_allowed && ctype == kSurface && connectible;
+            if (!finite_nonnegative4(radiance))
+                status = 2;
+            if (status != 0) {
+                complete = true;
+                nee = false;
+            }
+            if (nee) {
+                Density dd = direct_density;
+                write_nee_request(pool, path, cnt, cp, cbsdf, cwo, latest.position, direct_beta, dd);
+            }
+        }
+        phase<Sync>();
+        if (!active)
+            return;
+        // A complete path is read again only for its identity, status and radiance (the
+        // shadow walk, the film and the packet results), so the rest of its state is not
+        // written back.
+        if (cnt != old_count) {
+            // preceding = latest; latest = current (shaders/packet_pt_event_body.inc:453-460)
+            flags = (flags & ~(3u << F_PTYPE_SHIFT)) | (latest.type << F_PTYPE_SHIFT);
+            if (!complete) {
+                pool.preceding[path] = make_float4(latest.position.x, latest.position.y, latest.position.z, 0);
+                pool.latest_p[path] =
+                    make_float4(cp.position.x, cp.position.y, cp.position.z, cbsdf.g.alpha_x);
+                pool.latest_n[path] =
+                    make_float4(cp.shading_normal.x, cp.shading_normal.y, cp.shading_normal.z, cbsdf.g.alpha_y);
+                pool.latest_param[path] =
+                    make_float4(cbsdf.param[0], cbsdf.param[1], cbsdf.param[2], cbsdf.param[3]);
+                pool.latest_k[path] = make_float4(cbsdf.k[0], cbsdf.k[1], cbsdf.k[2], cbsdf.k[3]);
+            }
+            flags &= ~((3u << F_LTYPE_SHIFT) | F_LDELTA | (3u << F_LKIND_SHIFT) | (15u << F_LMASK_SHIFT) | F_LSMOOTH);
+            flags |= (ctype << F_LTYPE_SHIFT) | (cdelta ? F_LDELTA : 0u) | ((cbsdf.kind & 3u) << F_LKIND_SHIFT) |
+                     ((cbsdf.active_mask & 15u) << F_LMASK_SHIFT) | (cbsdf.g.smooth ? F_LSMOOTH : 0u);
+        }
+        flags = (flags & ~(F_MASK | F_ROULETTE)) | active_mask | (roulette ? F_ROULETTE : 0u);
+        flags = set_status(flags, status) | (complete ? F_COMPLETE : 0u);
+        ident.w = flags;
+        pool.ident[path] = ident;
+        pool.radiance[path] = to_float4(radiance);
+        if (!complete) {
+            cursor.z = cnt;
+            pool.cursor[path] = cursor;
+            pool.beta[path] = to_float4(beta);
+            float4 f;
+            int4 e;
+            store_density(density, f, e);
+            pool.dens_f[path] = f;
+            pool.dens_e[path] = e;
+            store_density(hero_previous, f, e);
+            pool.prev_f[path] = f;
+            pool.prev_e[path] = e;
+            pool.eta_scale[path] = to_float4(eta_scale);
+            pool.ray_o[path] = make_float4(ro.x, ro.y, ro.z, 0);
+            pool.ray_d[path] = make_float4(rd.x, rd.y, rd.z, 0);
+        }
+        keep = !complete;
+    }
+}
+// shade_path of the paths in the bin of family F.
 // Adjoint: the path-replay adjoint hooks are compiled in (the plain forward kernel carries none
 // of their registers).  The minimum of 512 resident threads per SM caps registers at 128, so
 // four 128-thread blocks fit an SM; the escape kernel (F = 3) fits without spilling, the
@@ -205,11 +572,13 @@ __global__ void __launch_bounds__(Block, 512 / Block) k_shade(const __grid_const
     extern __shared__ float sgrad[]; // adjoint only
     if (Adjoint)
         adjoint_begin(pool, sgrad);
-    const u32 count = pool.counters[4 + F];
+    u32 *event = pool.event(in);
+    if (F == 3 && blockIdx.x == 0 && threadIdx.x < kEventCounters)
+        pool.event(in ^ 1)[threadIdx.x] = 0;
+    const u32 count = event[kBinCount + F];
     const u32 *queue = pool.bins + size_t(F) * pool.bin_capacity;
     u32 *out_queue = pool.queue[in ^ 1];
     u32 *out_count = pool.counters + (in ^ 1);
-    const u32 capacity = s.max_depth + 2;
     // uniform trip count so warp-level appends see every lane of the warp
     const u32 stride = gridDim.x * blockDim.x;
     const u32 trips = (count + stride - 1) / stride;
@@ -217,346 +586,15 @@ __global__ void __launch_bounds__(Block, 512 / Block) k_shade(const __grid_const
         const u32 i = trip * stride + blockIdx.x * blockDim.x + threadIdx.x;
         bool keep = false, nee = false;
         u32 path = 0;
-        if (i < count) {
+        const bool active = i < count;
+        if (active)
             path = queue[i];
-            uint4 ident = pool.ident[path];
-            u32 flags = ident.w;
-            if (!(flags & F_COMPLETE)) {
-                uint4 cursor = pool.cursor[path];
-                const u64 index = (u64(cursor.y) << 32) | cursor.x;
-                u32 cnt = cursor.z;
-                const V4 lambda = from_float4(pool.lambda[path]);
-                V4 beta = from_float4(pool.beta[path]);
-                V4 radiance = from_float4(pool.radiance[path]);
-                Density density = load_density(pool.dens_f[path], pool.dens_e[path]);
-                const Density previous_density = load_density(pool.prev_f[path], pool.prev_e[path]);
-                Density hero_previous = previous_density;
-                V4 eta_scale = from_float4(pool.eta_scale[path]);
-                bool roulette = (flags & F_ROULETTE) != 0;
-                u32 active_mask = flags & F_MASK;
-                const float4 ro4 = pool.ray_o[path], rd4 = pool.ray_d[path];
-                V3 ro = v3(ro4.x, ro4.y, ro4.z), rd = v3(rd4.x, rd4.y, rd4.z);
-                const float4 hit = pool.hit[path];
-                u32 status = get_status(flags);
-                Density direct_density = density;
-                V4 direct_beta = beta;
-                bool direct_allowed = true;
-                const u32 old_count = cnt;
-                bool terminated = true;
-                // current vertex
-                u32 ctype = kSurface, cinst = kNone, clocal = 0, clight = kNone, cmat = kNone;
-                SurfacePoint cp;
-                cp.position = cp.error = cp.geometric_normal = cp.shading_normal = v3(0, 0, 0);
-                cp.inverse_area_pdf = 0;
-                Frame cframe;
-                HeroBsdf cbsdf;
-                cbsdf.kind = 0;
-                cbsdf.active_mask = active_mask;
-                cbsdf.g = {0, 0, true};
-                V4 cbeta = beta;
-                V3 cwo = v3(0, 0, 0), swo = v3(0, 0, 0);
-                bool pair_valid = false, cdelta = false, connectible = false;
-                do {
-                    if (cnt >= capacity || !nonzero4(beta))
-                        break;
-                    if (!finite3(ro) || !finite3(rd) || !finite_nonnegative4(beta)) {
-                        status = 2;
-                        break;
-                    }
-                    const u32 prim = __float_as_uint(hit.w);
-                    if (prim >= kHitArithmetic && prim != kNone) {
-                        status = prim == kHitInvalid ? 3u : prim == kHitExhausted ? 4u : 2u;
-                        break;
-                    }
-                    if (prim == kNone) {
-                        ctype = kEnvironment;
-                        clight = s.environment_light;
-                        cp.position = ro + rd;
-                        cp.geometric_normal = -rd;
-                        cp.shading_normal = -rd;
-                        cwo = -rd;
-                        cbeta = beta;
-                        connectible = true;
-                        ++cnt;
-                        break;
-                    }
-                    if constexpr (F == 3) {
-                        status = 3; // a surface hit never reaches the no-surface bin
-                        break;
-                    } else {
-                        const float t = hit.x, b1 = hit.y, b2 = hit.z;
-                        if (!isfinite(t) || t < 0 || !isfinite(b1) || !isfinite(b2) || prim >= s.prim_count) {
-                            status = 3;
-                            break;
-                        }
-                        cinst = s.tri_instance[prim];
-                        clocal = s.tri_local[prim];
-                        const DInstance &instance = s.instances[cinst];
-                        if (instance.material >= s.material_count) {
-                            status = 3;
-                            break;
-                        }
-                        // a mix root's hit was resolved by the closest-hit kernel
-                        cmat = (instance.resolve & kMixRoot) ? pool.material[path] : instance.material;
-                        ctype = kSurface;
-                        clight = instance.emission == kNone ? kNone : instance.emitter_begin + clocal;
-                        cwo = -rd;
-                        if (!hit_surface_point(s, prim, cinst, clocal, b1, b2, cp)) {
-                            status = 2;
-                            break;
-                        }
-                        const DMaterial material = s.materials[cmat];
-                        // an image reflectance reads its texture at the hit's footprint
-                        // (shaders/packet_pt_event_body.inc:147-163, packet_walk.h:39-49)
-                        RgbPolynomial image_rgb;
-                        bool image = false;
-                        if constexpr (F == 0) {
-                            if (Img && s.img.textured && material.kind == 3 && material.image_texture < s.img.texture_count) {
-                                F2 st, dstdx, dstdy;
-                                if (!texture_context(s, p, ident.x, ident.y, ident.z, cinst, clocal, b1, b2,
-                                                     cp.geometric_normal, rd, cnt - 1, st, dstdx, dstdy)) {
-                                    status = 2;
-                                    break;
-                                }
-                                image_rgb = rgb_polynomial(
-                                    s.img.rgb_table, image_reflectance_rgb(s.img, material.image_texture, st, dstdx, dstdy));
-                                image = true;
-                            }
-                        }
-                        if (!shading_frame(cp.shading_normal, cframe) ||
-                            !prepare_bsdf<F>(s, material, lambda, active_mask, cbsdf, image ? &image_rgb : nullptr)) {
-                            status = 2;
-                            break;
-                        }
-                        V3 ray_position, ray_error;
-                        ray_point(ro, rd, t, cp.curved, ray_position, ray_error);
-                        cp.error = cp.error + (vabs(cp.position - ray_position) + ray_error);
-                        if (!finite3(cp.error)) {
-                            status = 2;
-                            break;
-                        }
-                        cbeta = beta;
-                        connectible = hero_connectible(cbsdf);
-                        ++cnt;
-                        if (cnt == capacity)
-                            break;
-                        if (cnt - 2 >= p.emergency_limit) {
-                            status = 1;
-                            break;
-                        }
-                        // only a dielectric reads the lobe word, a smooth one only that of the
-                        // three, and the first event no roulette word
-                        const bool survival = roulette && cnt > 2;
-                        const u32 set = F == 2 ? (cbsdf.g.smooth ? (survival ? kDrawXW : kDrawX) : kDrawAll)
-                                               : (survival ? kDrawYZW : kDrawYZ);
-                        const uint4 draws = draw_words(s, p, ident.x, ident.y, ident.z, index, 4 + cnt - 2, set);
-                        swo = to_local(cframe, cwo);
-                        cbsdf.active_mask = active_mask;
-                        direct_density = density;
-                        direct_allowed = hero_continue(beta, eta_scale, roulette, cnt - 1, sample_uniform(p, draws.w));
-                        direct_beta = beta;
-                        connectible = hero_connectible(cbsdf);
-                        if (!direct_allowed)
-                            break;
-                        const HeroSample proposed = hero_sample_k<F>(cbsdf, swo, sample_uniform(p, draws.x),
-                                                                sample_uniform(p, draws.y), sample_uniform(p, draws.z));
-                        bool cont_valid = proposed.valid;
-                        if (proposed.valid && proposed.accepted) {
-                            hero_previous = direct_density;
-                            const Update adv = advance(direct_density, beta, proposed.numerator, proposed.pdf);
-                            cont_valid = adv.valid;
-                            if (adv.valid) {
-                                beta = adv.beta;
-                                density = adv.density;
-                            }
-                            hero_account_eta(eta_scale, roulette, proposed.eta, proposed.transmission);
-                            active_mask = 1;
-    #pragma unroll
-                            for (int k = 1; k < 4; ++k)
-                                if (density.lane[k].fraction > 0 || (fbits(beta.v[k]) & 0x7fffffffu))
-                                    active_mask |= 1u << k;
-                        }
-                        if (!cont_valid) {
-                            status = 2;
-                            break;
-                        }
-                        if (!proposed.accepted)
-                            break;
-                        pair_valid = true;
-                        V3 wi = to_world(cframe, proposed.wi);
-                        if (!unit_vector(wi, wi)) {
-                            status = 2;
-                            break;
-                        }
-                        if (!finite_nonnegative4(beta)) {
-                            status = 2;
-                            break;
-                        }
-                        if (proposed.delta)
-                            cdelta = true;
-                        const V3 origin = offset_point(cp.position, cp.error, cp.geometric_normal, wi);
-                        if (!finite3(origin)) {
-                            status = 2;
-                            break;
-                        }
-                        ro = origin;
-                        rd = wi;
-                        terminated = false;
-                    }
-                } while (false);
-                bool complete = terminated || status != 0 || cnt >= capacity || !nonzero4(beta);
-                // latest vertex (the previous event's) for MIS
-                const float4 lp4 = pool.latest_p[path], ln4 = pool.latest_n[path];
-                Latest latest;
-                latest.type = (flags >> F_LTYPE_SHIFT) & 3u;
-                latest.kind = (flags >> F_LKIND_SHIFT) & 3u;
-                latest.mask = (flags >> F_LMASK_SHIFT) & 15u;
-                latest.delta = (flags & F_LDELTA) != 0;
-                latest.smooth = (flags & F_LSMOOTH) != 0;
-                latest.position = v3(lp4.x, lp4.y, lp4.z);
-                latest.shading_normal = v3(ln4.x, ln4.y, ln4.z);
-                latest.alpha_x = lp4.w;
-                latest.alpha_y = ln4.w;
-                if (cnt != old_count && status == 0) {
-                    // hero_endpoint (shaders/hero_pt_helpers.h:157-184)
-                    V4 rad = v4(0);
-                    bool emission_ok = true;
-                    if (ctype == kEnvironment) {
-                        if (Img && s.img.env_image != kNone) {
-                            rad = environment_image_radiance4(s.img, rd, lambda);
-                        } else if (s.environment != kNone) {
-#pragma unroll
-                            for (int k = 0; k < 4; ++k)
-                                rad.v[k] = spectrum(s, s.environment, lambda.v[k]);
-                        }
-                        emission_ok = finite_nonnegative4(rad);
-                    } else {
-                        const V3 delta = latest.position - cp.position;
-                        const DInstance &instance = s.instances[cinst];
-                        if (!zero3(delta) && instance.emission != kNone) {
-                            const V3 dir = normalize3(delta);
-                            if (s.emission_two_sided[instance.emission] || dot(cp.geometric_normal, dir) > 0) {
-                                const u32 off = instance.emission * 471u;
-#pragma unroll
-                                for (int k = 0; k < 4; ++k)
-                                    rad.v[k] = cp.inverse_area_pdf == 0 ? 0.f : spectrum(s, off, lambda.v[k]);
-                                emission_ok = finite_nonnegative4(rad);
-                            }
-                        }
-                    }
-                    V4 endpoint = v4(0);
-                    if (!emission_ok) {
-                        status = 2;
-                    } else {
-                        const V4 value = mul4(cbeta, rad);
-                        if (cnt <= 2 || latest.delta || !nonzero4(value)) {
-                            endpoint = value;
-                        } else {
-                            latest.param = from_float4(pool.latest_param[path]);
-                            latest.k = from_float4(pool.latest_k[path]);
-                            const float4 pre = pool.preceding[path];
-                            bool ok;
-                            const V4 bsdf_pdf = represented_pdf<-1>(latest_bsdf(latest), latest.shading_normal, latest.position,
-                                                                v3(pre.x, pre.y, pre.z), ctype == kEnvironment,
-                                                                ctype == kEnvironment ? rd : cp.position, ok);
-                            // hero_history_light_pdf / direct_pdf (shaders/packet_transport.h:740-758)
-                            float lpdf = 0;
-                            const float selection = light_pmf(s, latest.position, latest.shading_normal, clight);
-                            if (ctype == kEnvironment) {
-                                // the constant environment has no unidirectional proposal;
-                                // the image's is its compensated table
-                                lpdf = (Img && s.img.env_image != kNone) ? environment_image_pdf(s.img, rd, true) * selection
-                                                                : 0.0f * selection;
-                            } else {
-                                const V3 dl = cp.position - latest.position;
-                                if (dot(dl, dl) > 0 && nonzero3(cp.geometric_normal) && clight < s.emitter_count)
-                                    lpdf = selection * light_geometry_pdf(s, clight, latest.position,
-                                                                          latest.shading_normal, cp);
-                            }
-                            if (!ok || !hero_weight(previous_density, value, ok ? bsdf_pdf : v4(__int_as_float(0x7fffffff)),
-                                                    v4(lpdf), endpoint))
-                                status = 2;
-                        }
-                    }
-                    radiance = add4(radiance, endpoint);
-                    if (Adjoint) {
-                        // replay: the emission's gradient over the vertices before this one,
-                        // then this diffuse vertex joins the history of what follows it
-                        uint4 h = pool.hist[path];
-                        if (status == 0 && nonzero4(endpoint))
-                            adjoint_accumulate(s, pool, sgrad, h, lambda, endpoint, pool.adj_w[path]);
-                        if (F == 0 && ctype == kSurface && status == 0) {
-                            const u32 m = cmat;
-                            if (__ldg(pool.adj_slot + m) != kNone) {
-                                h = history_push(h, m);
-                                pool.hist[path] = h;
-                            }
-                        }
-                    }
-                    // hero_direct (shaders/hero_pt_helpers.h:185-221) runs in the light-sample kernel
-                    // (k_nee), from the request this event leaves (write_nee_request); its failures fail the
-                    // path there.
-                    nee = F != 3 && status == 0 && cnt < capacity && direct_allowed && ctype == kSurface && connectible;
-                    if (!finite_nonnegative4(radiance))
-                        status = 2;
-                    if (status != 0) {
-                        complete = true;
-                        nee = false;
-                    }
-                    if (nee) {
-                        Density dd = direct_density;
-                        write_nee_request(pool, path, cnt, cp, cbsdf, cwo, latest.position, direct_beta, dd);
-                    }
-                }
-                // A complete path is read again only for its identity, status and radiance (the
-                // shadow walk, the film and the packet results), so the rest of its state is not
-                // written back.
-                if (cnt != old_count) {
-                    // preceding = latest; latest = current (shaders/packet_pt_event_body.inc:453-460)
-                    flags = (flags & ~(3u << F_PTYPE_SHIFT)) | (latest.type << F_PTYPE_SHIFT);
-                    if (!complete) {
-                        pool.preceding[path] = make_float4(latest.position.x, latest.position.y, latest.position.z, 0);
-                        pool.latest_p[path] =
-                            make_float4(cp.position.x, cp.position.y, cp.position.z, cbsdf.g.alpha_x);
-                        pool.latest_n[path] =
-                            make_float4(cp.shading_normal.x, cp.shading_normal.y, cp.shading_normal.z, cbsdf.g.alpha_y);
-                        pool.latest_param[path] =
-                            make_float4(cbsdf.param[0], cbsdf.param[1], cbsdf.param[2], cbsdf.param[3]);
-                        pool.latest_k[path] = make_float4(cbsdf.k[0], cbsdf.k[1], cbsdf.k[2], cbsdf.k[3]);
-                    }
-                    flags &= ~((3u << F_LTYPE_SHIFT) | F_LDELTA | (3u << F_LKIND_SHIFT) | (15u << F_LMASK_SHIFT) | F_LSMOOTH);
-                    flags |= (ctype << F_LTYPE_SHIFT) | (cdelta ? F_LDELTA : 0u) | ((cbsdf.kind & 3u) << F_LKIND_SHIFT) |
-                             ((cbsdf.active_mask & 15u) << F_LMASK_SHIFT) | (cbsdf.g.smooth ? F_LSMOOTH : 0u);
-                }
-                flags = (flags & ~(F_MASK | F_ROULETTE)) | active_mask | (roulette ? F_ROULETTE : 0u);
-                flags = set_status(flags, status) | (complete ? F_COMPLETE : 0u);
-                ident.w = flags;
-                pool.ident[path] = ident;
-                pool.radiance[path] = to_float4(radiance);
-                if (!complete) {
-                    cursor.z = cnt;
-                    pool.cursor[path] = cursor;
-                    pool.beta[path] = to_float4(beta);
-                    float4 f;
-                    int4 e;
-                    store_density(density, f, e);
-                    pool.dens_f[path] = f;
-                    pool.dens_e[path] = e;
-                    store_density(hero_previous, f, e);
-                    pool.prev_f[path] = f;
-                    pool.prev_e[path] = e;
-                    pool.eta_scale[path] = to_float4(eta_scale);
-                    pool.ray_o[path] = make_float4(ro.x, ro.y, ro.z, 0);
-                    pool.ray_d[path] = make_float4(rd.x, rd.y, rd.z, 0);
-                }
-                keep = !complete;
-            }
-        }
+        shade_path<F, Adjoint, Img, true>(s, p, pool, active, path, sgrad, keep, nee);
         const u32 slot = warp_append(out_count, keep);
         if (keep)
             out_queue[slot] = path;
         if (F != 3) {
-            const u32 nslot = warp_append(pool.counters + 8 + F, nee);
+            const u32 nslot = warp_append(event + kNeeCount + F, nee);
             if (nee)
                 pool.nee_queue[size_t(F) * pool.bin_capacity + nslot] = path;
         }
@@ -565,16 +603,172 @@ __global__ void __launch_bounds__(Block, 512 / Block) k_shade(const __grid_const
         adjoint_end(pool, sgrad);
 }
 
-// The light sample of one hero event (hero_direct, shaders/hero_pt_helpers.h:185-221) for the
-// paths of BSDF family F whose event asked for one: light selection, the light's point and
+// The light sample of one hero event (hero_direct, shaders/hero_pt_helpers.h:185-221) of a
+// path whose event (of BSDF family F) asked for one: light selection, the light's point and
 // radiance, the BSDF on the light direction, the balance weight, and the visibility segment
-// queued for the shadow kernel.  Its own failures (invalid arithmetic) fail the path.  Split
+// (shadow set).  Its own failures (invalid arithmetic) fail the path.  Split
 // from the shade kernel, which leaves the request (write_nee_request), so that each kernel
 // holds half the live state.
+template <int F, bool Img, bool Sync>
+RP_DEV void nee_path(const DeviceScene &s, const WaveParams &p, const PathPool &pool, bool active, u32 path, bool &shadow,
+                     float4 &sh_o, float4 &sh_d, float4 &sh_c, float4 &sh_t) {
+    uint4 ident = pool.ident[path];
+    const uint4 cursor = pool.cursor[path];
+    const u64 index = (u64(cursor.y) << 32) | cursor.x;
+    const V4 lambda = from_float4(pool.lambda[path]);
+    u32 cnt;
+    SurfacePoint cp;
+    HeroBsdf cbsdf;
+    V3 cwo, previous;
+    V4 direct_beta;
+    Density direct_density;
+    read_nee_request(pool, path, cnt, cp, cbsdf, cwo, previous, direct_beta, direct_density);
+    u32 status = 0;
+    // the light-sample draw: its first word selects the light; the next two, a point on an
+    // area light, are drawn only when an area light was selected (the same words either way)
+    const u32 block = 133 + cnt - 2;
+    // sample_li (shaders/packet_transport.h:470-553)
+    float selected_pmf = 0; // light_pmf of the selected light
+    Selected choice{kNone, 0};
+    bool env_image = false;
+    if (active) {
+        const float u0 = sample_uniform(p, draw_words(s, p, ident.x, ident.y, ident.z, index, block, kDrawX).x);
+        choice = light_sample<true>(s, cp.position, cp.shading_normal, u0, selected_pmf);
+        env_image = Img && s.img.env_image != kNone && choice.light == s.environment_light;
+    }
+    phase<Sync>();
+    V4 lbeta = v4(0);
+    float spdf = 0, geometry_pdf = 0; // geometry_pdf: light_geometry_pdf of the sampled point
+    bool li_ok = true, delta_light = false;
+    SurfacePoint lp;
+    lp.position = lp.error = lp.geometric_normal = lp.shading_normal = v3(0, 0, 0);
+    lp.inverse_area_pdf = 0;
+    V3 direction = v3(0, 0, 1);
+    const u32 sel = choice.light;
+    if (active && choice.pmf > 0) {
+        float u1 = 0, u2 = 0;
+        if (choice.light < s.emitter_count || env_image) {
+            const uint4 w = draw_words(s, p, ident.x, ident.y, ident.z, index, block, kDrawYZ);
+            u1 = sample_uniform(p, w.y);
+            u2 = sample_uniform(p, w.z);
+        }
+        V4 lrad = v4(0);
+        if (sel < s.emitter_count) {
+            if (!light_geometry_sample(s, sel, cp.position, cp.shading_normal, u1, u2, lp, spdf)) {
+                li_ok = false;
+            } else {
+                geometry_pdf = spdf;
+                spdf *= choice.pmf;
+                const V3 dl = lp.position - cp.position;
+                const float d2 = dot(dl, dl);
+                if (lp.inverse_area_pdf == 0 || !(d2 > 0)) {
+                    spdf = 0;
+                } else {
+                    direction = dl * (1.0f / sqrtf(d2));
+                    const DInstance &li = s.instances[s.emitter_instance[sel]];
+                    if (s.emission_two_sided[li.emission] || dot(lp.geometric_normal, -direction) > 0) {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            lrad.v[k] = spectrum(s, li.emission * 471u, lambda.v[k]);
+                    }
+                    li_ok = finite_nonnegative4(lrad);
+                }
+            }
+        } else if (sel < s.emitter_count + s.positional_count) {
+            const DPositional &L = s.positional[sel - s.emitter_count];
+            delta_light = true;
+            lp.position = v3(L.position[0], L.position[1], L.position[2]);
+            const V3 dl = lp.position - cp.position;
+            const float d2 = dot(dl, dl);
+            if (!(d2 > 0)) {
+                spdf = 0;
+            } else {
+                direction = dl * (1.0f / sqrtf(d2));
+                float falloff = 1;
+                const bool lit = positional_falloff(L, direction, falloff);
+                li_ok = lit;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    float intensity = spectrum(s, L.spectrum, lambda.v[k]);
+                    if (lit && !apply_falloff(L, falloff, intensity))
+                        li_ok = false;
+                    lrad.v[k] = intensity / d2;
+                }
+                spdf = choice.pmf;
+            }
+        } else if (env_image) {
+            // the environment image's compensated table (shaders/packet_transport.h:536-552)
+            float epdf = 0;
+            if (!sample_environment_image(s.img, u1, u2, true, direction, epdf)) {
+                li_ok = false;
+            } else {
+                lrad = environment_image_radiance4(s.img, direction, lambda);
+                spdf = epdf * choice.pmf;
+                lp.position = cp.position + (2 * s.scene_radius) * direction;
+                lp.geometric_normal = lp.shading_normal = -direction;
+            }
+        } else {
+            spdf = 0; // constant environment: pdf 0 for unidirectional PT
+        }
+        if (li_ok)
+            lbeta = spdf > 0 ? V4{{lrad.v[0] / spdf, lrad.v[1] / spdf, lrad.v[2] / spdf, lrad.v[3] / spdf}} : v4(0);
+        li_ok = li_ok && finite_nonnegative4(lbeta);
+    }
+    if (active && (!li_ok || !isfinite(spdf) || spdf < 0))
+        status = 2;
+    bool go = active && status == 0 && spdf > 0 && nonzero4(lbeta);
+    phase<Sync>();
+    Frame cframe;
+    V4 value = v4(0);
+    if (go) {
+        shading_frame(cp.shading_normal, cframe); // succeeded in the shade kernel
+        const HeroEval e = hero_evaluate_k<F == 3 ? 0 : F>(cbsdf, to_local(cframe, cwo), to_local(cframe, direction));
+        if (!e.valid)
+            status = 2;
+        else
+            value = scale4(mul4(mul4(direct_beta, e.f), lbeta), fabsf(dot(cp.shading_normal, direction)));
+        go = e.valid && nonzero4(value);
+    }
+    phase<Sync>();
+    if (go) {
+        V4 contribution = value;
+        bool weight_ok = true;
+        if (!delta_light) {
+            const float sel_pmf = selected_pmf >= 0 ? selected_pmf : light_pmf(s, cp.position, cp.shading_normal, sel);
+            const float lpdf = env_image                        ? environment_image_pdf(s.img, direction, true) * sel_pmf
+                               : nonzero3(lp.geometric_normal) ? sel_pmf * geometry_pdf
+                                                               : 0.0f;
+            bool ok;
+            const V4 bsdf_pdf = represented_pdf<F == 3 ? 0 : F>(cbsdf, cframe, cp.position, previous, env_image,
+                                                                env_image ? direction : lp.position, ok);
+            weight_ok = ok && hero_weight(direct_density, value, v4(lpdf), bsdf_pdf, contribution);
+        }
+        // visible(): offset both endpoints (shaders/packet_transport.h:377-446)
+        const V3 seg = lp.position - cp.position;
+        if (!zero3(seg)) {
+            const V3 so = offset_point(cp.position, cp.error, cp.geometric_normal, seg);
+            const V3 st = offset_point(lp.position, lp.error, lp.geometric_normal, -seg);
+            const V3 sd = st - so;
+            shadow = true;
+            sh_o = make_float4(so.x, so.y, so.z, kOneMinusEps);
+            sh_d = make_float4(sd.x, sd.y, sd.z, __uint_as_float(path));
+            sh_t = make_float4(st.x, st.y, st.z, 0);
+            sh_c = weight_ok ? to_float4(contribution) : make_float4(__int_as_float(0x7fffffff), 0, 0, 0);
+        }
+    }
+    if (status != 0) {
+        ident.w = set_status(ident.w, status) | F_COMPLETE;
+        pool.ident[path] = ident;
+        shadow = false;
+    }
+}
+// nee_path of the paths of family F with a request; the segments are queued for the shadow
+// kernel.
 template <int F, int Block = 128, bool Img = true>
 __global__ void __launch_bounds__(Block, 512 / Block) k_nee(const __grid_constant__ DeviceScene s,
-                                                            const __grid_constant__ WaveParams p, PathPool pool) {
-    const u32 count = pool.counters[8 + F];
+                                                            const __grid_constant__ WaveParams p, PathPool pool, int in) {
+    u32 *event = pool.event(in);
+    const u32 count = event[kNeeCount + F];
     const u32 *queue = pool.nee_queue + size_t(F) * pool.bin_capacity;
     const u32 stride = gridDim.x * blockDim.x;
     const u32 trips = (count + stride - 1) / stride;
@@ -582,163 +776,9 @@ __global__ void __launch_bounds__(Block, 512 / Block) k_nee(const __grid_constan
         const u32 i = trip * stride + blockIdx.x * blockDim.x + threadIdx.x;
         bool shadow = false;
         float4 sh_o = make_float4(0, 0, 0, 0), sh_d = sh_o, sh_c = sh_o, sh_t = sh_o;
-        if (i < count) {
-            const u32 path = queue[i];
-            uint4 ident = pool.ident[path];
-            const uint4 cursor = pool.cursor[path];
-            const u64 index = (u64(cursor.y) << 32) | cursor.x;
-            const V4 lambda = from_float4(pool.lambda[path]);
-            u32 cnt;
-            SurfacePoint cp;
-            HeroBsdf cbsdf;
-            V3 cwo, previous;
-            V4 direct_beta;
-            Density direct_density;
-            read_nee_request(pool, path, cnt, cp, cbsdf, cwo, previous, direct_beta, direct_density);
-            Latest latest;
-            latest.position = previous;
-            Frame cframe;
-            shading_frame(cp.shading_normal, cframe); // succeeded in the shade kernel
-            const bool pair_valid = false;
-            const V3 swo = v3(0, 0, 0);
-            u32 status = 0;
-            {
-                        // the light-sample draw: its first word selects the light; the next two, a
-                        // point on an area light, are drawn only when an area light was selected
-                        // (the same words either way)
-                        const u32 block = 133 + cnt - 2;
-                        const float u0 = sample_uniform(p, draw_words(s, p, ident.x, ident.y, ident.z, index, block, kDrawX).x);
-                        // sample_li (shaders/packet_transport.h:470-553)
-                        float selected_pmf = 0; // light_pmf of the selected light
-                        const Selected choice = light_sample<true>(s, cp.position, cp.shading_normal, u0, selected_pmf);
-                        float u1 = 0, u2 = 0;
-                        const bool env_image = Img && s.img.env_image != kNone && choice.light == s.environment_light;
-                        if (choice.pmf > 0 && (choice.light < s.emitter_count || env_image)) {
-                            const uint4 w = draw_words(s, p, ident.x, ident.y, ident.z, index, block, kDrawYZ);
-                            u1 = sample_uniform(p, w.y);
-                            u2 = sample_uniform(p, w.z);
-                        }
-                        V4 lbeta = v4(0);
-                        float spdf = 0, geometry_pdf = 0; // geometry_pdf: light_geometry_pdf of the sampled point
-                        bool li_ok = true, delta_light = false;
-                        SurfacePoint lp;
-                        lp.position = lp.error = lp.geometric_normal = lp.shading_normal = v3(0, 0, 0);
-                        lp.inverse_area_pdf = 0;
-                        V3 direction = v3(0, 0, 1);
-                        const u32 sel = choice.light;
-                        if (choice.pmf > 0) {
-                            V4 lrad = v4(0);
-                            if (sel < s.emitter_count) {
-                                if (!light_geometry_sample(s, sel, cp.position, cp.shading_normal, u1, u2, lp, spdf)) {
-                                    li_ok = false;
-                                } else {
-                                    geometry_pdf = spdf;
-                                    spdf *= choice.pmf;
-                                    const V3 dl = lp.position - cp.position;
-                                    const float d2 = dot(dl, dl);
-                                    if (lp.inverse_area_pdf == 0 || !(d2 > 0)) {
-                                        spdf = 0;
-                                    } else {
-                                        direction = dl * (1.0f / sqrtf(d2));
-                                        const DInstance &li = s.instances[s.emitter_instance[sel]];
-                                        if (s.emission_two_sided[li.emission] || dot(lp.geometric_normal, -direction) > 0) {
-#pragma unroll
-                                            for (int k = 0; k < 4; ++k)
-                                                lrad.v[k] = spectrum(s, li.emission * 471u, lambda.v[k]);
-                                        }
-                                        li_ok = finite_nonnegative4(lrad);
-                                    }
-                                }
-                            } else if (sel < s.emitter_count + s.positional_count) {
-                                const DPositional &L = s.positional[sel - s.emitter_count];
-                                delta_light = true;
-                                lp.position = v3(L.position[0], L.position[1], L.position[2]);
-                                const V3 dl = lp.position - cp.position;
-                                const float d2 = dot(dl, dl);
-                                if (!(d2 > 0)) {
-                                    spdf = 0;
-                                } else {
-                                    direction = dl * (1.0f / sqrtf(d2));
-#pragma unroll
-                                    for (int k = 0; k < 4; ++k) {
-                                        float intensity = spectrum(s, L.spectrum, lambda.v[k]);
-                                        if (!positional_intensity(L, direction, intensity))
-                                            li_ok = false;
-                                        lrad.v[k] = intensity / d2;
-                                    }
-                                    spdf = choice.pmf;
-                                }
-                            } else if (env_image) {
-                                // the environment image's compensated table
-                                // (shaders/packet_transport.h:536-552)
-                                float epdf = 0;
-                                if (!sample_environment_image(s.img, u1, u2, true, direction, epdf)) {
-                                    li_ok = false;
-                                } else {
-                                    lrad = environment_image_radiance4(s.img, direction, lambda);
-                                    spdf = epdf * choice.pmf;
-                                    lp.position = cp.position + (2 * s.scene_radius) * direction;
-                                    lp.geometric_normal = lp.shading_normal = -direction;
-                                }
-                            } else {
-                                spdf = 0; // constant environment: pdf 0 for unidirectional PT
-                            }
-                            if (li_ok)
-                                lbeta = spdf > 0 ? V4{{lrad.v[0] / spdf, lrad.v[1] / spdf, lrad.v[2] / spdf,
-                                                       lrad.v[3] / spdf}}
-                                                 : v4(0);
-                            li_ok = li_ok && finite_nonnegative4(lbeta);
-                        }
-                        if (!li_ok || !isfinite(spdf) || spdf < 0) {
-                            status = 2;
-                        } else if (spdf > 0 && nonzero4(lbeta)) {
-                            const HeroEval e = hero_evaluate_k<F == 3 ? 0 : F>(
-                                cbsdf, pair_valid ? swo : to_local(cframe, cwo), to_local(cframe, direction));
-                            if (!e.valid) {
-                                status = 2;
-                            } else {
-                                const V4 value = scale4(mul4(mul4(direct_beta, e.f), lbeta),
-                                                        fabsf(dot(cp.shading_normal, direction)));
-                                if (nonzero4(value)) {
-                                    V4 contribution = value;
-                                    bool weight_ok = true;
-                                    if (!delta_light) {
-                                        const float sel_pmf =
-                                            selected_pmf >= 0 ? selected_pmf : light_pmf(s, cp.position, cp.shading_normal, sel);
-                                        const float lpdf =
-                                            env_image ? environment_image_pdf(s.img, direction, true) * sel_pmf
-                                            : nonzero3(lp.geometric_normal) ? sel_pmf * geometry_pdf
-                                                                            : 0.0f;
-                                        bool ok;
-                                        const V4 bsdf_pdf = represented_pdf<F == 3 ? 0 : F>(
-                                            cbsdf, cp.shading_normal, cp.position, latest.position, env_image,
-                                            env_image ? direction : lp.position, ok);
-                                        weight_ok = ok && hero_weight(direct_density, value, v4(lpdf), bsdf_pdf, contribution);
-                                    }
-                                    // visible(): offset both endpoints (shaders/packet_transport.h:377-446)
-                                    const V3 seg = lp.position - cp.position;
-                                    if (!zero3(seg)) {
-                                        const V3 so = offset_point(cp.position, cp.error, cp.geometric_normal, seg);
-                                        const V3 st = offset_point(lp.position, lp.error, lp.geometric_normal, -seg);
-                                        const V3 sd = st - so;
-                                        shadow = true;
-                                        sh_o = make_float4(so.x, so.y, so.z, kOneMinusEps);
-                                        sh_d = make_float4(sd.x, sd.y, sd.z, __uint_as_float(path));
-                                        sh_t = make_float4(st.x, st.y, st.z, 0);
-                                        sh_c = weight_ok ? to_float4(contribution)
-                                                         : make_float4(__int_as_float(0x7fffffff), 0, 0, 0);
-                                    }
-                                }
-                            }
-                        }
-            }
-            if (status != 0) {
-                ident.w = set_status(ident.w, status) | F_COMPLETE;
-                pool.ident[path] = ident;
-                shadow = false;
-            }
-        }
-        const u32 sslot = warp_append(pool.counters + 2, shadow);
+        const bool active = i < count;
+        nee_path<F, Img, true>(s, p, pool, active, active ? queue[i] : 0, shadow, sh_o, sh_d, sh_c, sh_t);
+        const u32 sslot = warp_append(event + kShadowCount, shadow);
         if (shadow) {
             pool.sh_o[sslot] = sh_o;
             pool.sh_d[sslot] = sh_d;
@@ -786,16 +826,52 @@ __device__ __noinline__ u32 pass_through_visible(const DeviceScene &s, V3 o, V3 
     return 4;
 }
 
-// Visibility of the light samples (visible(), shaders/packet_transport.h:377-446, opaque surfaces)
-// Resolve: the scene has pass-through instances, which shadow rays cross (pass_through_visible).
+// What a light sample's visibility walk does to its path (visible(),
+// shaders/packet_transport.h:377-446): the contribution where nothing occludes it, or the
+// sample's failure.
+template <bool Adjoint>
+RP_DEV void shadow_result(const DeviceScene &s, const PathPool &pool, float *sgrad, const float4 &contribution, u32 path,
+                          u32 failure, bool occluded) {
+    if (!failure && occluded)
+        return;
+    uint4 ident = pool.ident[path];
+    if (failure) {
+        ident.w = set_status(ident.w, failure) | F_COMPLETE;
+        pool.ident[path] = ident;
+        return;
+    }
+    const float4 c = contribution;
+    if (isnan(c.x)) {
+        ident.w = set_status(ident.w, 2) | F_COMPLETE;
+        pool.ident[path] = ident;
+        return;
+    }
+    float4 r = pool.radiance[path];
+    r.x += c.x;
+    r.y += c.y;
+    r.z += c.z;
+    r.w += c.w;
+    pool.radiance[path] = r;
+    if (!finite_nonnegative4(from_float4(r))) {
+        ident.w = set_status(ident.w, 2) | F_COMPLETE;
+        pool.ident[path] = ident;
+    } else if (Adjoint) {
+        // replay: the light sample's gradient, over the history including its vertex
+        adjoint_accumulate(s, pool, sgrad, pool.hist[path], from_float4(pool.lambda[path]), from_float4(c),
+                           pool.adj_w[path]);
+    }
+}
+// Visibility of the light samples, opaque surfaces; Resolve: the scene has pass-through
+// instances, which shadow rays cross (pass_through_visible).
 template <bool Count, int Block = kTraceBlock, bool Adjoint = false, int Stack = kStackDepth, bool Resolve = false>
 __global__ void __launch_bounds__(Block, Stack <= kShortStack ? 1024 / Block : 1)
-    k_shadow(const __grid_constant__ DeviceScene s, PathPool pool, u32 boundary_limit) {
+    k_shadow(const __grid_constant__ DeviceScene s, PathPool pool, int in, u32 boundary_limit) {
     __shared__ uint2 stack[Stack * Block];
     extern __shared__ float sgrad[]; // adjoint only
     if (Adjoint)
         adjoint_begin(pool, sgrad);
-    const u32 count = pool.counters[2];
+    u32 *event = pool.event(in);
+    const u32 count = event[kShadowCount];
     u32 nodes = 0, tris = 0, rays = 0;
     for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         const float4 o = pool.sh_o[i], d = pool.sh_d[i];
@@ -808,41 +884,14 @@ __global__ void __launch_bounds__(Block, Stack <= kShortStack ? 1024 / Block : 1
                                                          occluded, stack + threadIdx.x, Block, boundary_limit, nodes,
                                                          tris, rays);
         } else {
-            if (!walk_any<Count, Stack, false>(s, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), o.w, occluded, stack + threadIdx.x,
-                                        Block, nodes, tris))
+            if (!walk_any<Count, Stack, false>(s, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), o.w, occluded,
+                                               stack + threadIdx.x, Block, nodes, tris))
                 failure = 3;
             ++rays;
         }
         if (Count && pool.lane_shadow)
             pool.lane_shadow[path] += rays - walks_before;
-        uint4 ident = pool.ident[path];
-        if (failure) {
-            ident.w = set_status(ident.w, failure) | F_COMPLETE;
-            pool.ident[path] = ident;
-            continue;
-        }
-        if (occluded)
-            continue;
-        const float4 c = pool.sh_c[i];
-        if (isnan(c.x)) {
-            ident.w = set_status(ident.w, 2) | F_COMPLETE;
-            pool.ident[path] = ident;
-            continue;
-        }
-        float4 r = pool.radiance[path];
-        r.x += c.x;
-        r.y += c.y;
-        r.z += c.z;
-        r.w += c.w;
-        pool.radiance[path] = r;
-        if (!finite_nonnegative4(from_float4(r))) {
-            ident.w = set_status(ident.w, 2) | F_COMPLETE;
-            pool.ident[path] = ident;
-        } else if (Adjoint) {
-            // replay: the light sample's gradient, over the history including its vertex
-            adjoint_accumulate(s, pool, sgrad, pool.hist[path], from_float4(pool.lambda[path]), from_float4(c),
-                               pool.adj_w[path]);
-        }
+        shadow_result<Adjoint>(s, pool, sgrad, pool.sh_c[i], path, failure, occluded);
     }
     if (Adjoint)
         adjoint_end(pool, sgrad);

@@ -816,7 +816,9 @@ RP_DEV bool spot_divide(float a, float b, float &r) {
     r = a / b;
     return normal_or_zero(r) && (r != 0 || a == 0);
 }
-RP_DEV bool positional_intensity(const DPositional &L, V3 wi, float &intensity) {
+// The falloff of a spot light toward -wi (1 for a point light), the same for every wavelength.
+RP_DEV bool positional_falloff(const DPositional &L, V3 wi, float &falloff) {
+    falloff = 1;
     if (L.kind == 0)
         return true;
     if (L.kind != 1)
@@ -850,9 +852,18 @@ RP_DEV bool positional_intensity(const DPositional &L, V3 wi, float &intensity) 
         return false;
     const float end = L.cos_falloff_end, start = L.cos_falloff_start;
     const float t = start == end ? (cosine < end ? 0.0f : 1.0f) : fminf(fmaxf((cosine - end) / (start - end), 0.0f), 1.0f);
-    const float falloff = start == end ? t : t * t * (3.0f - 2.0f * t);
+    falloff = start == end ? t : t * t * (3.0f - 2.0f * t);
+    return true;
+}
+RP_DEV bool apply_falloff(const DPositional &L, float falloff, float &intensity) {
+    if (L.kind == 0)
+        return true;
     intensity *= falloff;
     return isfinite(intensity) && intensity >= 0;
+}
+RP_DEV bool positional_intensity(const DPositional &L, V3 wi, float &intensity) {
+    float falloff;
+    return positional_falloff(L, wi, falloff) && apply_falloff(L, falloff, intensity);
 }
 
 // ------------------------------------------------------------------ traversal
@@ -998,9 +1009,8 @@ RP_DEV bool any_leaf(const DeviceScene &s, const WalkRay &r, float tmax, u32 ind
 // that axis's bounds NaN or infinite in the direction that leaves the axis unconstrained; the
 // NaN-ignoring min and max then skip it, which is conservative.
 struct WideRay {
-    float a_lo[3], a_hi[3], b_lo[3], b_hi[3]; // per axis, for the node being visited
-    float rcp_lo[3], rcp_hi[3];                // directed-rounding bounds of 1 / d
-    u32 negative;                              // axis bits: d < 0 (the near plane is the hi one)
+    float rcp_lo[3], rcp_hi[3]; // directed-rounding bounds of 1 / d
+    u32 negative;               // axis bits: d < 0 (the near plane is the hi one)
 };
 RP_DEV WideRay wide_ray(V3 d) {
     WideRay w;
@@ -1030,7 +1040,7 @@ RP_DEV float qfloat(u32 word, int byte) { return __uint_as_float(__byte_perm(wor
 // as bits at slot ^ order (near side first), leaves as bits at their slot.  Conservative: the
 // computed entry is at or below the true one and the exit at or above, so no child that holds
 // a hit in [0, tmax] is missed; all eight slots are tested without branches and masked.
-RP_DEV void wide_children(const WNode &n, V3 o, WideRay &w, float tmax, u32 order, u32 &inner, u32 &leaves) {
+RP_DEV void wide_children(const WNode &n, V3 o, const WideRay &w, float tmax, u32 order, u32 &inner, u32 &leaves) {
     const u32 meta = __float_as_uint(n.origin.w);
     const u32 imask = meta >> 24, lmask = n.links.z;
     const float p[3] = {n.origin.x, n.origin.y, n.origin.z}, oo[3] = {o.x, o.y, o.z};
@@ -1038,19 +1048,18 @@ RP_DEV void wide_children(const WNode &n, V3 o, WideRay &w, float tmax, u32 orde
     const u32 rows[6][2] = {{n.q0.x, n.q0.y}, {n.q0.z, n.q0.w}, {n.q1.x, n.q1.y},
                             {n.q1.z, n.q1.w}, {n.q2.x, n.q2.y}, {n.q2.z, n.q2.w}};
     u32 near_w[3][2], far_w[3][2];
+    float a_lo[3], a_hi[3], b_lo[3], b_hi[3]; // per axis
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         const float s = __uint_as_float(((meta >> (8 * a)) & 0xffu) << 23);
         const bool neg = (w.negative >> a) & 1u;
-        float d_lo, d_hi, c_lo, c_hi;
+        float d_lo, d_hi;
         // (p - o) / d, then minus 2^23 s / d
         interval_mul(__fsub_rd(p[a], oo[a]), __fsub_ru(p[a], oo[a]), w.rcp_lo[a], w.rcp_hi[a], neg, d_lo, d_hi);
-        w.b_lo[a] = __fmul_rd(s, w.rcp_lo[a]);
-        w.b_hi[a] = __fmul_ru(s, w.rcp_hi[a]);
-        c_lo = __fmaf_rd(-8388608.0f, w.b_hi[a], d_lo);
-        c_hi = __fmaf_ru(-8388608.0f, w.b_lo[a], d_hi);
-        w.a_lo[a] = c_lo;
-        w.a_hi[a] = c_hi;
+        b_lo[a] = __fmul_rd(s, w.rcp_lo[a]);
+        b_hi[a] = __fmul_ru(s, w.rcp_hi[a]);
+        a_lo[a] = __fmaf_rd(-8388608.0f, b_hi[a], d_lo);
+        a_hi[a] = __fmaf_ru(-8388608.0f, b_lo[a], d_hi);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             near_w[a][h] = neg ? rows[3 + a][h] : rows[a][h];
@@ -1064,8 +1073,8 @@ RP_DEV void wide_children(const WNode &n, V3 o, WideRay &w, float tmax, u32 orde
         float t0 = 0.0f, t1 = tmax;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            t0 = fmaxf(t0, __fmaf_rd(qfloat(near_w[a][h], byte), w.b_lo[a], w.a_lo[a]));
-            t1 = fminf(t1, __fmaf_ru(qfloat(far_w[a][h], byte), w.b_hi[a], w.a_hi[a]));
+            t0 = fmaxf(t0, __fmaf_rd(qfloat(near_w[a][h], byte), b_lo[a], a_lo[a]));
+            t1 = fminf(t1, __fmaf_ru(qfloat(far_w[a][h], byte), b_hi[a], a_hi[a]));
         }
         hits |= (t0 <= t1 ? 1u : 0u) << k;
     }

@@ -43,7 +43,7 @@ struct PathPool {
     float4 *hit;           // t, b1, b2, primitive bits
     // queues
     u32 *queue[2];
-    u32 *counters; // [0] queue0, [1] queue1, [2] shadow, [3] failures, [4..7] family bins
+    u32 *counters; // [0] queue0, [1] queue1, [3] failures, then the two event sets
     u32 *bins;     // 4 family bins of bin_capacity path ids each
     u32 bin_capacity;
     float4 *sh_o;  // shadow origin, tmax
@@ -59,7 +59,7 @@ struct PathPool {
     // density before this event's continuation, and the BSDF's per-wavelength parameters
     float4 *nee_p, *nee_n, *nee_g, *nee_e, *nee_wo, *nee_prev, *nee_beta, *nee_df, *nee_param, *nee_k;
     int4 *nee_de;
-    u32 *nee_queue; // three family queues of bin_capacity path ids; counts in counters[8..10]
+    u32 *nee_queue; // three family queues of bin_capacity path ids
     // per-lane walk counts of counting runs (pool slot = request lane), or nullptr: closest-hit
     // walks (written by the closest-hit kernel) and any-hit walks (by the shadow kernel, which
     // runs beside the next closest-hit walk, hence two arrays)
@@ -73,7 +73,14 @@ struct PathPool {
     const double *adj_cie;  // CIE 1931 table, 3 per nm from 360 nm
     double adj_inv_weight;  // 1 / film weight of a pixel (its sample count)
     u32 adj_params;         // gradient entries
+
+    // The counters of the event whose paths are in queue `in`: family bins, light samples and
+    // shadow segments.  Events alternate between two sets, and the
+    // escape shade kernel of an event, by when every kernel of the event before it has ended,
+    // clears the other set; its closest-hit kernel clears the queue it will fill.
+    RP_DEV u32 *event(int in) const { return counters + 16 + 16 * in; }
 };
+enum : u32 { kBinCount = 0, kNeeCount = 4, kShadowCount = 7, kEventCounters = 8 };
 
 // sampler: 0 independent, 1 Sobol, 2 Halton, 3 ZSobol (src/render_wire.h:41)
 struct WaveParams {
@@ -609,6 +616,26 @@ RP_DEV HeroBsdf latest_bsdf(const Latest &l) {
 // shaders/hero_pt_helpers.h:122-132 (hero_represented_pdf) for a surface vertex v with
 // finite neighbours (the neighbour after v may be at infinity: pass its direction).
 // K selects the BSDF family at compile time; -1 dispatches on the stored family.
+template <int K> RP_DEV V4 represented_pdf(const HeroBsdf &b, const Frame &f, V3 wb, V3 wa, bool &ok) {
+    HeroEval e;
+    if constexpr (K < 0)
+        e = hero_evaluate(b, to_local(f, normalize3(wb)), to_local(f, normalize3(wa)));
+    else
+        e = hero_evaluate_k<K>(b, to_local(f, normalize3(wb)), to_local(f, normalize3(wa)));
+    ok = e.valid;
+    return e.valid ? e.pdf : v4(0);
+}
+// with the vertex's frame already found
+template <int K>
+RP_DEV V4 represented_pdf(const HeroBsdf &b, const Frame &f, V3 position, V3 before, bool after_infinite, V3 after_point,
+                          bool &ok) {
+    ok = true;
+    const V3 wb = before - position;
+    const V3 wa = after_infinite ? after_point : after_point - position;
+    if (zero3(wb) || zero3(wa))
+        return v4(0);
+    return represented_pdf<K>(b, f, wb, wa, ok);
+}
 template <int K>
 RP_DEV V4 represented_pdf(const HeroBsdf &b, V3 shading_normal, V3 position, V3 before, bool after_infinite,
                           V3 after_point, bool &ok) {
@@ -622,16 +649,7 @@ RP_DEV V4 represented_pdf(const HeroBsdf &b, V3 shading_normal, V3 position, V3 
         ok = false;
         return v4(0);
     }
-    HeroEval e;
-    if constexpr (K < 0)
-        e = hero_evaluate(b, to_local(f, normalize3(wb)), to_local(f, normalize3(wa)));
-    else
-        e = hero_evaluate_k<K>(b, to_local(f, normalize3(wb)), to_local(f, normalize3(wa)));
-    if (!e.valid) {
-        ok = false;
-        return v4(0);
-    }
-    return e.pdf;
+    return represented_pdf<K>(b, f, wb, wa, ok);
 }
 // shaders/hero_pt_helpers.h:133-148 (hero_weight); returns false for invalid arithmetic
 RP_DEV bool hero_weight(const Density &prefix, V4 value, V4 sampled, V4 other, V4 &out) {

@@ -1193,18 +1193,6 @@ RP_DEV bool scalar_ray_valid(const ScalarPath &path) {
     return finite3(path.o) && finite3(path.d) && isfinite(path.throughput) && isfinite(path.radiance);
 }
 
-// Warp-aggregated append of `slot` to `queue` (counter `count`) for the lanes with `want`.
-RP_DEV void slot_append(u32 *queue, u32 *count, bool want, u32 slot) {
-    const u32 ballot = __ballot_sync(0xffffffffu, want);
-    const int lane = threadIdx.x & 31;
-    u32 base = 0;
-    if (lane == 0 && ballot)
-        base = atomicAdd(count, __popc(ballot));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (want)
-        queue[base + __popc(ballot & ((1u << lane) - 1))] = slot;
-}
-
 // Whether shade_event will take its medium-scattering branch for this hit: the same medium
 // lookup and free-flight draw, without consuming the draw.  Only groups the step warps; the
 // step itself decides.
@@ -1228,6 +1216,18 @@ RP_DEV bool hits_interface(const DeviceScene &s, const Hit &hit) {
         return false;
     const u32 material = s.instances[s.tri_instance[hit.prim]].material;
     return material < s.material_count && s.materials[material].scattering == kInterfaceScattering;
+}
+
+// Warp-aggregated append of `slot` to `queue` (counter `count`) for the lanes with `want`.
+RP_DEV void slot_append(u32 *queue, u32 *count, bool want, u32 slot) {
+    const u32 ballot = __ballot_sync(0xffffffffu, want);
+    const int lane = threadIdx.x & 31;
+    u32 base = 0;
+    if (lane == 0 && ballot)
+        base = atomicAdd(count, __popc(ballot));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (want)
+        queue[base + __popc(ballot & ((1u << lane) - 1))] = slot;
 }
 
 // Proc: the scene has procedural primitives.
