@@ -1512,6 +1512,21 @@ void attach_draw_tables(rp_scene *s, WaveParams &p) {
     p.draw_blocks = blocks;
 }
 
+// Waves of at most this many lanes run as whole paths (k_paths).
+constexpr u32 kWholePathLanes = 32768;
+void launch_paths(rp_scene *s, const WaveParams &p, const PathPool &pool, int in, u32 first, u32 lanes) {
+    const unsigned grid = grid_for(s->sm_count, lanes, kPathBlock, 64);
+    const bool img = s->ds.img.textured || s->ds.img.env_image != kNone, deep = s->wide_levels > u32(kShortStack);
+    if (img && deep)
+        k_paths<kStackDepth, true><<<grid, kPathBlock, 0, s->stream>>>(s->ds, p, pool, in, first);
+    else if (img)
+        k_paths<kShortStack, true><<<grid, kPathBlock, 0, s->stream>>>(s->ds, p, pool, in, first);
+    else if (deep)
+        k_paths<kStackDepth, false><<<grid, kPathBlock, 0, s->stream>>>(s->ds, p, pool, in, first);
+    else
+        k_paths<kShortStack, false><<<grid, kPathBlock, 0, s->stream>>>(s->ds, p, pool, in, first);
+}
+
 // One wave: raygen, then max_depth + 1 events of trace -> shade -> shadow.
 // The shadow walks of event e run on the side stream, overlapping the closest-hit walk of
 // event e + 1 on the scene stream; the shade kernels of e + 1 wait for them.  The two walks
@@ -1533,6 +1548,13 @@ void run_wave(rp_scene *s, const WaveParams &request_params, size_t adjoint_smem
     RP_CHECK(cudaMemsetAsync(pool.counters, 0, 64 * sizeof(u32), s->stream));
     k_raygen<<<grid_for(sms, p.lanes, 256, 16), 256, 0, s->stream>>>(s->ds, p, pool);
     s->done();
+    if (p.lanes <= kWholePathLanes && !s->resolve && !s->counting && !pool.hist) {
+        s->mark(2);
+        launch_paths(s, p, pool, 0, 0, p.lanes);
+        s->done();
+        RP_CHECK(cudaGetLastError());
+        return;
+    }
     int in = 0;
     const u32 events = s->ds.max_depth + 1;
     bool shadow_pending = false;

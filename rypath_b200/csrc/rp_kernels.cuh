@@ -902,6 +902,62 @@ __global__ void __launch_bounds__(Block, Stack <= kShortStack ? 1024 / Block : 1
     }
 }
 
+// Whole paths, one thread each: every event of the queue's paths from event `first` on, each
+// the closest hit, the event, its light sample and that sample's visibility in turn, on the
+// same path state as the wavefront kernels (so every lane's result is theirs).  A wave of few
+// lanes is bound by the launches of its events (about eleven kernels each), not by their work:
+// one launch runs it instead.  Its warps diverge over the families, so it is for waves of at
+// most kWholePathLanes lanes; scenes whose hits resolve before shading take the wavefront.
+constexpr int kPathBlock = 64;
+template <int Stack, bool Img>
+__global__ void __launch_bounds__(kPathBlock, 6) k_paths(const __grid_constant__ DeviceScene s,
+                                                         const __grid_constant__ WaveParams p, PathPool pool, int in,
+                                                         u32 first) {
+    __shared__ uint2 stack[Stack * kPathBlock];
+    const u32 count = pool.counters[in];
+    for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+        const u32 path = pool.queue[in][i];
+        u32 unused = 0;
+        for (u32 e = first; e <= s.max_depth; ++e) {
+            if (pool.ident[path].w & F_COMPLETE)
+                break;
+            const float4 o = pool.ray_o[path], d = pool.ray_d[path];
+            Hit h;
+            const bool hit_ok = walk_closest<false, Stack, false>(s, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z),
+                                                                  __int_as_float(0x7f800000), h, stack + threadIdx.x,
+                                                                  kPathBlock, unused, unused);
+            const u32 prim = hit_ok ? h.prim : kHitInvalid;
+            const u32 family = !hit_ok || h.prim == kNone ? 3u : u32(__ldg(s.tri_family + h.prim));
+            pool.hit[path] = make_float4(h.t, h.b1, h.b2, __uint_as_float(prim));
+            bool keep = false, nee = false, shadow = false;
+            float4 so, sd, sc, st;
+            if (family == 0) {
+                shade_path<0, false, Img, false>(s, p, pool, true, path, nullptr, keep, nee);
+                if (nee)
+                    nee_path<0, Img, false>(s, p, pool, true, path, shadow, so, sd, sc, st);
+            } else if (family == 1) {
+                shade_path<1, false, Img, false>(s, p, pool, true, path, nullptr, keep, nee);
+                if (nee)
+                    nee_path<1, Img, false>(s, p, pool, true, path, shadow, so, sd, sc, st);
+            } else if (family == 2) {
+                shade_path<2, false, Img, false>(s, p, pool, true, path, nullptr, keep, nee);
+                if (nee)
+                    nee_path<2, Img, false>(s, p, pool, true, path, shadow, so, sd, sc, st);
+            } else {
+                shade_path<3, false, Img, false>(s, p, pool, true, path, nullptr, keep, nee);
+            }
+            if (shadow) {
+                bool occluded;
+                const bool ok = walk_any<false, Stack, false>(s, v3(so.x, so.y, so.z), v3(sd.x, sd.y, sd.z), so.w,
+                                                              occluded, stack + threadIdx.x, kPathBlock, unused, unused);
+                shadow_result<false>(s, pool, nullptr, sc, path, ok ? 0u : 3u, occluded);
+            }
+            if (!keep)
+                break;
+        }
+    }
+}
+
 // packet_pt_result (shaders/packet_pt_step.h:225-239): 80-byte packet result per lane.  The
 // reserved words, which rypath leaves unread, carry the lane's closest-hit and any-hit walk
 // counts in counting runs (zero otherwise).
