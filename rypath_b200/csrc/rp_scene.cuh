@@ -999,18 +999,21 @@ RP_DEV bool any_leaf(const DeviceScene &s, const WalkRay &r, float tmax, u32 ind
     return intersect_triangle(r, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), v3(c.x, c.y, c.z), tmax, t, b1, b2);
 }
 
-// The quantized planes of a wide node against a ray, in interval arithmetic.  Along an axis
-// the plane of byte q lies at p + q s (real arithmetic; the builder guarantees lo planes at
-// or below and hi planes at or above the child's box), and the ray reaches it at
-// t = (p - o) / d + q s / d.  With [a_lo, a_hi] containing (p - o) / d - 2^23 s / d and
-// [b_lo, b_hi] containing s / d, a lower bound of t is fmaf_rd(2^23 + q, b_lo, a_lo) and an upper
-// bound fmaf_ru(2^23 + q, b_hi, a_hi), where 2^23 + q is the float whose bits are 0x4b0000qq
-// (one byte permute).  A direction component of zero (or one whose reciprocal overflows) makes
-// that axis's bounds NaN or infinite in the direction that leaves the axis unconstrained; the
-// NaN-ignoring min and max then skip it, which is conservative.
+// The quantized planes of a wide node against a ray.  Along an axis the plane of byte q lies at
+// p + q s (real arithmetic; the builder guarantees lo planes at or below and hi planes at or
+// above the child's box), and the ray reaches it at t = (p - o) / d + q s / d.  With u = 2^-24,
+// inv = 1 / d rounded, D = (p - o) inv rounded, b = 2^15 s inv (exact) and Q = 1 + 2^-15 q, the
+// float whose bits are 0x3f80qq00 (one byte permute), t' = Q b + (D - b) in rounded arithmetic
+// is within 5.1 u |D| + 1.1 u |b| of t; taking 8 u |D| + 4 u |b| off the offset D - b for the
+// near planes and adding it for the far ones (each another u (|D| + |b|)) bounds t on either
+// side, about 2^-7 of a quantization step wider than t' itself.  A direction component of zero
+// (or one whose reciprocal overflows) makes that axis's bounds NaN or infinite in the direction
+// that leaves the axis unconstrained; the NaN-ignoring min and max then skip it, which is
+// conservative.  The bounds' multiplications and additions run on the FMA pipe: the walk is
+// bound by issue and by the ALU pipe, which the permutes, minima and maxima fill.
 struct WideRay {
-    float rcp_lo[3], rcp_hi[3]; // directed-rounding bounds of 1 / d
-    u32 negative;               // axis bits: d < 0 (the near plane is the hi one)
+    float inv[3];
+    u32 negative; // axis bits: d < 0 (the near plane is the hi one)
 };
 RP_DEV WideRay wide_ray(V3 d) {
     WideRay w;
@@ -1018,66 +1021,57 @@ RP_DEV WideRay wide_ray(V3 d) {
     w.negative = 0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        w.rcp_lo[a] = __frcp_rd(dd[a]);
-        w.rcp_hi[a] = __frcp_ru(dd[a]);
+        w.inv[a] = 1.0f / dd[a];
         w.negative |= (__float_as_uint(dd[a]) >> 31) << a;
     }
     return w;
 }
-// [lo, hi] bounds of x * y for x in [x_lo, x_hi] and y in [y_lo, y_hi] with y of one sign.
-RP_DEV void interval_mul(float x_lo, float x_hi, float y_lo, float y_hi, bool y_negative, float &lo, float &hi) {
-    if (!y_negative) {
-        lo = __fmul_rd(x_lo, x_lo >= 0 ? y_lo : y_hi);
-        hi = __fmul_ru(x_hi, x_hi >= 0 ? y_hi : y_lo);
-    } else {
-        lo = __fmul_rd(x_hi, x_hi >= 0 ? y_lo : y_hi);
-        hi = __fmul_ru(x_lo, x_lo >= 0 ? y_hi : y_lo);
-    }
-}
-RP_DEV float qfloat(u32 word, int byte) { return __uint_as_float(__byte_perm(word, 0x4b000000u, 0x7540u | u32(byte))); }
+RP_DEV float qfloat(u32 word, int byte) { return __uint_as_float(__byte_perm(word, 0x3f800000u, 0x7604u | u32(byte) << 4)); }
 
 // The children of a wide node whose boxes the ray's segment [0, tmax] may enter: internal ones
 // as bits at slot ^ order (near side first), leaves as bits at their slot.  Conservative: the
 // computed entry is at or below the true one and the exit at or above, so no child that holds
 // a hit in [0, tmax] is missed; all eight slots are tested without branches and masked.
-RP_DEV void wide_children(const WNode &n, V3 o, const WideRay &w, float tmax, u32 order, u32 &inner, u32 &leaves) {
-    const u32 meta = __float_as_uint(n.origin.w);
-    const u32 imask = meta >> 24, lmask = n.links.z;
-    const float p[3] = {n.origin.x, n.origin.y, n.origin.z}, oo[3] = {o.x, o.y, o.z};
-    // byte words of each bound row: lo.x, lo.y, lo.z, hi.x, hi.y, hi.z (slots 0-3, 4-7)
-    const u32 rows[6][2] = {{n.q0.x, n.q0.y}, {n.q0.z, n.q0.w}, {n.q1.x, n.q1.y},
-                            {n.q1.z, n.q1.w}, {n.q2.x, n.q2.y}, {n.q2.z, n.q2.w}};
+RP_DEV void wide_children(const WNode *np, float4 origin, uint4 links, V3 o, const WideRay &w, float tmax, u32 order, u32 &inner,
+                          u32 &leaves) {
+    const u32 meta = __float_as_uint(origin.w);
+    const u32 imask = meta >> 24, lmask = links.z;
+    const float p[3] = {origin.x, origin.y, origin.z}, oo[3] = {o.x, o.y, o.z};
+    // byte words of each bound row (slots 0-3, 4-7): lo.x, lo.y, lo.z, hi.x, hi.y, hi.z; the ray's
+    // near and far rows of an axis are loaded where they lie, which spares selecting them
+    const uint2 *rows = reinterpret_cast<const uint2 *>(&np->q0);
     u32 near_w[3][2], far_w[3][2];
-    float a_lo[3], a_hi[3], b_lo[3], b_hi[3]; // per axis
+    float b[3], a_near[3], a_far[3]; // per axis
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         const float s = __uint_as_float(((meta >> (8 * a)) & 0xffu) << 23);
         const bool neg = (w.negative >> a) & 1u;
-        float d_lo, d_hi;
-        // (p - o) / d, then minus 2^23 s / d
-        interval_mul(__fsub_rd(p[a], oo[a]), __fsub_ru(p[a], oo[a]), w.rcp_lo[a], w.rcp_hi[a], neg, d_lo, d_hi);
-        b_lo[a] = __fmul_rd(s, w.rcp_lo[a]);
-        b_hi[a] = __fmul_ru(s, w.rcp_hi[a]);
-        a_lo[a] = __fmaf_rd(-8388608.0f, b_hi[a], d_lo);
-        a_hi[a] = __fmaf_ru(-8388608.0f, b_lo[a], d_hi);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            near_w[a][h] = neg ? rows[3 + a][h] : rows[a][h];
-            far_w[a][h] = neg ? rows[a][h] : rows[3 + a][h];
-        }
+        const float D = (p[a] - oo[a]) * w.inv[a];
+        b[a] = (s * 32768.0f) * w.inv[a];
+        const float offset = D - b[a];
+        const float margin = fmaf(fabsf(D), 0x1p-21f, fmaf(fabsf(b[a]), 0x1p-22f, kFltMin));
+        a_near[a] = offset - margin;
+        a_far[a] = offset + margin;
+        const uint2 near = __ldg(rows + (neg ? 3 + a : a)), far = __ldg(rows + (neg ? a : 3 + a));
+        near_w[a][0] = near.x;
+        near_w[a][1] = near.y;
+        far_w[a][0] = far.x;
+        far_w[a][1] = far.y;
     }
-    u32 hits = 0;
+    u32 misses = 0;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
+    for (int k = 7; k >= 0; --k) {
         const int h = k >> 2, byte = k & 3;
         float t0 = 0.0f, t1 = tmax;
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            t0 = fmaxf(t0, __fmaf_rd(qfloat(near_w[a][h], byte), b_lo[a], a_lo[a]));
-            t1 = fminf(t1, __fmaf_ru(qfloat(far_w[a][h], byte), b_hi[a], a_hi[a]));
+            t0 = fmaxf(t0, fmaf(qfloat(near_w[a][h], byte), b[a], a_near[a]));
+            t1 = fminf(t1, fmaf(qfloat(far_w[a][h], byte), b[a], a_far[a]));
         }
-        hits |= (t0 <= t1 ? 1u : 0u) << k;
+        // the sign of t1 - t0 (an infinite pair gives a positive NaN: a hit)
+        misses = __funnelshift_l(__float_as_uint(t1 - t0), misses, 1);
     }
+    const u32 hits = ~misses;
     leaves = hits & lmask;
     u32 m = hits & imask; // to traversal order: bit k moves to k ^ order
     if (order & 1u)
@@ -1113,24 +1107,20 @@ RP_DEV bool walk_closest(const DeviceScene &s, V3 o, V3 d, float tmax, Hit &h, u
     u32 node = 0;
     for (u32 guard = 0; guard <= s.wnode_count; ++guard) {
         const WNode *np = s.wnodes + node;
-        WNode n;
-        n.origin = __ldg(&np->origin);
-        n.links = __ldg(&np->links);
-        n.q0 = __ldg(&np->q0);
-        n.q1 = __ldg(&np->q1);
-        n.q2 = __ldg(&np->q2);
+        const float4 origin = __ldg(&np->origin);
+        const uint4 links = __ldg(&np->links);
         if (Count)
             ++nodes_visited;
         u32 inner, leaves;
-        wide_children(n, o, wr, h.t, order, inner, leaves);
-        const u32 lmask = n.links.z;
+        wide_children(np, origin, links, o, wr, h.t, order, inner, leaves);
+        const u32 lmask = links.z;
         while (leaves) {
             const u32 k = __ffs(leaves) - 1;
             leaves &= leaves - 1;
-            closest_leaf<Count, Proc>(s, r, tmax, h, n.links.y + __popc(lmask & ((1u << k) - 1)), tris_tested);
+            closest_leaf<Count, Proc>(s, r, tmax, h, links.y + __popc(lmask & ((1u << k) - 1)), tris_tested);
         }
-        const u32 imask = __float_as_uint(n.origin.w) >> 24;
-        u32 base = n.links.x, group_mask = imask;
+        const u32 imask = __float_as_uint(origin.w) >> 24;
+        u32 base = links.x, group_mask = imask;
         if (!inner) {
             if (sp == 0)
                 return true;
@@ -1177,27 +1167,23 @@ RP_DEV bool walk_any(const DeviceScene &s, V3 o, V3 d, float tmax, bool &occlude
     u32 node = 0;
     for (u32 guard = 0; guard <= s.wnode_count; ++guard) {
         const WNode *np = s.wnodes + node;
-        WNode n;
-        n.origin = __ldg(&np->origin);
-        n.links = __ldg(&np->links);
-        n.q0 = __ldg(&np->q0);
-        n.q1 = __ldg(&np->q1);
-        n.q2 = __ldg(&np->q2);
+        const float4 origin = __ldg(&np->origin);
+        const uint4 links = __ldg(&np->links);
         if (Count)
             ++nodes_visited;
         u32 inner, leaves;
-        wide_children(n, o, wr, tmax, order, inner, leaves);
-        const u32 lmask = n.links.z;
+        wide_children(np, origin, links, o, wr, tmax, order, inner, leaves);
+        const u32 lmask = links.z;
         while (leaves) {
             const u32 k = __ffs(leaves) - 1;
             leaves &= leaves - 1;
-            if (any_leaf<Count, Proc>(s, r, tmax, n.links.y + __popc(lmask & ((1u << k) - 1)), tris_tested)) {
+            if (any_leaf<Count, Proc>(s, r, tmax, links.y + __popc(lmask & ((1u << k) - 1)), tris_tested)) {
                 occluded = true;
                 return true;
             }
         }
-        const u32 imask = __float_as_uint(n.origin.w) >> 24;
-        u32 base = n.links.x, group_mask = imask;
+        const u32 imask = __float_as_uint(origin.w) >> 24;
+        u32 base = links.x, group_mask = imask;
         if (!inner) {
             if (sp == 0)
                 return true;
