@@ -896,7 +896,8 @@ int grid_for(int sm_count, u32 work, int block, int per_sm) {
 // counting and without the adjoint may run on it.
 constexpr size_t pool_bytes(u32 lanes, bool full) {
     const size_t v16 = (size_t(lanes) * 16 + 255) & ~size_t(255), v4 = (size_t(lanes) * 4 + 255) & ~size_t(255);
-    return 33 * v16 + 9 * v4 + 256 + (full ? v16 + 3 * v4 : 0);
+    const size_t v8 = (size_t(lanes) * 8 + 255) & ~size_t(255);
+    return 25 * v16 + v8 + 9 * v4 + 256 + (full ? v16 + 3 * v4 : 0);
 }
 size_t carve_pool(unsigned char *base, u32 lanes, bool full, PathPool *out) {
     const size_t v16 = (size_t(lanes) * 16 + 255) & ~size_t(255), v4 = (size_t(lanes) * 4 + 255) & ~size_t(255);
@@ -908,19 +909,14 @@ size_t carve_pool(unsigned char *base, u32 lanes, bool full, PathPool *out) {
     };
     PathPool q{};
     q.ident = reinterpret_cast<uint4 *>(take(v16));
-    q.cursor = reinterpret_cast<uint4 *>(take(v16));
-    float4 **f4[] = {&q.lambda, &q.lambda_pdf, &q.beta, &q.radiance, &q.dens_f, &q.prev_f, &q.eta_scale, &q.ray_o,
-                     &q.ray_d, &q.latest_p, &q.latest_n, &q.latest_param, &q.latest_k, &q.preceding, &q.hit,
-                     &q.sh_o, &q.sh_d, &q.sh_c};
+    q.index = reinterpret_cast<uint2 *>(take((size_t(lanes) * 8 + 255) & ~size_t(255)));
+    float4 **f4[] = {&q.lambda, &q.lambda_pdf, &q.beta, &q.radiance, &q.dens_f[0], &q.dens_f[1], &q.eta_scale, &q.ray_o,
+                     &q.ray_d[0], &q.ray_d[1], &q.latest_p[0], &q.latest_p[1], &q.latest_n, &q.latest_param, &q.latest_k,
+                     &q.hit, &q.sh_o, &q.sh_d, &q.sh_c, &q.nee_g, &q.nee_e, &q.nee_beta};
     for (auto p : f4)
         *p = reinterpret_cast<float4 *>(take(v16));
-    q.dens_e = reinterpret_cast<int4 *>(take(v16));
-    q.prev_e = reinterpret_cast<int4 *>(take(v16));
-    float4 **nee[] = {&q.nee_p, &q.nee_n, &q.nee_g, &q.nee_e, &q.nee_wo, &q.nee_prev, &q.nee_beta, &q.nee_df,
-                      &q.nee_param, &q.nee_k};
-    for (auto p : nee)
-        *p = reinterpret_cast<float4 *>(take(v16));
-    q.nee_de = reinterpret_cast<int4 *>(take(v16));
+    q.dens_e[0] = reinterpret_cast<int4 *>(take(v16));
+    q.dens_e[1] = reinterpret_cast<int4 *>(take(v16));
     q.queue[0] = reinterpret_cast<u32 *>(take(v4));
     q.queue[1] = reinterpret_cast<u32 *>(take(v4));
     q.bins = reinterpret_cast<u32 *>(take(4 * v4));
@@ -941,7 +937,7 @@ size_t carve_pool(unsigned char *base, u32 lanes, bool full, PathPool *out) {
 }
 // Every PathPool member is a pointer carved above, set elsewhere (stats, the adjoint's), or
 // a count: a new member changes this size and so comes past this check.
-static_assert(sizeof(PathPool) == 50 * sizeof(void *) + 16, "PathPool changed: review carve_pool");
+static_assert(sizeof(PathPool) == 43 * sizeof(void *) + 16, "PathPool changed: review carve_pool");
 
 } // namespace
 
@@ -1407,30 +1403,30 @@ void launch_shadow(const rp_scene *s, const PathPool &pool, int in, unsigned gri
 // others: it is short, and a fork and a join cost more than it.
 constexpr int kShadeBlock = 256;
 template <int F, int Block, bool Adjoint, bool Img>
-void launch_family(rp_scene *s, const WaveParams &p, const PathPool &pool, int in, unsigned grid, size_t smem,
+void launch_family(rp_scene *s, const WaveParams &p, const PathPool &pool, int in, u32 event, unsigned grid, size_t smem,
                    cudaStream_t st) {
     // counting runs time each family kernel alone: all run one after another on the scene
     // stream, so each one's events bracket its own work (side by side they share the SMs)
     if (s->counting)
         s->mark_family(F, st);
-    k_shade<F, Block, Adjoint, Img><<<grid, Block, smem, st>>>(s->ds, p, pool, in);
+    k_shade<F, Block, Adjoint, Img><<<grid, Block, smem, st>>>(s->ds, p, pool, in, event);
     if constexpr (F != 3)
-        k_nee<F, Block, Img><<<grid, Block, 0, st>>>(s->ds, p, pool, in);
+        k_nee<F, Block, Img><<<grid, Block, 0, st>>>(s->ds, p, pool, in, event);
     if (s->counting)
         s->done_family(st);
 }
 template <int Block, bool Adjoint, bool Img>
-void launch_families(rp_scene *s, const WaveParams &p, const PathPool &pool, int in, unsigned grid, size_t smem) {
+void launch_families(rp_scene *s, const WaveParams &p, const PathPool &pool, int in, u32 event, unsigned grid, size_t smem) {
     const u32 mask = s->family_mask;
     const bool fork = !s->counting && (mask & (mask - 1)) != 0;
     if (!fork) {
-        launch_family<3, Block, Adjoint, Img>(s, p, pool, in, grid, smem, s->stream);
+        launch_family<3, Block, Adjoint, Img>(s, p, pool, in, event, grid, smem, s->stream);
         if (mask & 1u)
-            launch_family<0, Block, Adjoint, Img>(s, p, pool, in, grid, smem, s->stream);
+            launch_family<0, Block, Adjoint, Img>(s, p, pool, in, event, grid, smem, s->stream);
         if (mask & 2u)
-            launch_family<1, Block, Adjoint, Img>(s, p, pool, in, grid, smem, s->stream);
+            launch_family<1, Block, Adjoint, Img>(s, p, pool, in, event, grid, smem, s->stream);
         if (mask & 4u)
-            launch_family<2, Block, Adjoint, Img>(s, p, pool, in, grid, smem, s->stream);
+            launch_family<2, Block, Adjoint, Img>(s, p, pool, in, event, grid, smem, s->stream);
         return;
     }
     const bool used[3] = {(mask & 2u) != 0, (mask & 4u) != 0, true};
@@ -1439,12 +1435,12 @@ void launch_families(rp_scene *s, const WaveParams &p, const PathPool &pool, int
         if (used[k])
             RP_CHECK(cudaStreamWaitEvent(s->family[k], s->forked, 0));
     if (mask & 1u)
-        launch_family<0, Block, Adjoint, Img>(s, p, pool, in, grid, smem, s->stream);
+        launch_family<0, Block, Adjoint, Img>(s, p, pool, in, event, grid, smem, s->stream);
     if (mask & 2u)
-        launch_family<1, Block, Adjoint, Img>(s, p, pool, in, grid, smem, s->family[0]);
+        launch_family<1, Block, Adjoint, Img>(s, p, pool, in, event, grid, smem, s->family[0]);
     if (mask & 4u)
-        launch_family<2, Block, Adjoint, Img>(s, p, pool, in, grid, smem, s->family[1]);
-    launch_family<3, Block, Adjoint, Img>(s, p, pool, in, grid, smem, s->family[2]);
+        launch_family<2, Block, Adjoint, Img>(s, p, pool, in, event, grid, smem, s->family[1]);
+    launch_family<3, Block, Adjoint, Img>(s, p, pool, in, event, grid, smem, s->family[2]);
     for (int k = 0; k < 3; ++k)
         if (used[k]) {
             RP_CHECK(cudaEventRecord(s->family_done[k], s->family[k]));
@@ -1454,14 +1450,14 @@ void launch_families(rp_scene *s, const WaveParams &p, const PathPool &pool, int
 u32 family_kernels(const rp_scene *s) { return 2 * u32(__builtin_popcount(s->family_mask)) + 1; }
 // The plain shade kernels for scenes without images (the adjoint keeps the full ones).
 template <int Block, bool Adjoint>
-void launch_shade(rp_scene *s, const WaveParams &p, const PathPool &pool, int in, unsigned grid, size_t smem) {
+void launch_shade(rp_scene *s, const WaveParams &p, const PathPool &pool, int in, u32 event, unsigned grid, size_t smem) {
     if constexpr (!Adjoint) {
         if (!s->ds.img.textured && s->ds.img.env_image == kNone) {
-            launch_families<Block, false, false>(s, p, pool, in, grid, smem);
+            launch_families<Block, false, false>(s, p, pool, in, event, grid, smem);
             return;
         }
     }
-    launch_families<Block, Adjoint, true>(s, p, pool, in, grid, smem);
+    launch_families<Block, Adjoint, true>(s, p, pool, in, event, grid, smem);
 }
 
 // Sobol sampler with Owen randomisation: attaches the tables of the draw blocks of the scene's
@@ -1514,17 +1510,17 @@ void attach_draw_tables(rp_scene *s, WaveParams &p) {
 
 // Waves of at most this many lanes run as whole paths (k_paths).
 constexpr u32 kWholePathLanes = 32768;
-void launch_paths(rp_scene *s, const WaveParams &p, const PathPool &pool, int in, u32 first, u32 lanes) {
-    const unsigned grid = grid_for(s->sm_count, lanes, kPathBlock, 64);
+void launch_paths(rp_scene *s, const WaveParams &p, const PathPool &pool) {
+    const unsigned grid = grid_for(s->sm_count, p.lanes, kPathBlock, 64);
     const bool img = s->ds.img.textured || s->ds.img.env_image != kNone, deep = s->wide_levels > u32(kShortStack);
     if (img && deep)
-        k_paths<kStackDepth, true><<<grid, kPathBlock, 0, s->stream>>>(s->ds, p, pool, in, first);
+        k_paths<kStackDepth, true><<<grid, kPathBlock, 0, s->stream>>>(s->ds, p, pool);
     else if (img)
-        k_paths<kShortStack, true><<<grid, kPathBlock, 0, s->stream>>>(s->ds, p, pool, in, first);
+        k_paths<kShortStack, true><<<grid, kPathBlock, 0, s->stream>>>(s->ds, p, pool);
     else if (deep)
-        k_paths<kStackDepth, false><<<grid, kPathBlock, 0, s->stream>>>(s->ds, p, pool, in, first);
+        k_paths<kStackDepth, false><<<grid, kPathBlock, 0, s->stream>>>(s->ds, p, pool);
     else
-        k_paths<kShortStack, false><<<grid, kPathBlock, 0, s->stream>>>(s->ds, p, pool, in, first);
+        k_paths<kShortStack, false><<<grid, kPathBlock, 0, s->stream>>>(s->ds, p, pool);
 }
 
 // One wave: raygen, then max_depth + 1 events of trace -> shade -> shadow.
@@ -1550,7 +1546,7 @@ void run_wave(rp_scene *s, const WaveParams &request_params, size_t adjoint_smem
     s->done();
     if (p.lanes <= kWholePathLanes && !s->resolve && !s->counting && !pool.hist) {
         s->mark(2);
-        launch_paths(s, p, pool, 0, 0, p.lanes);
+        launch_paths(s, p, pool);
         s->done();
         RP_CHECK(cudaGetLastError());
         return;
@@ -1574,9 +1570,9 @@ void run_wave(rp_scene *s, const WaveParams &request_params, size_t adjoint_smem
         const size_t smem = adjoint_smem;
         const unsigned shade_grid = grid_for(sms, p.lanes, kShadeBlock, 2048 / kShadeBlock);
         if (pool.hist)
-            launch_shade<kShadeBlock, true>(s, p, pool, in, shade_grid, smem);
+            launch_shade<kShadeBlock, true>(s, p, pool, in, e, shade_grid, smem);
         else
-            launch_shade<kShadeBlock, false>(s, p, pool, in, shade_grid, 0);
+            launch_shade<kShadeBlock, false>(s, p, pool, in, e, shade_grid, 0);
         s->done();
         RP_CHECK(cudaEventRecord(s->forked, s->stream));
         RP_CHECK(cudaStreamWaitEvent(s->side, s->forked, 0));
@@ -3087,7 +3083,7 @@ void batch_wave_kernels(rp_scene *s, const WaveParams &p, const Batch &b, u32 wa
             RP_CHECK(cudaStreamWaitEvent(st, s->joined, 0));
             shadow_pending = false;
         }
-        launch_shade<SB, false>(s, p, pool, in, shade_grid, 0);
+        launch_shade<SB, false>(s, p, pool, in, e, shade_grid, 0);
         RP_CHECK(cudaEventRecord(s->forked, st));
         RP_CHECK(cudaStreamWaitEvent(s->side, s->forked, 0));
         launch_shadow<false, TB, false>(s, pool, in, trace_grid, 0, s->side, p.boundary_limit);
@@ -3941,9 +3937,8 @@ static __device__ __align__(256) unsigned char g_static_scratch[RP_STATIC_SCRATC
 
 namespace {
 
-static_assert(pool_bytes(RP_STATIC_MAX_LANES, false) <= RP_STATIC_SCRATCH_BYTES &&
-                  pool_bytes(RP_STATIC_MAX_LANES + 1, false) > RP_STATIC_SCRATCH_BYTES,
-              "RP_STATIC_MAX_LANES is the largest request that fits the static scratch");
+static_assert(pool_bytes(RP_STATIC_MAX_LANES, false) <= RP_STATIC_SCRATCH_BYTES,
+              "a request of RP_STATIC_MAX_LANES fits the static scratch");
 
 // Device address of the scratch array in the current device's context.  The caller keeps it
 // with the scene, whose own device memory lives in the same context: a scene cannot outlive
@@ -4012,18 +4007,18 @@ rp_status rp_cuda_sample_device_static(rp_scene *s, const rp_request *request, r
         for (u32 ev = 0; ev < s->ds.max_depth + 1; ++ev) {
             launch_trace<false, kTraceBlock>(s, pool, in, grid_for(sms, p.lanes, kTraceBlock, 12), st, p.boundary_limit);
             const unsigned shade_grid = grid_for(sms, p.lanes, 128, 16);
-            k_shade<3><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in);
+            k_shade<3><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in, ev);
             if (s->family_mask & 1u) {
-                k_shade<0><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in);
-                k_nee<0><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in);
+                k_shade<0><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in, ev);
+                k_nee<0><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in, ev);
             }
             if (s->family_mask & 2u) {
-                k_shade<1><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in);
-                k_nee<1><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in);
+                k_shade<1><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in, ev);
+                k_nee<1><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in, ev);
             }
             if (s->family_mask & 4u) {
-                k_shade<2><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in);
-                k_nee<2><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in);
+                k_shade<2><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in, ev);
+                k_nee<2><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in, ev);
             }
             launch_shadow<false, kTraceBlock, false>(s, pool, in, grid_for(sms, p.lanes, kTraceBlock, 12), 0, st, p.boundary_limit);
             in ^= 1;

@@ -33,17 +33,17 @@ RP_DEV void raygen_lane(const DeviceScene &s, const RasterCam &cam, const WavePa
         if (!finite3(o) || !finite3(d))
             flags = set_status(flags, 2) | F_COMPLETE;
         pool.ident[slot] = make_uint4(b.pixel, b.sample_low, b.sample_high, flags);
-        pool.cursor[slot] = make_uint4(u32(b.index), u32(b.index >> 32), 1, slot);
+        pool.index[slot] = make_uint2(u32(b.index), u32(b.index >> 32));
         pool.lambda[slot] = to_float4(lambda);
         pool.lambda_pdf[slot] = to_float4(pdf);
         pool.beta[slot] = make_float4(1, 1, 1, 1);
         pool.radiance[slot] = make_float4(0, 0, 0, 0);
-        pool.dens_f[slot] = pool.prev_f[slot] = make_float4(.5f, .5f, .5f, .5f);
-        pool.dens_e[slot] = pool.prev_e[slot] = make_int4(1, 1, 1, 1);
+        pool.dens_f[0][slot] = make_float4(.5f, .5f, .5f, .5f); // read before [1] is
+        pool.dens_e[0][slot] = make_int4(1, 1, 1, 1);
         pool.eta_scale[slot] = make_float4(1, 1, 1, 1);
         pool.ray_o[slot] = make_float4(o.x, o.y, o.z, 0);
-        pool.ray_d[slot] = make_float4(d.x, d.y, d.z, 0);
-        pool.latest_p[slot] = make_float4(o.x, o.y, o.z, 0);
+        pool.ray_d[0][slot] = make_float4(d.x, d.y, d.z, 0);
+        pool.latest_p[0][slot] = make_float4(o.x, o.y, o.z, 0);
         pool.latest_n[slot] = make_float4(0, 0, 0, 0);
         pool.queue[0][slot] = slot;
         if (pool.lane_closest) {
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(Block, Stack <= kShortStack ? 1024 / Block : 1
         if (i < count) {
             path = queue[i];
             if (!(pool.ident[path].w & F_COMPLETE)) {
-                const float4 o = pool.ray_o[path], d = pool.ray_d[path];
+                const float4 o = pool.ray_o[path], d = pool.ray_d[in][path];
                 const u32 walks_before = rays;
                 Hit h;
                 const bool ok = walk_closest<Count, Stack, Resolve>(s, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z),
@@ -205,33 +205,33 @@ template <bool Sync> RP_DEV void phase() {
 }
 // One hero event of path `path` after its closest hit (shaders/packet_pt_event_body.inc:11-461),
 // a hit of BSDF family F (3: no surface -- environment or a failed query).  keep: the path
-// goes on; nee: its event left a light-sample request.  Sync: the whole block calls this
+// goes on; nee: its event left a light-sample request.  in: the parity of its queue;
+// event_index: events before this one (every path of the wave has had as many).  Sync: the whole block calls this
 // (`active` clear where it has no path), and its warps meet between the phases of the event.
 template <int F, bool Adjoint, bool Img, bool Sync>
-RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool &pool, bool active, u32 path, float *sgrad,
-                       bool &keep, bool &nee) {
+RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool &pool, int in, u32 event_index,
+                       bool active, u32 path, float *sgrad, bool &keep, bool &nee) {
     const u32 capacity = s.max_depth + 2;
     uint4 ident = pool.ident[path];
     u32 flags = ident.w;
     active = active && !(flags & F_COMPLETE);
     {
-        uint4 cursor = pool.cursor[path];
-        const u64 index = (u64(cursor.y) << 32) | cursor.x;
-        u32 cnt = cursor.z;
+        const uint2 index2 = pool.index[path];
+        const u64 index = (u64(index2.y) << 32) | index2.x;
+        u32 cnt = event_index + 1; // vertices so far, the camera's included
         const V4 lambda = from_float4(pool.lambda[path]);
         V4 beta = from_float4(pool.beta[path]);
-        V4 radiance = from_float4(pool.radiance[path]);
-        Density density = load_density(pool.dens_f[path], pool.dens_e[path]);
-        const Density previous_density = load_density(pool.prev_f[path], pool.prev_e[path]);
-        Density hero_previous = previous_density;
-        V4 eta_scale = from_float4(pool.eta_scale[path]);
+        Density density = load_density(pool.dens_f[in][path], pool.dens_e[in][path]);
+        V4 eta_scale = v4(1);
+        if (event_index)
+            eta_scale = from_float4(pool.eta_scale[path]);
         bool roulette = (flags & F_ROULETTE) != 0;
         u32 active_mask = flags & F_MASK;
-        const float4 ro4 = pool.ray_o[path], rd4 = pool.ray_d[path];
+        const float4 ro4 = pool.ray_o[path], rd4 = pool.ray_d[in][path];
         V3 ro = v3(ro4.x, ro4.y, ro4.z), rd = v3(rd4.x, rd4.y, rd4.z);
         const float4 hit = pool.hit[path];
         u32 status = get_status(flags);
-        Density direct_density = density;
+        const Density direct_density = density;
         V4 direct_beta = beta;
         bool direct_allowed = true;
         const u32 old_count = cnt;
@@ -353,7 +353,6 @@ RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool
                 draws = draw_words(s, p, ident.x, ident.y, ident.z, index, 4 + cnt - 2, set);
                 swo = to_local(cframe, cwo);
                 cbsdf.active_mask = active_mask;
-                direct_density = density;
                 direct_allowed = hero_continue(beta, eta_scale, roulette, cnt - 1, sample_uniform(p, draws.w));
                 direct_beta = beta;
                 connectible = hero_connectible(cbsdf);
@@ -365,7 +364,6 @@ RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool
                                                         sample_uniform(p, draws.y), sample_uniform(p, draws.z));
                 bool cont_valid = proposed.valid;
                 if (proposed.valid && proposed.accepted) {
-                    hero_previous = direct_density;
                     const Update adv = advance(direct_density, beta, proposed.numerator, proposed.pdf);
                     cont_valid = adv.valid;
                     if (adv.valid) {
@@ -408,18 +406,14 @@ RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool
         }
         phase<Sync>();
         bool complete = terminated || status != 0 || cnt >= capacity || !nonzero4(beta);
-        // latest vertex (the previous event's) for MIS
-        const float4 lp4 = pool.latest_p[path], ln4 = pool.latest_n[path];
+        // latest vertex (the previous event's) for MIS; what only a weighted emission reads of
+        // it is loaded there
         Latest latest;
         latest.type = (flags >> F_LTYPE_SHIFT) & 3u;
         latest.kind = (flags >> F_LKIND_SHIFT) & 3u;
         latest.mask = (flags >> F_LMASK_SHIFT) & 15u;
         latest.delta = (flags & F_LDELTA) != 0;
         latest.smooth = (flags & F_LSMOOTH) != 0;
-        latest.position = v3(lp4.x, lp4.y, lp4.z);
-        latest.shading_normal = v3(ln4.x, ln4.y, ln4.z);
-        latest.alpha_x = lp4.w;
-        latest.alpha_y = ln4.w;
         if (cnt != old_count && status == 0) {
             // hero_endpoint (shaders/hero_pt_helpers.h:157-184)
             V4 rad = v4(0);
@@ -434,9 +428,13 @@ RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool
                 }
                 emission_ok = finite_nonnegative4(rad);
             } else {
-                const V3 delta = latest.position - cp.position;
                 const DInstance &instance = s.instances[cinst];
-                if (!zero3(delta) && instance.emission != kNone) {
+                V3 delta = v3(0, 0, 0);
+                if (instance.emission != kNone) {
+                    const float4 lp4 = pool.latest_p[in][path];
+                    delta = v3(lp4.x, lp4.y, lp4.z) - cp.position;
+                }
+                if (!zero3(delta)) {
                     const V3 dir = normalize3(delta);
                     if (s.emission_two_sided[instance.emission] || dot(cp.geometric_normal, dir) > 0) {
                         const u32 off = instance.emission * 471u;
@@ -455,9 +453,15 @@ RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool
                 if (cnt <= 2 || latest.delta || !nonzero4(value)) {
                     endpoint = value;
                 } else {
+                    const float4 lp4 = pool.latest_p[in][path], ln4 = pool.latest_n[path];
+                    latest.position = v3(lp4.x, lp4.y, lp4.z);
+                    latest.shading_normal = v3(ln4.x, ln4.y, ln4.z);
+                    latest.alpha_x = lp4.w;
+                    latest.alpha_y = ln4.w;
                     latest.param = from_float4(pool.latest_param[path]);
-                    latest.k = from_float4(pool.latest_k[path]);
-                    const float4 pre = pool.preceding[path];
+                    latest.k = latest.kind == 1 ? from_float4(pool.latest_k[path]) : v4(0);
+                    const float4 pre = pool.latest_p[in ^ 1][path]; // the vertex before it
+                    const Density previous_density = load_density(pool.dens_f[in ^ 1][path], pool.dens_e[in ^ 1][path]);
                     bool ok;
                     const V4 bsdf_pdf = represented_pdf<-1>(latest_bsdf(latest), latest.shading_normal, latest.position,
                                                         v3(pre.x, pre.y, pre.z), ctype == kEnvironment,
@@ -481,7 +485,13 @@ RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool
                         status = 2;
                 }
             }
-            radiance = add4(radiance, endpoint);
+            // radiance is finite and nonnegative while its path lives; a zero endpoint leaves it
+            bool radiance_ok = true;
+            if (endpoint.v[0] != 0 || endpoint.v[1] != 0 || endpoint.v[2] != 0 || endpoint.v[3] != 0) {
+                const V4 radiance = add4(from_float4(pool.radiance[path]), endpoint);
+                pool.radiance[path] = to_float4(radiance);
+                radiance_ok = finite_nonnegative4(radiance);
+            }
             if (Adjoint) {
                 // replay: the emission's gradient over the vertices before this one,
                 // then this diffuse vertex joins the history of what follows it
@@ -497,38 +507,38 @@ RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool
                 }
             }
             // hero_direct (shaders/hero_pt_helpers.h:185-221) runs in the light-sample kernel
-            // (k_nee), from the request this event leaves (write_nee_request); its failures fail the
-            // path there.
+            // (k_nee), from the request this event leaves; its failures fail the path there.
             nee = F != 3 && status == 0 && cnt < capacity && direct_allowed && ctype == kSurface && connectible;
-            if (!finite_nonnegative4(radiance))
+            if (!radiance_ok)
                 status = 2;
             if (status != 0) {
                 complete = true;
                 nee = false;
             }
             if (nee) {
-                Density dd = direct_density;
-                write_nee_request(pool, path, cnt, cp, cbsdf, cwo, latest.position, direct_beta, dd);
+                pool.nee_g[path] = make_float4(cp.geometric_normal.x, cp.geometric_normal.y, cp.geometric_normal.z, 0);
+                pool.nee_e[path] = make_float4(cp.error.x, cp.error.y, cp.error.z, 0);
+                pool.nee_beta[path] = to_float4(direct_beta);
             }
         }
         phase<Sync>();
         if (!active)
             return;
-        // A complete path is read again only for its identity, status and radiance (the
-        // shadow walk, the film and the packet results), so the rest of its state is not
-        // written back.
+        // A complete path is read again only for its identity, status and radiance (the shadow
+        // walk, the film and the packet results) and, with a light sample, its vertex, so the
+        // rest of its state is not written back.
         if (cnt != old_count) {
             // preceding = latest; latest = current (shaders/packet_pt_event_body.inc:453-460)
             flags = (flags & ~(3u << F_PTYPE_SHIFT)) | (latest.type << F_PTYPE_SHIFT);
-            if (!complete) {
-                pool.preceding[path] = make_float4(latest.position.x, latest.position.y, latest.position.z, 0);
-                pool.latest_p[path] =
+            if (!complete || nee) {
+                pool.latest_p[in ^ 1][path] =
                     make_float4(cp.position.x, cp.position.y, cp.position.z, cbsdf.g.alpha_x);
                 pool.latest_n[path] =
                     make_float4(cp.shading_normal.x, cp.shading_normal.y, cp.shading_normal.z, cbsdf.g.alpha_y);
                 pool.latest_param[path] =
                     make_float4(cbsdf.param[0], cbsdf.param[1], cbsdf.param[2], cbsdf.param[3]);
-                pool.latest_k[path] = make_float4(cbsdf.k[0], cbsdf.k[1], cbsdf.k[2], cbsdf.k[3]);
+                if (F == 1)
+                    pool.latest_k[path] = make_float4(cbsdf.k[0], cbsdf.k[1], cbsdf.k[2], cbsdf.k[3]);
             }
             flags &= ~((3u << F_LTYPE_SHIFT) | F_LDELTA | (3u << F_LKIND_SHIFT) | (15u << F_LMASK_SHIFT) | F_LSMOOTH);
             flags |= (ctype << F_LTYPE_SHIFT) | (cdelta ? F_LDELTA : 0u) | ((cbsdf.kind & 3u) << F_LKIND_SHIFT) |
@@ -538,22 +548,17 @@ RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool
         flags = set_status(flags, status) | (complete ? F_COMPLETE : 0u);
         ident.w = flags;
         pool.ident[path] = ident;
-        pool.radiance[path] = to_float4(radiance);
         if (!complete) {
-            cursor.z = cnt;
-            pool.cursor[path] = cursor;
             pool.beta[path] = to_float4(beta);
             float4 f;
             int4 e;
             store_density(density, f, e);
-            pool.dens_f[path] = f;
-            pool.dens_e[path] = e;
-            store_density(hero_previous, f, e);
-            pool.prev_f[path] = f;
-            pool.prev_e[path] = e;
-            pool.eta_scale[path] = to_float4(eta_scale);
+            pool.dens_f[in ^ 1][path] = f;
+            pool.dens_e[in ^ 1][path] = e;
+            if (F == 2)
+                pool.eta_scale[path] = to_float4(eta_scale); // only transmission changes it
             pool.ray_o[path] = make_float4(ro.x, ro.y, ro.z, 0);
-            pool.ray_d[path] = make_float4(rd.x, rd.y, rd.z, 0);
+            pool.ray_d[in ^ 1][path] = make_float4(rd.x, rd.y, rd.z, 0);
         }
         keep = !complete;
     }
@@ -568,7 +573,8 @@ RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool
 // the plain kernels).
 template <int F, int Block = 128, bool Adjoint = false, bool Img = true>
 __global__ void __launch_bounds__(Block, 512 / Block) k_shade(const __grid_constant__ DeviceScene s,
-                                                              const __grid_constant__ WaveParams p, PathPool pool, int in) {
+                                                              const __grid_constant__ WaveParams p, PathPool pool, int in,
+                                                              u32 event_index) {
     extern __shared__ float sgrad[]; // adjoint only
     if (Adjoint)
         adjoint_begin(pool, sgrad);
@@ -589,7 +595,7 @@ __global__ void __launch_bounds__(Block, 512 / Block) k_shade(const __grid_const
         const bool active = i < count;
         if (active)
             path = queue[i];
-        shade_path<F, Adjoint, Img, true>(s, p, pool, active, path, sgrad, keep, nee);
+        shade_path<F, Adjoint, Img, true>(s, p, pool, in, event_index, active, path, sgrad, keep, nee);
         const u32 slot = warp_append(out_count, keep);
         if (keep)
             out_queue[slot] = path;
@@ -607,26 +613,25 @@ __global__ void __launch_bounds__(Block, 512 / Block) k_shade(const __grid_const
 // path whose event (of BSDF family F) asked for one: light selection, the light's point and
 // radiance, the BSDF on the light direction, the balance weight, and the visibility segment
 // (shadow set).  Its own failures (invalid arithmetic) fail the path.  Split
-// from the shade kernel, which leaves the request (write_nee_request), so that each kernel
+// from the shade kernel, which leaves the request, so that each kernel
 // holds half the live state.
 template <int F, bool Img, bool Sync>
-RP_DEV void nee_path(const DeviceScene &s, const WaveParams &p, const PathPool &pool, bool active, u32 path, bool &shadow,
-                     float4 &sh_o, float4 &sh_d, float4 &sh_c, float4 &sh_t) {
+RP_DEV void nee_path(const DeviceScene &s, const WaveParams &p, const PathPool &pool, int in, u32 event_index, bool active,
+                     u32 path, bool &shadow, float4 &sh_o, float4 &sh_d, float4 &sh_c, float4 &sh_t) {
     uint4 ident = pool.ident[path];
-    const uint4 cursor = pool.cursor[path];
-    const u64 index = (u64(cursor.y) << 32) | cursor.x;
+    const uint2 index2 = pool.index[path];
+    const u64 index = (u64(index2.y) << 32) | index2.x;
     const V4 lambda = from_float4(pool.lambda[path]);
-    u32 cnt;
     SurfacePoint cp;
     HeroBsdf cbsdf;
     V3 cwo, previous;
     V4 direct_beta;
     Density direct_density;
-    read_nee_request(pool, path, cnt, cp, cbsdf, cwo, previous, direct_beta, direct_density);
+    read_nee_request<F>(pool, in, path, ident.w, cp, cbsdf, cwo, previous, direct_beta, direct_density);
     u32 status = 0;
     // the light-sample draw: its first word selects the light; the next two, a point on an
     // area light, are drawn only when an area light was selected (the same words either way)
-    const u32 block = 133 + cnt - 2;
+    const u32 block = 133 + event_index;
     // sample_li (shaders/packet_transport.h:470-553)
     float selected_pmf = 0; // light_pmf of the selected light
     Selected choice{kNone, 0};
@@ -766,7 +771,8 @@ RP_DEV void nee_path(const DeviceScene &s, const WaveParams &p, const PathPool &
 // kernel.
 template <int F, int Block = 128, bool Img = true>
 __global__ void __launch_bounds__(Block, 512 / Block) k_nee(const __grid_constant__ DeviceScene s,
-                                                            const __grid_constant__ WaveParams p, PathPool pool, int in) {
+                                                            const __grid_constant__ WaveParams p, PathPool pool, int in,
+                                                            u32 event_index) {
     u32 *event = pool.event(in);
     const u32 count = event[kNeeCount + F];
     const u32 *queue = pool.nee_queue + size_t(F) * pool.bin_capacity;
@@ -777,7 +783,7 @@ __global__ void __launch_bounds__(Block, 512 / Block) k_nee(const __grid_constan
         bool shadow = false;
         float4 sh_o = make_float4(0, 0, 0, 0), sh_d = sh_o, sh_c = sh_o, sh_t = sh_o;
         const bool active = i < count;
-        nee_path<F, Img, true>(s, p, pool, active, active ? queue[i] : 0, shadow, sh_o, sh_d, sh_c, sh_t);
+        nee_path<F, Img, true>(s, p, pool, in, event_index, active, active ? queue[i] : 0, shadow, sh_o, sh_d, sh_c, sh_t);
         const u32 sslot = warp_append(event + kShadowCount, shadow);
         if (shadow) {
             pool.sh_o[sslot] = sh_o;
@@ -902,8 +908,7 @@ __global__ void __launch_bounds__(Block, Stack <= kShortStack ? 1024 / Block : 1
     }
 }
 
-// Whole paths, one thread each: every event of the queue's paths from event `first` on, each
-// the closest hit, the event, its light sample and that sample's visibility in turn, on the
+// Whole paths, one thread each: every event of a wave's paths, each the closest hit, the event, its light sample and that sample's visibility in turn, on the
 // same path state as the wavefront kernels (so every lane's result is theirs).  A wave of few
 // lanes is bound by the launches of its events (about eleven kernels each), not by their work:
 // one launch runs it instead.  Its warps diverge over the families, so it is for waves of at
@@ -911,17 +916,15 @@ __global__ void __launch_bounds__(Block, Stack <= kShortStack ? 1024 / Block : 1
 constexpr int kPathBlock = 64;
 template <int Stack, bool Img>
 __global__ void __launch_bounds__(kPathBlock, 6) k_paths(const __grid_constant__ DeviceScene s,
-                                                         const __grid_constant__ WaveParams p, PathPool pool, int in,
-                                                         u32 first) {
+                                                         const __grid_constant__ WaveParams p, PathPool pool) {
     __shared__ uint2 stack[Stack * kPathBlock];
-    const u32 count = pool.counters[in];
-    for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-        const u32 path = pool.queue[in][i];
+    for (u32 path = blockIdx.x * blockDim.x + threadIdx.x; path < p.lanes; path += gridDim.x * blockDim.x) {
         u32 unused = 0;
-        for (u32 e = first; e <= s.max_depth; ++e) {
+        for (u32 e = 0; e <= s.max_depth; ++e) {
+            const int in = int(e & 1u);
             if (pool.ident[path].w & F_COMPLETE)
                 break;
-            const float4 o = pool.ray_o[path], d = pool.ray_d[path];
+            const float4 o = pool.ray_o[path], d = pool.ray_d[in][path];
             Hit h;
             const bool hit_ok = walk_closest<false, Stack, false>(s, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z),
                                                                   __int_as_float(0x7f800000), h, stack + threadIdx.x,
@@ -932,19 +935,19 @@ __global__ void __launch_bounds__(kPathBlock, 6) k_paths(const __grid_constant__
             bool keep = false, nee = false, shadow = false;
             float4 so, sd, sc, st;
             if (family == 0) {
-                shade_path<0, false, Img, false>(s, p, pool, true, path, nullptr, keep, nee);
+                shade_path<0, false, Img, false>(s, p, pool, in, e, true, path, nullptr, keep, nee);
                 if (nee)
-                    nee_path<0, Img, false>(s, p, pool, true, path, shadow, so, sd, sc, st);
+                    nee_path<0, Img, false>(s, p, pool, in, e, true, path, shadow, so, sd, sc, st);
             } else if (family == 1) {
-                shade_path<1, false, Img, false>(s, p, pool, true, path, nullptr, keep, nee);
+                shade_path<1, false, Img, false>(s, p, pool, in, e, true, path, nullptr, keep, nee);
                 if (nee)
-                    nee_path<1, Img, false>(s, p, pool, true, path, shadow, so, sd, sc, st);
+                    nee_path<1, Img, false>(s, p, pool, in, e, true, path, shadow, so, sd, sc, st);
             } else if (family == 2) {
-                shade_path<2, false, Img, false>(s, p, pool, true, path, nullptr, keep, nee);
+                shade_path<2, false, Img, false>(s, p, pool, in, e, true, path, nullptr, keep, nee);
                 if (nee)
-                    nee_path<2, Img, false>(s, p, pool, true, path, shadow, so, sd, sc, st);
+                    nee_path<2, Img, false>(s, p, pool, in, e, true, path, shadow, so, sd, sc, st);
             } else {
-                shade_path<3, false, Img, false>(s, p, pool, true, path, nullptr, keep, nee);
+                shade_path<3, false, Img, false>(s, p, pool, in, e, true, path, nullptr, keep, nee);
             }
             if (shadow) {
                 bool occluded;

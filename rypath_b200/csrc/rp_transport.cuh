@@ -29,17 +29,19 @@ RP_DEV u32 set_status(u32 f, u32 s) { return (f & ~(7u << F_STATUS_SHIFT)) | (s 
 // Structure-of-arrays path pool: one slot per lane of the wave.
 struct PathPool {
     uint4 *ident;      // pixel, sample_low, sample_high, flags
-    uint4 *cursor;     // sobol index lo, hi, vertex count, lane
+    uint2 *index;      // Sobol index
     float4 *lambda, *lambda_pdf, *beta, *radiance;
-    float4 *dens_f, *prev_f; // hero density fractions (arrival / previous)
-    int4 *dens_e, *prev_e;   // and exponents
+    // Arrays in pairs hold the values at the start of the event in [in], in the parity of the
+    // event's queue, and take those after it in [in ^ 1]: the event before's density and vertex
+    // and this event's ray stay where they are, for its MIS weight and its light sample.
+    float4 *dens_f[2]; // hero density fractions
+    int4 *dens_e[2];   // and exponents
     float4 *eta_scale;
-    float4 *ray_o, *ray_d;
-    float4 *latest_p;      // latest vertex position, alpha_x
+    float4 *ray_o, *ray_d[2];
+    float4 *latest_p[2];   // latest vertex position, alpha_x
     float4 *latest_n;      // latest shading normal, alpha_y
     float4 *latest_param;  // per-wavelength reflectance or eta
-    float4 *latest_k;      // per-wavelength conductor k
-    float4 *preceding;     // position of the vertex before latest
+    float4 *latest_k;      // per-wavelength conductor k (conductors only)
     float4 *hit;           // t, b1, b2, primitive bits
     // queues
     u32 *queue[2];
@@ -54,11 +56,9 @@ struct PathPool {
     // statistics (optional)
     unsigned long long *stats; // closest [0] nodes, [1] triangles, [2] rays; shadow [3] rays, [4] nodes, [5] triangles
     // light-sample requests, one per path (written by the shade kernel, read by k_nee): the
-    // vertex (position + vertex count, shading normal + BSDF bits, geometric normal + alpha_x,
-    // error + alpha_y), the outgoing direction, the previous vertex, the throughput and hero
-    // density before this event's continuation, and the BSDF's per-wavelength parameters
-    float4 *nee_p, *nee_n, *nee_g, *nee_e, *nee_wo, *nee_prev, *nee_beta, *nee_df, *nee_param, *nee_k;
-    int4 *nee_de;
+    // geometric normal, the position's error and the throughput before this event's
+    // continuation; the rest is the latest vertex and the values of the event's start
+    float4 *nee_g, *nee_e, *nee_beta;
     u32 *nee_queue; // three family queues of bin_capacity path ids
     // per-lane walk counts of counting runs (pool slot = request lane), or nullptr: closest-hit
     // walks (written by the closest-hit kernel) and any-hit walks (by the shadow kernel, which
@@ -679,52 +679,37 @@ RP_DEV void store_density(const Density &d, float4 &f, int4 &e) {
     e = make_int4(d.lane[0].exponent, d.lane[1].exponent, d.lane[2].exponent, d.lane[3].exponent);
 }
 
-// The light-sample request of a path's event (PathPool::nee_*).
-RP_DEV void write_nee_request(const PathPool &pool, u32 path, u32 cnt, const SurfacePoint &cp, const HeroBsdf &b,
-                              V3 wo, V3 previous, V4 beta, const Density &density) {
-    const u32 bits = (b.kind & 3u) | ((b.active_mask & 15u) << 2) | (b.g.smooth ? 64u : 0u);
-    pool.nee_p[path] = make_float4(cp.position.x, cp.position.y, cp.position.z, __uint_as_float(cnt));
-    pool.nee_n[path] = make_float4(cp.shading_normal.x, cp.shading_normal.y, cp.shading_normal.z, __uint_as_float(bits));
-    pool.nee_g[path] = make_float4(cp.geometric_normal.x, cp.geometric_normal.y, cp.geometric_normal.z, b.g.alpha_x);
-    pool.nee_e[path] = make_float4(cp.error.x, cp.error.y, cp.error.z, b.g.alpha_y);
-    pool.nee_wo[path] = make_float4(wo.x, wo.y, wo.z, 0);
-    pool.nee_prev[path] = make_float4(previous.x, previous.y, previous.z, 0);
-    pool.nee_beta[path] = to_float4(beta);
-    float4 f;
-    int4 e;
-    store_density(density, f, e);
-    pool.nee_df[path] = f;
-    pool.nee_de[path] = e;
-    pool.nee_param[path] = make_float4(b.param[0], b.param[1], b.param[2], b.param[3]);
-    pool.nee_k[path] = make_float4(b.k[0], b.k[1], b.k[2], b.k[3]);
-}
-RP_DEV void read_nee_request(const PathPool &pool, u32 path, u32 &cnt, SurfacePoint &cp, HeroBsdf &b, V3 &wo,
+// The light-sample request of a path's event (PathPool::nee_*), a vertex of family F.
+template <int F>
+RP_DEV void read_nee_request(const PathPool &pool, int in, u32 path, u32 flags, SurfacePoint &cp, HeroBsdf &b, V3 &wo,
                              V3 &previous, V4 &beta, Density &density) {
-    const float4 pp = pool.nee_p[path], n = pool.nee_n[path], g = pool.nee_g[path], e = pool.nee_e[path];
-    const float4 w = pool.nee_wo[path], v = pool.nee_prev[path], pa = pool.nee_param[path], k = pool.nee_k[path];
-    cnt = __float_as_uint(pp.w);
-    const u32 bits = __float_as_uint(n.w);
+    const float4 pp = pool.latest_p[in ^ 1][path], n = pool.latest_n[path], g = pool.nee_g[path], e = pool.nee_e[path];
+    const float4 w = pool.ray_d[in][path], v = pool.latest_p[in][path], pa = pool.latest_param[path];
     cp.position = v3(pp.x, pp.y, pp.z);
     cp.shading_normal = v3(n.x, n.y, n.z);
     cp.geometric_normal = v3(g.x, g.y, g.z);
     cp.error = v3(e.x, e.y, e.z);
     cp.inverse_area_pdf = 0;
     cp.world_extent = 0;
-    b.kind = bits & 3u;
-    b.active_mask = (bits >> 2) & 15u;
-    b.g = {g.w, e.w, (bits & 64u) != 0};
+    b.kind = F;
+    b.active_mask = (flags >> F_LMASK_SHIFT) & 15u;
+    b.g = {pp.w, n.w, (flags & F_LSMOOTH) != 0};
     b.param[0] = pa.x;
     b.param[1] = pa.y;
     b.param[2] = pa.z;
     b.param[3] = pa.w;
-    b.k[0] = k.x;
-    b.k[1] = k.y;
-    b.k[2] = k.z;
-    b.k[3] = k.w;
-    wo = v3(w.x, w.y, w.z);
+    b.k[0] = b.k[1] = b.k[2] = b.k[3] = 0;
+    if constexpr (F == 1) {
+        const float4 k = pool.latest_k[path];
+        b.k[0] = k.x;
+        b.k[1] = k.y;
+        b.k[2] = k.z;
+        b.k[3] = k.w;
+    }
+    wo = -v3(w.x, w.y, w.z);
     previous = v3(v.x, v.y, v.z);
     beta = from_float4(pool.nee_beta[path]);
-    density = load_density(pool.nee_df[path], pool.nee_de[path]);
+    density = load_density(pool.dens_f[in][path], pool.dens_e[in][path]);
 }
 
 // shaders/packet_transport.h:77-83
