@@ -886,8 +886,8 @@ int grid_for(int sm_count, u32 work, int block, int per_sm) {
     return int(std::max<u32>(1, std::min<u32>(needed, u32(sm_count * per_sm))));
 }
 
-// The structure-of-arrays carve of a path pool of `lanes` slots over `base` (nullptr: only
-// the size is computed): the 16-byte arrays, the queues and family bins, the counters, and,
+// The carve of a path pool of `lanes` slots over `base` (nullptr: only
+// the size is computed): the records, the queues and family bins, the counters, and,
 // when `full`, the arrays only some runs read (shadow targets and resolved materials of
 // scenes with pass-through or mix surfaces, per-lane walk counts of counting runs).  Every
 // slice starts on a 256-byte boundary.  The scene pool and the allocation-free scratch both
@@ -896,11 +896,12 @@ int grid_for(int sm_count, u32 work, int block, int per_sm) {
 // counting and without the adjoint may run on it.
 constexpr size_t pool_bytes(u32 lanes, bool full) {
     const size_t v16 = (size_t(lanes) * 16 + 255) & ~size_t(255), v4 = (size_t(lanes) * 4 + 255) & ~size_t(255);
-    const size_t v8 = (size_t(lanes) * 8 + 255) & ~size_t(255);
-    return 25 * v16 + v8 + 9 * v4 + 256 + (full ? v16 + 3 * v4 : 0);
+    const size_t v32 = (size_t(lanes) * 32 + 255) & ~size_t(255), v64 = (size_t(lanes) * 64 + 255) & ~size_t(255);
+    return 3 * v64 + 7 * v32 + 5 * v16 + 9 * v4 + 256 + (full ? v16 + 3 * v4 : 0);
 }
 size_t carve_pool(unsigned char *base, u32 lanes, bool full, PathPool *out) {
     const size_t v16 = (size_t(lanes) * 16 + 255) & ~size_t(255), v4 = (size_t(lanes) * 4 + 255) & ~size_t(255);
+    const size_t v32 = (size_t(lanes) * 32 + 255) & ~size_t(255), v64 = (size_t(lanes) * 64 + 255) & ~size_t(255);
     size_t off = 0;
     auto take = [&](size_t n) {
         unsigned char *p = base ? base + off : nullptr;
@@ -908,15 +909,16 @@ size_t carve_pool(unsigned char *base, u32 lanes, bool full, PathPool *out) {
         return p;
     };
     PathPool q{};
-    q.ident = reinterpret_cast<uint4 *>(take(v16));
-    q.index = reinterpret_cast<uint2 *>(take((size_t(lanes) * 8 + 255) & ~size_t(255)));
-    float4 **f4[] = {&q.lambda, &q.lambda_pdf, &q.beta, &q.radiance, &q.dens_f[0], &q.dens_f[1], &q.eta_scale, &q.ray_o,
-                     &q.ray_d[0], &q.ray_d[1], &q.latest_p[0], &q.latest_p[1], &q.latest_n, &q.latest_param, &q.latest_k,
-                     &q.hit, &q.sh_o, &q.sh_d, &q.sh_c, &q.nee_g, &q.nee_e, &q.nee_beta};
+    q.ident_index = reinterpret_cast<uint4 *>(take(v32));
+    float4 **records[] = {&q.spectrum, &q.throughput, &q.densities[0], &q.densities[1], &q.rays[0], &q.rays[1]};
+    for (auto p : records)
+        *p = reinterpret_cast<float4 *>(take(v32));
+    float4 **vertices[] = {&q.vertices[0], &q.vertices[1], &q.requests};
+    for (auto p : vertices)
+        *p = reinterpret_cast<float4 *>(take(v64));
+    float4 **f4[] = {&q.radiances, &q.hits, &q.sh_o, &q.sh_d, &q.sh_c};
     for (auto p : f4)
         *p = reinterpret_cast<float4 *>(take(v16));
-    q.dens_e[0] = reinterpret_cast<int4 *>(take(v16));
-    q.dens_e[1] = reinterpret_cast<int4 *>(take(v16));
     q.queue[0] = reinterpret_cast<u32 *>(take(v4));
     q.queue[1] = reinterpret_cast<u32 *>(take(v4));
     q.bins = reinterpret_cast<u32 *>(take(4 * v4));
@@ -937,7 +939,7 @@ size_t carve_pool(unsigned char *base, u32 lanes, bool full, PathPool *out) {
 }
 // Every PathPool member is a pointer carved above, set elsewhere (stats, the adjoint's), or
 // a count: a new member changes this size and so comes past this check.
-static_assert(sizeof(PathPool) == 43 * sizeof(void *) + 16, "PathPool changed: review carve_pool");
+static_assert(sizeof(PathPool) == 32 * sizeof(void *) + 16, "PathPool changed: review carve_pool");
 
 } // namespace
 
@@ -1448,16 +1450,13 @@ void launch_families(rp_scene *s, const WaveParams &p, const PathPool &pool, int
         }
 }
 u32 family_kernels(const rp_scene *s) { return 2 * u32(__builtin_popcount(s->family_mask)) + 1; }
-// The plain shade kernels for scenes without images (the adjoint keeps the full ones).
+// The plain shade kernels for scenes without images.
 template <int Block, bool Adjoint>
 void launch_shade(rp_scene *s, const WaveParams &p, const PathPool &pool, int in, u32 event, unsigned grid, size_t smem) {
-    if constexpr (!Adjoint) {
-        if (!s->ds.img.textured && s->ds.img.env_image == kNone) {
-            launch_families<Block, false, false>(s, p, pool, in, event, grid, smem);
-            return;
-        }
-    }
-    launch_families<Block, Adjoint, true>(s, p, pool, in, event, grid, smem);
+    if (!s->ds.img.textured && s->ds.img.env_image == kNone)
+        launch_families<Block, Adjoint, false>(s, p, pool, in, event, grid, smem);
+    else
+        launch_families<Block, Adjoint, true>(s, p, pool, in, event, grid, smem);
 }
 
 // Sobol sampler with Owen randomisation: attaches the tables of the draw blocks of the scene's

@@ -32,19 +32,18 @@ RP_DEV void raygen_lane(const DeviceScene &s, const RasterCam &cam, const WavePa
         u32 flags = 15u | F_ROULETTE | (kCamera << F_LTYPE_SHIFT);
         if (!finite3(o) || !finite3(d))
             flags = set_status(flags, 2) | F_COMPLETE;
-        pool.ident[slot] = make_uint4(b.pixel, b.sample_low, b.sample_high, flags);
-        pool.index[slot] = make_uint2(u32(b.index), u32(b.index >> 32));
-        pool.lambda[slot] = to_float4(lambda);
-        pool.lambda_pdf[slot] = to_float4(pdf);
-        pool.beta[slot] = make_float4(1, 1, 1, 1);
-        pool.radiance[slot] = make_float4(0, 0, 0, 0);
-        pool.dens_f[0][slot] = make_float4(.5f, .5f, .5f, .5f); // read before [1] is
-        pool.dens_e[0][slot] = make_int4(1, 1, 1, 1);
-        pool.eta_scale[slot] = make_float4(1, 1, 1, 1);
-        pool.ray_o[slot] = make_float4(o.x, o.y, o.z, 0);
-        pool.ray_d[0][slot] = make_float4(d.x, d.y, d.z, 0);
-        pool.latest_p[0][slot] = make_float4(o.x, o.y, o.z, 0);
-        pool.latest_n[slot] = make_float4(0, 0, 0, 0);
+        pool.ident(slot) = make_uint4(b.pixel, b.sample_low, b.sample_high, flags);
+        pool.index(slot) = make_uint4(u32(b.index), u32(b.index >> 32), 0, 0);
+        pool.lambda(slot) = to_float4(lambda);
+        pool.lambda_pdf(slot) = to_float4(pdf);
+        pool.beta(slot) = make_float4(1, 1, 1, 1);
+        pool.radiance(slot) = make_float4(0, 0, 0, 0);
+        pool.dens_f(0, slot) = make_float4(.5f, .5f, .5f, .5f); // read before [1] is
+        pool.dens_e(0, slot) = make_int4(1, 1, 1, 1);
+        pool.eta_scale(slot) = make_float4(1, 1, 1, 1);
+        pool.ray_o(0, slot) = make_float4(o.x, o.y, o.z, 0);
+        pool.ray_d(0, slot) = make_float4(d.x, d.y, d.z, 0);
+        pool.vertex(0, slot)[0] = make_float4(o.x, o.y, o.z, 0);
         pool.queue[0][slot] = slot;
         if (pool.lane_closest) {
             pool.lane_closest[slot] = 0;
@@ -74,7 +73,7 @@ constexpr u32 kHitInvalid = 0xfffffffeu, kHitExhausted = 0xfffffffdu, kHitArithm
 // written to pool.material).  Returns the family to bin (3 for a failure or a miss) and sets
 // `prim` to the primitive or failure code to record.
 template <bool Count, int Stack>
-__device__ __noinline__ u32 resolve_hit(const DeviceScene &s, const PathPool &pool, u32 path, V3 ro, V3 rd, Hit &h,
+__device__ __noinline__ u32 resolve_hit(const DeviceScene &s, const PathPool &pool, int in, u32 path, V3 ro, V3 rd, Hit &h,
                                         u32 &prim, uint2 *stack, int stride, u32 boundary_limit, u32 &nodes, u32 &tris,
                                         u32 &rays) {
     u32 crossings = 0;
@@ -133,7 +132,7 @@ __device__ __noinline__ u32 resolve_hit(const DeviceScene &s, const PathPool &po
         break;
     }
     if (moved)
-        pool.ray_o[path] = make_float4(ro.x, ro.y, ro.z, 0);
+        pool.ray_o(in, path) = make_float4(ro.x, ro.y, ro.z, 0);
     return prim >= kHitArithmetic || prim == kNone ? 3u : family;
 }
 
@@ -161,8 +160,8 @@ __global__ void __launch_bounds__(Block, Stack <= kShortStack ? 1024 / Block : 1
         u32 family = 4, path = 0;
         if (i < count) {
             path = queue[i];
-            if (!(pool.ident[path].w & F_COMPLETE)) {
-                const float4 o = pool.ray_o[path], d = pool.ray_d[in][path];
+            if (!(pool.ident(path).w & F_COMPLETE)) {
+                const float4 o = pool.ray_o(in, path), d = pool.ray_d(in, path);
                 const u32 walks_before = rays;
                 Hit h;
                 const bool ok = walk_closest<Count, Stack, Resolve>(s, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z),
@@ -172,9 +171,9 @@ __global__ void __launch_bounds__(Block, Stack <= kShortStack ? 1024 / Block : 1
                 u32 prim = ok ? h.prim : kHitInvalid;
                 family = (!ok || h.prim == kNone) ? 3u : u32(__ldg(s.tri_family + h.prim));
                 if (Resolve && family == kResolveFamily)
-                    family = resolve_hit<Count, Stack>(s, pool, path, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), h, prim,
+                    family = resolve_hit<Count, Stack>(s, pool, in, path, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), h, prim,
                                                        stack + threadIdx.x, Block, boundary_limit, nodes, tris, rays);
-                pool.hit[path] = make_float4(h.t, h.b1, h.b2, __uint_as_float(prim));
+                pool.hit(path) = make_float4(h.t, h.b1, h.b2, __uint_as_float(prim));
                 if (Count && pool.lane_closest)
                     pool.lane_closest[path] += rays - walks_before;
             }
@@ -196,9 +195,10 @@ __global__ void __launch_bounds__(Block, Stack <= kShortStack ? 1024 / Block : 1
 }
 
 // The warps of a block meet between two phases of a long straight run of code, so that a line of
-// instructions fetched for one serves them all: the shade kernels run five thousand
-// instructions an event once each, and their warps, left to drift apart, spend a third to half
-// of their cycles waiting for instructions.
+// instructions fetched for one serves them all: the shade kernels run some four thousand
+// instructions an event once each, and their warps, left to drift apart, spent up to 6.9 of 17
+// cycles an instruction waiting for instructions (0.9 so; the textured box 24.8 -> 13.4 ms of
+// shading, the Cornell box 14.0 -> 12.1).  Blocks of 256 serve better than of 128 or 512.
 template <bool Sync> RP_DEV void phase() {
     if (Sync)
         __syncthreads();
@@ -212,24 +212,24 @@ template <int F, bool Adjoint, bool Img, bool Sync>
 RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool &pool, int in, u32 event_index,
                        bool active, u32 path, float *sgrad, bool &keep, bool &nee) {
     const u32 capacity = s.max_depth + 2;
-    uint4 ident = pool.ident[path];
+    uint4 ident = pool.ident(path);
     u32 flags = ident.w;
     active = active && !(flags & F_COMPLETE);
     {
-        const uint2 index2 = pool.index[path];
+        const uint4 index2 = pool.index(path);
         const u64 index = (u64(index2.y) << 32) | index2.x;
         u32 cnt = event_index + 1; // vertices so far, the camera's included
-        const V4 lambda = from_float4(pool.lambda[path]);
-        V4 beta = from_float4(pool.beta[path]);
-        Density density = load_density(pool.dens_f[in][path], pool.dens_e[in][path]);
+        const V4 lambda = from_float4(pool.lambda(path));
+        V4 beta = from_float4(pool.beta(path));
+        Density density = load_density(pool.dens_f(in, path), pool.dens_e(in, path));
         V4 eta_scale = v4(1);
         if (event_index)
-            eta_scale = from_float4(pool.eta_scale[path]);
+            eta_scale = from_float4(pool.eta_scale(path));
         bool roulette = (flags & F_ROULETTE) != 0;
         u32 active_mask = flags & F_MASK;
-        const float4 ro4 = pool.ray_o[path], rd4 = pool.ray_d[in][path];
+        const float4 ro4 = pool.ray_o(in, path), rd4 = pool.ray_d(in, path);
         V3 ro = v3(ro4.x, ro4.y, ro4.z), rd = v3(rd4.x, rd4.y, rd4.z);
-        const float4 hit = pool.hit[path];
+        const float4 hit = pool.hit(path);
         u32 status = get_status(flags);
         const Density direct_density = density;
         V4 direct_beta = beta;
@@ -431,7 +431,7 @@ RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool
                 const DInstance &instance = s.instances[cinst];
                 V3 delta = v3(0, 0, 0);
                 if (instance.emission != kNone) {
-                    const float4 lp4 = pool.latest_p[in][path];
+                    const float4 lp4 = pool.vertex(in, path)[0];
                     delta = v3(lp4.x, lp4.y, lp4.z) - cp.position;
                 }
                 if (!zero3(delta)) {
@@ -453,15 +453,16 @@ RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool
                 if (cnt <= 2 || latest.delta || !nonzero4(value)) {
                     endpoint = value;
                 } else {
-                    const float4 lp4 = pool.latest_p[in][path], ln4 = pool.latest_n[path];
+                    const float4 *vertex = pool.vertex(in, path);
+                    const float4 lp4 = vertex[0], ln4 = vertex[1];
                     latest.position = v3(lp4.x, lp4.y, lp4.z);
                     latest.shading_normal = v3(ln4.x, ln4.y, ln4.z);
                     latest.alpha_x = lp4.w;
                     latest.alpha_y = ln4.w;
-                    latest.param = from_float4(pool.latest_param[path]);
-                    latest.k = latest.kind == 1 ? from_float4(pool.latest_k[path]) : v4(0);
-                    const float4 pre = pool.latest_p[in ^ 1][path]; // the vertex before it
-                    const Density previous_density = load_density(pool.dens_f[in ^ 1][path], pool.dens_e[in ^ 1][path]);
+                    latest.param = from_float4(vertex[2]);
+                    latest.k = latest.kind == 1 ? from_float4(vertex[3]) : v4(0);
+                    const float4 pre = pool.vertex(in ^ 1, path)[0]; // the vertex before it
+                    const Density previous_density = load_density(pool.dens_f(in ^ 1, path), pool.dens_e(in ^ 1, path));
                     bool ok;
                     const V4 bsdf_pdf = represented_pdf<-1>(latest_bsdf(latest), latest.shading_normal, latest.position,
                                                         v3(pre.x, pre.y, pre.z), ctype == kEnvironment,
@@ -488,8 +489,8 @@ RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool
             // radiance is finite and nonnegative while its path lives; a zero endpoint leaves it
             bool radiance_ok = true;
             if (endpoint.v[0] != 0 || endpoint.v[1] != 0 || endpoint.v[2] != 0 || endpoint.v[3] != 0) {
-                const V4 radiance = add4(from_float4(pool.radiance[path]), endpoint);
-                pool.radiance[path] = to_float4(radiance);
+                const V4 radiance = add4(from_float4(pool.radiance(path)), endpoint);
+                pool.radiance(path) = to_float4(radiance);
                 radiance_ok = finite_nonnegative4(radiance);
             }
             if (Adjoint) {
@@ -516,9 +517,10 @@ RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool
                 nee = false;
             }
             if (nee) {
-                pool.nee_g[path] = make_float4(cp.geometric_normal.x, cp.geometric_normal.y, cp.geometric_normal.z, 0);
-                pool.nee_e[path] = make_float4(cp.error.x, cp.error.y, cp.error.z, 0);
-                pool.nee_beta[path] = to_float4(direct_beta);
+                float4 *request = pool.request(path);
+                request[0] = make_float4(cp.geometric_normal.x, cp.geometric_normal.y, cp.geometric_normal.z, 0);
+                request[1] = make_float4(cp.error.x, cp.error.y, cp.error.z, 0);
+                request[2] = to_float4(direct_beta);
             }
         }
         phase<Sync>();
@@ -531,14 +533,12 @@ RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool
             // preceding = latest; latest = current (shaders/packet_pt_event_body.inc:453-460)
             flags = (flags & ~(3u << F_PTYPE_SHIFT)) | (latest.type << F_PTYPE_SHIFT);
             if (!complete || nee) {
-                pool.latest_p[in ^ 1][path] =
-                    make_float4(cp.position.x, cp.position.y, cp.position.z, cbsdf.g.alpha_x);
-                pool.latest_n[path] =
-                    make_float4(cp.shading_normal.x, cp.shading_normal.y, cp.shading_normal.z, cbsdf.g.alpha_y);
-                pool.latest_param[path] =
-                    make_float4(cbsdf.param[0], cbsdf.param[1], cbsdf.param[2], cbsdf.param[3]);
+                float4 *vertex = pool.vertex(in ^ 1, path);
+                vertex[0] = make_float4(cp.position.x, cp.position.y, cp.position.z, cbsdf.g.alpha_x);
+                vertex[1] = make_float4(cp.shading_normal.x, cp.shading_normal.y, cp.shading_normal.z, cbsdf.g.alpha_y);
+                vertex[2] = make_float4(cbsdf.param[0], cbsdf.param[1], cbsdf.param[2], cbsdf.param[3]);
                 if (F == 1)
-                    pool.latest_k[path] = make_float4(cbsdf.k[0], cbsdf.k[1], cbsdf.k[2], cbsdf.k[3]);
+                    vertex[3] = make_float4(cbsdf.k[0], cbsdf.k[1], cbsdf.k[2], cbsdf.k[3]);
             }
             flags &= ~((3u << F_LTYPE_SHIFT) | F_LDELTA | (3u << F_LKIND_SHIFT) | (15u << F_LMASK_SHIFT) | F_LSMOOTH);
             flags |= (ctype << F_LTYPE_SHIFT) | (cdelta ? F_LDELTA : 0u) | ((cbsdf.kind & 3u) << F_LKIND_SHIFT) |
@@ -547,18 +547,18 @@ RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool
         flags = (flags & ~(F_MASK | F_ROULETTE)) | active_mask | (roulette ? F_ROULETTE : 0u);
         flags = set_status(flags, status) | (complete ? F_COMPLETE : 0u);
         ident.w = flags;
-        pool.ident[path] = ident;
+        pool.ident(path) = ident;
         if (!complete) {
-            pool.beta[path] = to_float4(beta);
+            pool.beta(path) = to_float4(beta);
             float4 f;
             int4 e;
             store_density(density, f, e);
-            pool.dens_f[in ^ 1][path] = f;
-            pool.dens_e[in ^ 1][path] = e;
+            pool.dens_f(in ^ 1, path) = f;
+            pool.dens_e(in ^ 1, path) = e;
             if (F == 2)
-                pool.eta_scale[path] = to_float4(eta_scale); // only transmission changes it
-            pool.ray_o[path] = make_float4(ro.x, ro.y, ro.z, 0);
-            pool.ray_d[in ^ 1][path] = make_float4(rd.x, rd.y, rd.z, 0);
+                pool.eta_scale(path) = to_float4(eta_scale); // only transmission changes it
+            pool.ray_o(in ^ 1, path) = make_float4(ro.x, ro.y, ro.z, 0);
+            pool.ray_d(in ^ 1, path) = make_float4(rd.x, rd.y, rd.z, 0);
         }
         keep = !complete;
     }
@@ -618,10 +618,10 @@ __global__ void __launch_bounds__(Block, 512 / Block) k_shade(const __grid_const
 template <int F, bool Img, bool Sync>
 RP_DEV void nee_path(const DeviceScene &s, const WaveParams &p, const PathPool &pool, int in, u32 event_index, bool active,
                      u32 path, bool &shadow, float4 &sh_o, float4 &sh_d, float4 &sh_c, float4 &sh_t) {
-    uint4 ident = pool.ident[path];
-    const uint2 index2 = pool.index[path];
+    uint4 ident = pool.ident(path);
+    const uint4 index2 = pool.index(path);
     const u64 index = (u64(index2.y) << 32) | index2.x;
-    const V4 lambda = from_float4(pool.lambda[path]);
+    const V4 lambda = from_float4(pool.lambda(path));
     SurfacePoint cp;
     HeroBsdf cbsdf;
     V3 cwo, previous;
@@ -763,7 +763,7 @@ RP_DEV void nee_path(const DeviceScene &s, const WaveParams &p, const PathPool &
     }
     if (status != 0) {
         ident.w = set_status(ident.w, status) | F_COMPLETE;
-        pool.ident[path] = ident;
+        pool.ident(path) = ident;
         shadow = false;
     }
 }
@@ -840,30 +840,30 @@ RP_DEV void shadow_result(const DeviceScene &s, const PathPool &pool, float *sgr
                           u32 failure, bool occluded) {
     if (!failure && occluded)
         return;
-    uint4 ident = pool.ident[path];
+    uint4 ident = pool.ident(path);
     if (failure) {
         ident.w = set_status(ident.w, failure) | F_COMPLETE;
-        pool.ident[path] = ident;
+        pool.ident(path) = ident;
         return;
     }
     const float4 c = contribution;
     if (isnan(c.x)) {
         ident.w = set_status(ident.w, 2) | F_COMPLETE;
-        pool.ident[path] = ident;
+        pool.ident(path) = ident;
         return;
     }
-    float4 r = pool.radiance[path];
+    float4 r = pool.radiance(path);
     r.x += c.x;
     r.y += c.y;
     r.z += c.z;
     r.w += c.w;
-    pool.radiance[path] = r;
+    pool.radiance(path) = r;
     if (!finite_nonnegative4(from_float4(r))) {
         ident.w = set_status(ident.w, 2) | F_COMPLETE;
-        pool.ident[path] = ident;
+        pool.ident(path) = ident;
     } else if (Adjoint) {
         // replay: the light sample's gradient, over the history including its vertex
-        adjoint_accumulate(s, pool, sgrad, pool.hist[path], from_float4(pool.lambda[path]), from_float4(c),
+        adjoint_accumulate(s, pool, sgrad, pool.hist[path], from_float4(pool.lambda(path)), from_float4(c),
                            pool.adj_w[path]);
     }
 }
@@ -922,16 +922,16 @@ __global__ void __launch_bounds__(kPathBlock, 6) k_paths(const __grid_constant__
         u32 unused = 0;
         for (u32 e = 0; e <= s.max_depth; ++e) {
             const int in = int(e & 1u);
-            if (pool.ident[path].w & F_COMPLETE)
+            if (pool.ident(path).w & F_COMPLETE)
                 break;
-            const float4 o = pool.ray_o[path], d = pool.ray_d[in][path];
+            const float4 o = pool.ray_o(in, path), d = pool.ray_d(in, path);
             Hit h;
             const bool hit_ok = walk_closest<false, Stack, false>(s, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z),
                                                                   __int_as_float(0x7f800000), h, stack + threadIdx.x,
                                                                   kPathBlock, unused, unused);
             const u32 prim = hit_ok ? h.prim : kHitInvalid;
             const u32 family = !hit_ok || h.prim == kNone ? 3u : u32(__ldg(s.tri_family + h.prim));
-            pool.hit[path] = make_float4(h.t, h.b1, h.b2, __uint_as_float(prim));
+            pool.hit(path) = make_float4(h.t, h.b1, h.b2, __uint_as_float(prim));
             bool keep = false, nee = false, shadow = false;
             float4 so, sd, sc, st;
             if (family == 0) {
@@ -972,8 +972,8 @@ struct PacketResult {
 };
 __global__ void k_results(PathPool pool, u32 lanes, float filter_weight, PacketResult *out) {
     for (u32 lane = blockIdx.x * blockDim.x + threadIdx.x; lane < lanes; lane += gridDim.x * blockDim.x) {
-        const uint4 id = pool.ident[lane];
-        const float4 l = pool.lambda[lane], pdf = pool.lambda_pdf[lane], r = pool.radiance[lane];
+        const uint4 id = pool.ident(lane);
+        const float4 l = pool.lambda(lane), pdf = pool.lambda_pdf(lane), r = pool.radiance(lane);
         PacketResult res;
         res.status = (id.w & F_COMPLETE) ? get_status(id.w) : 2u;
         res.pixel = id.x;
@@ -1043,11 +1043,11 @@ RP_DEV void film_add_compatibility(const double (&xyz)[3], double weight, const 
 }
 RP_DEV bool film_add_lane(const PathPool &pool, u32 lane, const double *cie, double weight, const FilmClamp &clamp,
                           FilmPixel &f) {
-    const uint4 id = pool.ident[lane];
+    const uint4 id = pool.ident(lane);
     const u32 status = (id.w & F_COMPLETE) ? get_status(id.w) : 2u;
     if (status != 0)
         return false;
-    const float4 l4 = pool.lambda[lane], p4 = pool.lambda_pdf[lane], r4 = pool.radiance[lane];
+    const float4 l4 = pool.lambda(lane), p4 = pool.lambda_pdf(lane), r4 = pool.radiance(lane);
     const float lam[4] = {l4.x, l4.y, l4.z, l4.w}, pdf[4] = {p4.x, p4.y, p4.z, p4.w}, rad[4] = {r4.x, r4.y, r4.z, r4.w};
     double xyz[3] = {0, 0, 0};
 #pragma unroll
@@ -1079,7 +1079,7 @@ RP_DEV bool film_add_lane(const PathPool &pool, u32 lane, const double *cie, dou
 // cleared with the wave's counters, so callers accumulate it per wave.
 __global__ void k_count_failures(PathPool pool, u32 lanes) {
     for (u32 lane = blockIdx.x * blockDim.x + threadIdx.x; lane < lanes; lane += gridDim.x * blockDim.x) {
-        const u32 w = pool.ident[lane].w;
+        const u32 w = pool.ident(lane).w;
         if (!(w & F_COMPLETE) || get_status(w) != 0)
             atomicAdd(pool.counters + 3, 1u);
     }
@@ -1130,10 +1130,10 @@ __global__ void k_film(PathPool pool, u32 pixel_count, u32 samples, const double
 __global__ void k_frame_packet(PathPool pool, u32 pixel_count, u32 pixel_begin, u32 sample_low, u32 sample_high,
                                const double *cie, float *xyz, u32 *failures) {
     for (u32 px = blockIdx.x * blockDim.x + threadIdx.x; px < pixel_count; px += gridDim.x * blockDim.x) {
-        const uint4 id = pool.ident[px];
+        const uint4 id = pool.ident(px);
         bool valid = (id.w & F_COMPLETE) && get_status(id.w) == 0 && id.x == pixel_begin + px && id.y == sample_low &&
                      id.z == sample_high;
-        const float4 l4 = pool.lambda[px], p4 = pool.lambda_pdf[px], r4 = pool.radiance[px];
+        const float4 l4 = pool.lambda(px), p4 = pool.lambda_pdf(px), r4 = pool.radiance(px);
         const float lam[4] = {l4.x, l4.y, l4.z, l4.w}, pdf[4] = {p4.x, p4.y, p4.z, p4.w}, rad[4] = {r4.x, r4.y, r4.z, r4.w};
         bool secondary = false, terminated = false;
         float v[3] = {0, 0, 0};

@@ -26,23 +26,42 @@ enum : u32 {
 RP_DEV u32 get_status(u32 f) { return (f >> F_STATUS_SHIFT) & 7u; }
 RP_DEV u32 set_status(u32 f, u32 s) { return (f & ~(7u << F_STATUS_SHIFT)) | (s << F_STATUS_SHIFT); }
 
-// Structure-of-arrays path pool: one slot per lane of the wave.
+// Path pool: one slot per lane of the wave.  What a kernel reads or writes together lies
+// together in records of 32 or 64 bytes, whole 32-byte sectors: after the first event the bins
+// list their paths out of order, and sixteen bytes of one array at a time would fetch two
+// sectors for the bytes of one.
 struct PathPool {
-    uint4 *ident;      // pixel, sample_low, sample_high, flags
-    uint2 *index;      // Sobol index
-    float4 *lambda, *lambda_pdf, *beta, *radiance;
-    // Arrays in pairs hold the values at the start of the event in [in], in the parity of the
+    uint4 *ident_index; // 2: pixel, sample_low, sample_high, flags; Sobol index lo, hi
+    float4 *spectrum;   // 2: lambda, lambda pdf
+    float4 *throughput; // 2: beta, eta scale
+    float4 *radiances;
+    float4 *hits;       // t, b1, b2, primitive bits
+    // Records in pairs hold the values at the start of the event in [in], in the parity of the
     // event's queue, and take those after it in [in ^ 1]: the event before's density and vertex
     // and this event's ray stay where they are, for its MIS weight and its light sample.
-    float4 *dens_f[2]; // hero density fractions
-    int4 *dens_e[2];   // and exponents
-    float4 *eta_scale;
-    float4 *ray_o, *ray_d[2];
-    float4 *latest_p[2];   // latest vertex position, alpha_x
-    float4 *latest_n;      // latest shading normal, alpha_y
-    float4 *latest_param;  // per-wavelength reflectance or eta
-    float4 *latest_k;      // per-wavelength conductor k (conductors only)
-    float4 *hit;           // t, b1, b2, primitive bits
+    float4 *densities[2]; // 2: hero density fractions, exponents (int4 bits)
+    float4 *rays[2];      // 2: origin, direction
+    float4 *vertices[2];  // 4: the latest vertex: position + alpha_x, shading normal + alpha_y,
+                          // reflectance or eta per wavelength, conductor k (conductors only)
+    // light-sample requests, written by the shade kernel and read by k_nee
+    float4 *requests;     // 4: geometric normal, position error, throughput before the continuation
+
+    RP_DEV uint4 &ident(u32 path) const { return ident_index[2 * size_t(path)]; }
+    RP_DEV uint4 &index(u32 path) const { return ident_index[2 * size_t(path) + 1]; }
+    RP_DEV float4 &lambda(u32 path) const { return spectrum[2 * size_t(path)]; }
+    RP_DEV float4 &lambda_pdf(u32 path) const { return spectrum[2 * size_t(path) + 1]; }
+    RP_DEV float4 &beta(u32 path) const { return throughput[2 * size_t(path)]; }
+    RP_DEV float4 &eta_scale(u32 path) const { return throughput[2 * size_t(path) + 1]; }
+    RP_DEV float4 &radiance(u32 path) const { return radiances[path]; }
+    RP_DEV float4 &hit(u32 path) const { return hits[path]; }
+    RP_DEV float4 &dens_f(int in, u32 path) const { return densities[in][2 * size_t(path)]; }
+    RP_DEV int4 &dens_e(int in, u32 path) const {
+        return reinterpret_cast<int4 *>(densities[in])[2 * size_t(path) + 1];
+    }
+    RP_DEV float4 &ray_o(int in, u32 path) const { return rays[in][2 * size_t(path)]; }
+    RP_DEV float4 &ray_d(int in, u32 path) const { return rays[in][2 * size_t(path) + 1]; }
+    RP_DEV float4 *vertex(int in, u32 path) const { return vertices[in] + 4 * size_t(path); }
+    RP_DEV float4 *request(u32 path) const { return requests + 4 * size_t(path); }
     // queues
     u32 *queue[2];
     u32 *counters; // [0] queue0, [1] queue1, [3] failures, then the two event sets
@@ -55,10 +74,6 @@ struct PathPool {
     u32 *material; // material a mix-root hit resolved to (written by the closest-hit kernel)
     // statistics (optional)
     unsigned long long *stats; // closest [0] nodes, [1] triangles, [2] rays; shadow [3] rays, [4] nodes, [5] triangles
-    // light-sample requests, one per path (written by the shade kernel, read by k_nee): the
-    // geometric normal, the position's error and the throughput before this event's
-    // continuation; the rest is the latest vertex and the values of the event's start
-    float4 *nee_g, *nee_e, *nee_beta;
     u32 *nee_queue; // three family queues of bin_capacity path ids
     // per-lane walk counts of counting runs (pool slot = request lane), or nullptr: closest-hit
     // walks (written by the closest-hit kernel) and any-hit walks (by the shadow kernel, which
@@ -679,12 +694,13 @@ RP_DEV void store_density(const Density &d, float4 &f, int4 &e) {
     e = make_int4(d.lane[0].exponent, d.lane[1].exponent, d.lane[2].exponent, d.lane[3].exponent);
 }
 
-// The light-sample request of a path's event (PathPool::nee_*), a vertex of family F.
+// The light-sample request of a path's event, a vertex of family F.
 template <int F>
 RP_DEV void read_nee_request(const PathPool &pool, int in, u32 path, u32 flags, SurfacePoint &cp, HeroBsdf &b, V3 &wo,
                              V3 &previous, V4 &beta, Density &density) {
-    const float4 pp = pool.latest_p[in ^ 1][path], n = pool.latest_n[path], g = pool.nee_g[path], e = pool.nee_e[path];
-    const float4 w = pool.ray_d[in][path], v = pool.latest_p[in][path], pa = pool.latest_param[path];
+    const float4 *vertex = pool.vertex(in ^ 1, path), *request = pool.request(path);
+    const float4 pp = vertex[0], n = vertex[1], pa = vertex[2], g = request[0], e = request[1];
+    const float4 w = pool.ray_d(in, path), v = pool.vertex(in, path)[0];
     cp.position = v3(pp.x, pp.y, pp.z);
     cp.shading_normal = v3(n.x, n.y, n.z);
     cp.geometric_normal = v3(g.x, g.y, g.z);
@@ -700,7 +716,7 @@ RP_DEV void read_nee_request(const PathPool &pool, int in, u32 path, u32 flags, 
     b.param[3] = pa.w;
     b.k[0] = b.k[1] = b.k[2] = b.k[3] = 0;
     if constexpr (F == 1) {
-        const float4 k = pool.latest_k[path];
+        const float4 k = vertex[3];
         b.k[0] = k.x;
         b.k[1] = k.y;
         b.k[2] = k.z;
@@ -708,8 +724,8 @@ RP_DEV void read_nee_request(const PathPool &pool, int in, u32 path, u32 flags, 
     }
     wo = -v3(w.x, w.y, w.z);
     previous = v3(v.x, v.y, v.z);
-    beta = from_float4(pool.nee_beta[path]);
-    density = load_density(pool.dens_f[in][path], pool.dens_e[in][path]);
+    beta = from_float4(request[2]);
+    density = load_density(pool.dens_f(in, path), pool.dens_e(in, path));
 }
 
 // shaders/packet_transport.h:77-83
