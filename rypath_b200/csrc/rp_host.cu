@@ -1354,6 +1354,7 @@ std::string validate_request(const rp_scene *s, const rp_request &r) {
     return {};
 }
 
+constexpr u32 kStreamLevels = 5;
 // The scalar step kernel: the plain one, or the full one for scenes with conductors,
 // dielectrics or procedural primitives.
 void launch_scalar_step(const rp_scene *s, unsigned grid, const WaveParams &p, const ScalarParams &q,
@@ -1364,29 +1365,45 @@ void launch_scalar_step(const rp_scene *s, unsigned grid, const WaveParams &p, c
         k_scalar_step<false><<<grid, kTraceBlock, 0, s->stream>>>(s->ds, p, q, w, parity);
 }
 
+// Whether walks of this scene's tree stream (rp_walk.cuh): where rays visit about six nodes or
+// more, so that what the longest of 32 waits for outweighs the streaming's own bookkeeping.
+bool use_stream(const rp_scene *s) { return s->wide_levels >= kStreamLevels; }
 // The closest-hit and shadow kernels with the traversal stack the built tree needs, resolving
-// pass-through and mix-root hits when the scene has them.
+// pass-through and mix-root hits when the scene has them.  Stream: the streaming form.
 template <bool Count, int Block, int Stack>
-void launch_trace_stack(const rp_scene *s, const PathPool &pool, int in, unsigned grid, cudaStream_t st, u32 limit) {
-    if (s->resolve)
+void launch_trace_stack(const rp_scene *s, const PathPool &pool, int in, unsigned grid, cudaStream_t st, u32 limit,
+                        bool stream) {
+    if (s->resolve) {
         k_trace<Count, Block, Stack, true><<<grid, Block, 0, st>>>(s->ds, pool, in, limit);
-    else
-        k_trace<Count, Block, Stack, false><<<grid, Block, 0, st>>>(s->ds, pool, in, limit);
+        return;
+    }
+    if constexpr (!Count)
+        if (stream) {
+            k_trace<false, Block, Stack, false, true><<<grid, Block, 0, st>>>(s->ds, pool, in, limit);
+            return;
+        }
+    k_trace<Count, Block, Stack, false><<<grid, Block, 0, st>>>(s->ds, pool, in, limit);
 }
 template <bool Count, int Block>
-void launch_trace(const rp_scene *s, const PathPool &pool, int in, unsigned grid, cudaStream_t st, u32 limit) {
+void launch_trace(const rp_scene *s, const PathPool &pool, int in, unsigned grid, cudaStream_t st, u32 limit, bool stream) {
     if (s->wide_levels <= u32(kShortStack))
-        launch_trace_stack<Count, Block, kShortStack>(s, pool, in, grid, st, limit);
+        launch_trace_stack<Count, Block, kShortStack>(s, pool, in, grid, st, limit, stream);
     else
-        launch_trace_stack<Count, Block, kStackDepth>(s, pool, in, grid, st, limit);
+        launch_trace_stack<Count, Block, kStackDepth>(s, pool, in, grid, st, limit, stream);
 }
 template <bool Count, int Block, bool Adjoint, int Stack>
 void launch_shadow_stack(const rp_scene *s, const PathPool &pool, int in, unsigned grid, size_t smem, cudaStream_t st,
                          u32 limit) {
-    if (s->resolve)
+    if (s->resolve) {
         k_shadow<Count, Block, Adjoint, Stack, true><<<grid, Block, smem, st>>>(s->ds, pool, in, limit);
-    else
-        k_shadow<Count, Block, Adjoint, Stack, false><<<grid, Block, smem, st>>>(s->ds, pool, in, limit);
+        return;
+    }
+    if constexpr (!Count && !Adjoint)
+        if (use_stream(s)) {
+            k_shadow<false, Block, false, Stack, false, true><<<grid, Block, smem, st>>>(s->ds, pool, in, limit);
+            return;
+        }
+    k_shadow<Count, Block, Adjoint, Stack, false><<<grid, Block, smem, st>>>(s->ds, pool, in, limit);
 }
 template <bool Count, int Block, bool Adjoint>
 void launch_shadow(const rp_scene *s, const PathPool &pool, int in, unsigned grid, size_t smem, cudaStream_t st, u32 limit) {
@@ -1557,9 +1574,9 @@ void run_wave(rp_scene *s, const WaveParams &request_params, size_t adjoint_smem
         s->mark(0);
         const unsigned trace_grid = grid_for(sms, p.lanes, kTraceBlock, 12);
         if (s->counting)
-            launch_trace<true, kTraceBlock>(s, pool, in, trace_grid, s->stream, p.boundary_limit);
+            launch_trace<true, kTraceBlock>(s, pool, in, trace_grid, s->stream, p.boundary_limit, e > 0 && use_stream(s));
         else
-            launch_trace<false, kTraceBlock>(s, pool, in, trace_grid, s->stream, p.boundary_limit);
+            launch_trace<false, kTraceBlock>(s, pool, in, trace_grid, s->stream, p.boundary_limit, e > 0 && use_stream(s));
         s->done();
         if (shadow_pending) {
             RP_CHECK(cudaStreamWaitEvent(s->stream, s->joined, 0));
@@ -1623,6 +1640,7 @@ ScalarSlots scalar_slots(rp_scene *s, u32 count) {
     w.count = count;
     w.remaining = s->scalar_counters + 2;
     w.qcount = s->scalar_counters + 4; // zeroed with the wave's counters
+    w.next_slot = s->scalar_counters + 12;
     return w;
 }
 
@@ -1695,6 +1713,8 @@ void run_scalar_wave(rp_scene *s, const WaveParams &request_params, u32 boundary
                 k_scalar_walk<true, kShortStack><<<walk_grid, kTraceBlock, 0, s->stream>>>(s->ds, p, w, parity, s->stats);
             else if (s->counting)
                 k_scalar_walk<true, kStackDepth><<<walk_grid, kTraceBlock, 0, s->stream>>>(s->ds, p, w, parity, s->stats);
+            else if (short_stack && use_stream(s))
+                k_scalar_walk<false, kShortStack, false, true><<<walk_grid, kTraceBlock, 0, s->stream>>>(s->ds, p, w, parity, s->stats);
             else if (short_stack)
                 k_scalar_walk<false, kShortStack><<<walk_grid, kTraceBlock, 0, s->stream>>>(s->ds, p, w, parity, s->stats);
             else
@@ -3077,7 +3097,7 @@ void batch_wave_kernels(rp_scene *s, const WaveParams &p, const Batch &b, u32 wa
     int in = 0;
     bool shadow_pending = false;
     for (u32 e = 0; e <= s->ds.max_depth; ++e) {
-        launch_trace<false, TB>(s, pool, in, trace_grid, st, p.boundary_limit);
+        launch_trace<false, TB>(s, pool, in, trace_grid, st, p.boundary_limit, e > 0 && use_stream(s));
         if (shadow_pending) {
             RP_CHECK(cudaStreamWaitEvent(st, s->joined, 0));
             shadow_pending = false;
@@ -4004,7 +4024,8 @@ rp_status rp_cuda_sample_device_static(rp_scene *s, const rp_request *request, r
         k_raygen<<<grid_for(sms, p.lanes, 256, 16), 256, 0, st>>>(s->ds, p, pool);
         int in = 0;
         for (u32 ev = 0; ev < s->ds.max_depth + 1; ++ev) {
-            launch_trace<false, kTraceBlock>(s, pool, in, grid_for(sms, p.lanes, kTraceBlock, 12), st, p.boundary_limit);
+            launch_trace<false, kTraceBlock>(s, pool, in, grid_for(sms, p.lanes, kTraceBlock, 12), st, p.boundary_limit,
+                                             ev > 0 && use_stream(s));
             const unsigned shade_grid = grid_for(sms, p.lanes, 128, 16);
             k_shade<3><<<shade_grid, 128, 0, st>>>(s->ds, p, pool, in, ev);
             if (s->family_mask & 1u) {

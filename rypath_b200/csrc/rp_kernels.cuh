@@ -2,6 +2,7 @@
 #pragma once
 
 #include "rp_transport.cuh"
+#include "rp_walk.cuh"
 
 namespace rp {
 
@@ -139,17 +140,64 @@ __device__ __noinline__ u32 resolve_hit(const DeviceScene &s, const PathPool &po
 // Closest-hit queries for the active queue; each path is then appended to the bin of the
 // BSDF family it hit (0 diffuse, 1 conductor, 2 dielectric, 3 miss or failed query), so the
 // shade stage runs one specialised kernel per family ("material-sorted shading").
+struct TraceRays {
+    const DeviceScene &s;
+    const PathPool &pool;
+    const u32 *queue;
+    int in;
+    u32 *event;
+    StagedAppend bins;
+    u32 path;
+
+    template <class W> RP_DEV bool load(u32 i, W &w) {
+        path = queue[i];
+        if (pool.ident(path).w & F_COMPLETE)
+            return false;
+        const float4 o = pool.ray_o(in, path), d = pool.ray_d(in, path);
+        w.start(s, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), __int_as_float(0x7f800000));
+        return true;
+    }
+    template <class W> RP_DEV void finish(bool done, const W &w) {
+        u32 family = 4;
+        if (done) {
+            const u32 prim = w.ok ? w.h.prim : kHitInvalid;
+            family = (!w.ok || w.h.prim == kNone) ? 3u : u32(__ldg(s.tri_family + w.h.prim));
+            pool.hit(path) = make_float4(w.h.t, w.h.b1, w.h.b2, __uint_as_float(prim));
+        }
+#pragma unroll
+        for (u32 f = 0; f < 4; ++f)
+            bins.push(f, family == f, path, event + kBinCount + f, pool.bins + size_t(f) * pool.bin_capacity);
+    }
+    RP_DEV void flush() {
+#pragma unroll
+        for (u32 f = 0; f < 4; ++f)
+            bins.flush(f, event + kBinCount + f, pool.bins + size_t(f) * pool.bin_capacity);
+    }
+};
+// Blocks per SM of the walk kernels: with the short stack, eight of 128 threads (64 registers)
+// for the plain form and six (80) for the streaming one, whose state spills at 64.
+constexpr int walk_blocks(int block, int stack, bool stream) {
+    return stack > kShortStack ? 1 : (stream ? 768 : 1024) / block;
+}
 // Stack: traversal stack entries per thread (kShortStack for shallow trees, whose walks then
 // fit eight 128-thread blocks per SM).
 // Resolve: the scene has pass-through, mix-root or procedural instances (resolve_hit).
-template <bool Count, int Block = kTraceBlock, int Stack = kStackDepth, bool Resolve = false>
-__global__ void __launch_bounds__(Block, Stack <= kShortStack ? 1024 / Block : 1)
+// Stream: walk_stream, else a ray a thread at a time (use_stream says when).
+template <bool Count, int Block = kTraceBlock, int Stack = kStackDepth, bool Resolve = false, bool Stream = false>
+__global__ void __launch_bounds__(Block, walk_blocks(Block, Stack, Stream))
     k_trace(const __grid_constant__ DeviceScene s, PathPool pool, int in, u32 boundary_limit) {
     __shared__ uint2 stack[Stack * Block];
     const u32 count = pool.counters[in];
     u32 *event = pool.event(in);
     if (blockIdx.x == 0 && threadIdx.x == 0)
         pool.counters[in ^ 1] = 0;
+    if constexpr (Stream) {
+        static_assert(!Count && !Resolve);
+        __shared__ u32 stage[Block / 32 * 4 * kStageEntries];
+        TraceRays io{s, pool, pool.queue[in], in, event, {stage + (threadIdx.x >> 5) * 4 * kStageEntries, 0}, 0};
+        walk_stream<Walker<false, Stack, false>>(s, count, event + kTraceNext, stack + threadIdx.x, Block, io);
+        return;
+    }
     const u32 *queue = pool.queue[in];
     u32 nodes = 0, tris = 0, rays = 0;
     const u32 stride = gridDim.x * blockDim.x;
@@ -867,10 +915,31 @@ RP_DEV void shadow_result(const DeviceScene &s, const PathPool &pool, float *sgr
                            pool.adj_w[path]);
     }
 }
+template <bool Adjoint> struct ShadowRays {
+    const DeviceScene &s;
+    const PathPool &pool;
+    float *sgrad;
+    u32 entry;
+
+    template <class W> RP_DEV bool load(u32 i, W &w) {
+        entry = i;
+        const float4 o = pool.sh_o[i], d = pool.sh_d[i];
+        w.start(s, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), o.w);
+        return true;
+    }
+    template <class W> RP_DEV void finish(bool done, const W &w) {
+        if (!done)
+            return;
+        const u32 path = __float_as_uint(pool.sh_d[entry].w);
+        shadow_result<Adjoint>(s, pool, sgrad, pool.sh_c[entry], path, w.ok ? 0u : 3u, w.h.prim != kNone);
+    }
+    RP_DEV void flush() {}
+};
 // Visibility of the light samples, opaque surfaces; Resolve: the scene has pass-through
 // instances, which shadow rays cross (pass_through_visible).
-template <bool Count, int Block = kTraceBlock, bool Adjoint = false, int Stack = kStackDepth, bool Resolve = false>
-__global__ void __launch_bounds__(Block, Stack <= kShortStack ? 1024 / Block : 1)
+template <bool Count, int Block = kTraceBlock, bool Adjoint = false, int Stack = kStackDepth, bool Resolve = false,
+          bool Stream = false>
+__global__ void __launch_bounds__(Block, walk_blocks(Block, Stack, Stream))
     k_shadow(const __grid_constant__ DeviceScene s, PathPool pool, int in, u32 boundary_limit) {
     __shared__ uint2 stack[Stack * Block];
     extern __shared__ float sgrad[]; // adjoint only
@@ -879,25 +948,31 @@ __global__ void __launch_bounds__(Block, Stack <= kShortStack ? 1024 / Block : 1
     u32 *event = pool.event(in);
     const u32 count = event[kShadowCount];
     u32 nodes = 0, tris = 0, rays = 0;
-    for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-        const float4 o = pool.sh_o[i], d = pool.sh_d[i];
-        const u32 path = __float_as_uint(d.w);
-        const u32 walks_before = rays;
-        bool occluded;
-        u32 failure = 0;
-        if (Resolve) {
-            failure = pass_through_visible<Count, Stack>(s, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), o.w, pool.sh_t[i],
-                                                         occluded, stack + threadIdx.x, Block, boundary_limit, nodes,
-                                                         tris, rays);
-        } else {
-            if (!walk_any<Count, Stack, false>(s, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), o.w, occluded,
-                                               stack + threadIdx.x, Block, nodes, tris))
-                failure = 3;
-            ++rays;
+    if constexpr (Stream) {
+        static_assert(!Count && !Resolve);
+        ShadowRays<Adjoint> io{s, pool, sgrad, 0};
+        walk_stream<Walker<true, Stack, false>>(s, count, event + kShadowNext, stack + threadIdx.x, Block, io);
+    } else {
+        for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+            const float4 o = pool.sh_o[i], d = pool.sh_d[i];
+            const u32 path = __float_as_uint(d.w);
+            const u32 walks_before = rays;
+            bool occluded;
+            u32 failure = 0;
+            if (Resolve) {
+                failure = pass_through_visible<Count, Stack>(s, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), o.w, pool.sh_t[i],
+                                                             occluded, stack + threadIdx.x, Block, boundary_limit, nodes,
+                                                             tris, rays);
+            } else {
+                if (!walk_any<Count, Stack, false>(s, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), o.w, occluded,
+                                                   stack + threadIdx.x, Block, nodes, tris))
+                    failure = 3;
+                ++rays;
+            }
+            if (Count && pool.lane_shadow)
+                pool.lane_shadow[path] += rays - walks_before;
+            shadow_result<Adjoint>(s, pool, sgrad, pool.sh_c[i], path, failure, occluded);
         }
-        if (Count && pool.lane_shadow)
-            pool.lane_shadow[path] += rays - walks_before;
-        shadow_result<Adjoint>(s, pool, sgrad, pool.sh_c[i], path, failure, occluded);
     }
     if (Adjoint)
         adjoint_end(pool, sgrad);

@@ -89,13 +89,13 @@ struct PathPool {
     double adj_inv_weight;  // 1 / film weight of a pixel (its sample count)
     u32 adj_params;         // gradient entries
 
-    // The counters of the event whose paths are in queue `in`: family bins, light samples and
-    // shadow segments.  Events alternate between two sets, and the
+    // The counters of the event whose paths are in queue `in`: family bins, light samples,
+    // shadow segments and the two walks' next rays.  Events alternate between two sets, and the
     // escape shade kernel of an event, by when every kernel of the event before it has ended,
     // clears the other set; its closest-hit kernel clears the queue it will fill.
     RP_DEV u32 *event(int in) const { return counters + 16 + 16 * in; }
 };
-enum : u32 { kBinCount = 0, kNeeCount = 4, kShadowCount = 7, kEventCounters = 8 };
+enum : u32 { kBinCount = 0, kNeeCount = 4, kShadowCount = 7, kTraceNext = 8, kShadowNext = 9, kEventCounters = 10 };
 
 // sampler: 0 independent, 1 Sobol, 2 Halton, 3 ZSobol (src/render_wire.h:41)
 struct WaveParams {
