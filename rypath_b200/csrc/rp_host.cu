@@ -1360,9 +1360,9 @@ constexpr u32 kStreamLevels = 5;
 void launch_scalar_step(const rp_scene *s, unsigned grid, const WaveParams &p, const ScalarParams &q,
                         const ScalarSlots &w, int parity) {
     if (s->scalar_full)
-        k_scalar_step<true><<<grid, kTraceBlock, 0, s->stream>>>(s->ds, p, q, w, parity);
+        k_scalar_step<true><<<grid, kStepBlock, 0, s->stream>>>(s->ds, p, q, w, parity);
     else
-        k_scalar_step<false><<<grid, kTraceBlock, 0, s->stream>>>(s->ds, p, q, w, parity);
+        k_scalar_step<false><<<grid, kStepBlock, 0, s->stream>>>(s->ds, p, q, w, parity);
 }
 
 // Whether walks of this scene's tree stream (rp_walk.cuh): where rays visit about six nodes or
@@ -1644,13 +1644,13 @@ ScalarSlots scalar_slots(rp_scene *s, u32 count) {
     return w;
 }
 
-// Slots of the scalar wavefront (at most this many paths in flight per wave), and the
-// walk/step trips between two host reads of the wave's remaining lanes.  262,144 slots of
-// about 230 bytes (path, connection, mode, hit, queue entries) keep the path state (60 MB)
-// in L2 and give the step kernel several paths per resident thread; measured on the fog box
-// (1024x1024, 16 spp) with the step queues: 2^16 slots 314 ms, 2^17 317 ms, 2^18 300 ms;
-// without them 2^17 415 ms, 2^19 529 ms, 2^20 634 ms.
-constexpr u32 kScalarSlots = 1u << 18;
+// Slots of the scalar wavefront for each SM (at most this many paths in flight per wave), and
+// the walk/step trips between two host reads of the wave's remaining lanes.  2,048 slots are
+// four for each thread of the step kernel (two blocks of 256 an SM) and two for each of the
+// walk (eight of 128), so a trip's passes over them are whole, and the state of the 303,104 paths
+// of 148 SMs (70 MB) stays in L2.  Fog box 512x512, 16 spp: 2^18 slots, whose last step pass is
+// half empty, 34.0 ms, 148 x 2048 32.5 ms.
+constexpr u32 kScalarSlotsPerSm = 2048;
 constexpr int kScalarTripsPerCheck = 8;
 
 // One wave of the scalar transport, one record per lane in s->scalar_records: camera rays,
@@ -1662,9 +1662,9 @@ void run_scalar_wave(rp_scene *s, const WaveParams &request_params, u32 boundary
     if (!s->step_blocks) {
         int per_sm = 0;
         if (s->scalar_full)
-            RP_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_scalar_step<true>, kTraceBlock, 0));
+            RP_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_scalar_step<true>, kStepBlock, 0));
         else
-            RP_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_scalar_step<false>, kTraceBlock, 0));
+            RP_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_scalar_step<false>, kStepBlock, 0));
         s->step_blocks = std::max(1, per_sm);
     }
     s->mark(3);
@@ -1679,12 +1679,12 @@ void run_scalar_wave(rp_scene *s, const WaveParams &request_params, u32 boundary
     q.fresh_index = s->scalar_fresh_index;
     q.next_lane = s->scalar_counters;
     q.stats = s->stats;
-    const u32 slots = std::min<u32>(std::max<u32>(p.lanes, 1), kScalarSlots);
+    const u32 slots = std::min<u32>(std::max<u32>(p.lanes, 1), u32(s->sm_count) * kScalarSlotsPerSm);
     const ScalarSlots w = scalar_slots(s, slots);
     const u32 lanes = p.lanes;
     RP_CHECK(cudaMemcpyAsync(w.remaining, &lanes, sizeof(u32), cudaMemcpyHostToDevice, s->stream));
     const int walk_grid = grid_for(s->sm_count, slots, kTraceBlock, 8);
-    const int step_grid = grid_for(s->sm_count, slots, kTraceBlock, s->step_blocks);
+    const int step_grid = grid_for(s->sm_count, slots, kStepBlock, s->step_blocks);
     const bool short_stack = s->wide_levels <= u32(kShortStack);
     s->mark(2, 2);
     k_scalar_slots_init<<<grid_for(s->sm_count, slots, 256, 8), 256, 0, s->stream>>>(w.mode, slots);

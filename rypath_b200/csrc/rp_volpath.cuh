@@ -306,7 +306,7 @@ RP_DEV bool incident_delta(const Incident &l) { return l.kind == kIncidentPositi
 
 // ------------------------------------------------------------------ path state
 // ScalarState (shaders/scalar_transport.h:38-52), kept in a wavefront slot between trips.
-struct ScalarPath {
+struct __align__(16) ScalarPath {
     u32 lane, pixel, slo, shi, status, scatterings;
     u64 index;
     float wavelength, radiance;
@@ -324,7 +324,7 @@ enum : u32 { kAfterContinue = 0, kAfterFinish = 1, kAfterFail = 2 /* + status <<
 // trace, or visible_shadow (:1570-1576) in scenes without media.  It carries the contribution
 // it adds when it resolves with transmittance T: a surface sample adds a * T, a medium sample
 // checks value = a * T and adds b * value (shaders/render.metal:2237-2260).
-struct Connection {
+struct __align__(16) Connection {
     V3 o, d;         // current leg; d is a unit vector except for the vacuum query
     float remaining; // leg length (world), or the parametric limit of the vacuum query
     V3 end;
@@ -673,9 +673,11 @@ RP_DEV u32 dielectric_lobe_word(const DeviceScene &s, const WaveParams &p, u32 p
 }
 
 // One event after the path ray's closest hit: scalar_shade (shaders/scalar_transport.h:286-900)
-// for diffuse, conductor and dielectric surfaces and null interfaces.  A light sample that needs a connection leaves it in
-// `c` (returning kEventConnect) after the continuation has been sampled: the two use disjoint
-// draws, and the connection's contribution and status are applied before the continuation's.
+// for diffuse, conductor and dielectric surfaces and null interfaces, in two parts around its
+// light sample, so that the warps of a block can meet between them.  A light sample that needs
+// a connection leaves it in `c` (returning kEventConnect) after the continuation has been
+// sampled: the two use disjoint draws, and the connection's contribution and status are applied
+// before the continuation's.
 // The surface point of a path hit: any primitive kind, or triangles alone in the plain kernel.
 template <bool Full>
 RP_DEV bool scalar_surface_point(const DeviceScene &s, u32 prim, u32 inst, u32 local, float b1, float b2,
@@ -684,11 +686,27 @@ RP_DEV bool scalar_surface_point(const DeviceScene &s, u32 prim, u32 inst, u32 l
         return hit_surface_point(s, prim, inst, local, b1, b2, point);
     return triangle_surface_point(s, inst, local, b1, b2, true, point);
 }
+// What a path event holds across its light sample (shade_begin to shade_end).
+enum : int { kEventLight = 3 }; // shade_begin: the event goes on after its light sample
+struct ScalarEvent {
+    bool medium, wants_light, microfacet, directional_offset;
+    V3 position, normal; // the light sample's context
+    float selection, ux, uy;
+    uint4 words;  // phase or BSDF words
+    V3 direction; // medium: the ray's unit direction
+    u32 inst;
+    SurfacePoint point;
+    float rho;
+    V3 n, area_reference;
+    ScalarBsdf bsdf;
+    Frame frame;
+    V3 wo;
+};
 // Full: the scene has conductor or dielectric surfaces, procedural primitives or image
 // reflectance (their code is compiled out of the plain step kernel).
 template <bool Full>
-RP_DEV int shade_event(const DeviceScene &s, const WaveParams &p, const ScalarParams &q, ScalarPath &path, bool ok,
-                       const Hit &hit, Connection &c) {
+RP_DEV int shade_begin(const DeviceScene &s, const WaveParams &p, const ScalarParams &q, ScalarPath &path, bool ok,
+                       const Hit &hit, ScalarEvent &ev) {
     if (!ok) {
         path.status = S_HIT;
         return kEventFinished;
@@ -739,65 +757,15 @@ RP_DEV int shade_event(const DeviceScene &s, const WaveParams &p, const ScalarPa
                 path.throughput *= sc / total;
                 const uint4 light_words = medium_words(p, path.pixel, path.slo, path.shi, path.medium_draw);
                 const uint4 phase_words = medium_words(p, path.pixel, path.slo, path.shi, path.medium_draw);
-                const float g = __ldg(m + 1413);
-                // medium_direct (shaders/render.metal:2237-2260)
-                const Incident light = scalar_light_sample(s, path.wavelength, position, v3(0, 0, 0),
-                                                           u01(light_words.x), u01(light_words.y), u01(light_words.z));
-                if (!light.valid) {
-                    path.status = S_ARITHMETIC;
-                    return kEventFinished;
-                }
-                bool connect = false;
-                if (light.pdf > 0 && light.radiance != 0) {
-                    V3 cd;
-                    // connection (shaders/scalar_lighting.h:121-133): the environment's is unbounded
-                    const bool unbounded = light.kind == kIncidentEnvironment;
-                    if (light.kind == kIncidentArea) {
-                        const V3 delta = light.target.position - position;
-                        cd = shadow_segment_direction(position, delta, light.target,
-                                                      dot(light.target.geometric_normal, -delta));
-                    } else {
-                        cd = unbounded ? light.direction : light.endpoint - position;
-                    }
-                    if (!connection_begin(position, cd, unbounded ? finf() : kOneMinusEps, path.current_medium, c)) {
-                        path.status = S_ARITHMETIC;
-                        return kEventFinished;
-                    }
-                    const float phase = hg_phase(-direction, light.direction, g);
-                    const float weight = incident_delta(light) ? 1.f : power_weight(light.pdf, phase);
-                    c.medium_sample = true;
-                    c.a = ((phase / light.pdf) * weight) * light.radiance;
-                    c.b = path.throughput;
-                    connect = true;
-                }
-                // phase continuation and roulette
-                u32 after = kAfterContinue;
-                const V3 wi_dir = hg_sample(-direction, g, u01(phase_words.x), u01(phase_words.y));
-                const float pdf = hg_phase(-direction, wi_dir, g);
-                if (!finite3(wi_dir) || !(pdf > 0) || !isfinite(pdf)) {
-                    after = kAfterFail | (S_ARITHMETIC << 8);
-                } else {
-                    path.previous_bsdf_pdf = pdf;
-                    ++path.scatterings;
-                    if (path.scatterings >= 3 && phase_words.z >= 0xc0000000u) {
-                        after = kAfterFinish;
-                    } else {
-                        if (path.scatterings >= 3)
-                            path.throughput /= .75f;
-                        path.previous_delta = false;
-                        path.prev_p = position;
-                        path.prev_n = v3(0, 0, 0);
-                        path.escape_weight = 1;
-                        path.o = position;
-                        path.d = wi_dir;
-                        path.boundary_crossings = 0;
-                    }
-                }
-                if (connect) {
-                    c.after = after;
-                    return kEventConnect;
-                }
-                return apply_after(path, after);
+                ev.medium = ev.wants_light = true;
+                ev.position = position;
+                ev.normal = v3(0, 0, 0);
+                ev.selection = u01(light_words.x);
+                ev.ux = u01(light_words.y);
+                ev.uy = u01(light_words.z);
+                ev.direction = direction;
+                ev.words = phase_words;
+                return kEventLight;
             }
         }
     }
@@ -985,13 +953,115 @@ RP_DEV int shade_event(const DeviceScene &s, const WaveParams &p, const ScalarPa
     // the third word decides the roulette, from the third scattering on
     const uint4 bsdf_words = draw_words(s, p, path.pixel, path.slo, path.shi, path.index, 1 + 2 * bounce,
                                         path.scatterings >= 2 ? kDrawXYZ | kDrawCoarseZ : kDrawXY);
+    ev.medium = false;
+    ev.wants_light = s.model != kModelDemo && !dirac;
+    ev.position = point.position;
+    ev.normal = context_normal;
+    ev.selection = sample_uniform(p, light_words.x);
+    ev.ux = sample_uniform(p, light_words.y);
+    ev.uy = sample_uniform(p, light_words.z);
+    ev.words = bsdf_words;
+    ev.inst = inst;
+    ev.point = point;
+    ev.rho = rho;
+    ev.n = n;
+    ev.area_reference = area_reference;
+    ev.microfacet = microfacet;
+    ev.directional_offset = directional_offset;
+    if (Full) {
+        ev.bsdf = bsdf;
+        ev.frame = frame;
+        ev.wo = wo;
+    }
+    return kEventLight;
+}
+// The rest of the event, once its light is sampled.
+template <bool Full>
+RP_DEV int shade_end(const DeviceScene &s, const WaveParams &p, ScalarPath &path, const Hit &hit, const ScalarEvent &ev,
+                     const Incident &light, Connection &c) {
+    if (ev.medium) {
+        const V3 position = ev.position, direction = ev.direction;
+        const uint4 phase_words = ev.words;
+        const float g = __ldg(medium_record(s, path.current_medium) + 1413);
+        // medium_direct (shaders/render.metal:2237-2260)
+        if (!light.valid) {
+            path.status = S_ARITHMETIC;
+            return kEventFinished;
+        }
+        bool connect = false;
+        if (light.pdf > 0 && light.radiance != 0) {
+            V3 cd;
+            // connection (shaders/scalar_lighting.h:121-133): the environment's is unbounded
+            const bool unbounded = light.kind == kIncidentEnvironment;
+            if (light.kind == kIncidentArea) {
+                const V3 delta = light.target.position - position;
+                cd = shadow_segment_direction(position, delta, light.target,
+                                              dot(light.target.geometric_normal, -delta));
+            } else {
+                cd = unbounded ? light.direction : light.endpoint - position;
+            }
+            if (!connection_begin(position, cd, unbounded ? finf() : kOneMinusEps, path.current_medium, c)) {
+                path.status = S_ARITHMETIC;
+                return kEventFinished;
+            }
+            const float phase = hg_phase(-direction, light.direction, g);
+            const float weight = incident_delta(light) ? 1.f : power_weight(light.pdf, phase);
+            c.medium_sample = true;
+            c.a = ((phase / light.pdf) * weight) * light.radiance;
+            c.b = path.throughput;
+            connect = true;
+        }
+        // phase continuation and roulette
+        u32 after = kAfterContinue;
+        const V3 wi_dir = hg_sample(-direction, g, u01(phase_words.x), u01(phase_words.y));
+        const float pdf = hg_phase(-direction, wi_dir, g);
+        if (!finite3(wi_dir) || !(pdf > 0) || !isfinite(pdf)) {
+            after = kAfterFail | (S_ARITHMETIC << 8);
+        } else {
+            path.previous_bsdf_pdf = pdf;
+            ++path.scatterings;
+            if (path.scatterings >= 3 && phase_words.z >= 0xc0000000u) {
+                after = kAfterFinish;
+            } else {
+                if (path.scatterings >= 3)
+                    path.throughput /= .75f;
+                path.previous_delta = false;
+                path.prev_p = position;
+                path.prev_n = v3(0, 0, 0);
+                path.escape_weight = 1;
+                path.o = position;
+                path.d = wi_dir;
+                path.boundary_crossings = 0;
+            }
+        }
+        if (connect) {
+            c.after = after;
+            return kEventConnect;
+        }
+        return apply_after(path, after);
+    }
+    const u32 bounce = path.scatterings;
+    const DInstance &instance = s.instances[ev.inst];
+    const SurfacePoint &point = ev.point;
+    const bool microfacet = Full && ev.microfacet, directional_offset = ev.directional_offset;
+    const float rho = ev.rho;
+    const V3 n = ev.n, wo = Full ? ev.wo : v3(0, 0, 0), area_reference = ev.area_reference, context_normal = ev.normal;
+    ScalarBsdf bsdf{};
+    Frame frame{};
+    if (Full) {
+        bsdf = ev.bsdf;
+        frame = ev.frame;
+    }
+    const bool dirac = microfacet && bsdf.g.smooth; // delta_only (shaders/scattering.h:25-28)
+    const bool both_hemispheres = microfacet && bsdf.kind == 2;
+    const uint4 bsdf_words = ev.words;
     // light sample: the demo model's sky sampled uniformly over the sphere with the
     // cosine-ratio weight (:709-781); PBRT scenes' lights with power-heuristic MIS (:783-835).
     // Dirac surfaces take no light sample.
     bool connect = false;
     if (s.model == kModelDemo) {
         const float E = 1.0f; // sky_radiance of the demo model
-        const float uz = sample_uniform(p, light_words.x), uv = sample_uniform(p, light_words.y);
+        const float uz = ev.selection, uv = ev.ux;
         const float z = 1.0f - 2.0f * uz;
         const float r = sqrtf(fmaxf(0.0f, 1.0f - z * z));
         const float phi = 2.0f * kPi * uv;
@@ -1033,9 +1103,6 @@ RP_DEV int shade_event(const DeviceScene &s, const WaveParams &p, const ScalarPa
             connect = true;
         }
     } else if (!dirac) {
-        const Incident light = scalar_light_sample(s, path.wavelength, point.position, context_normal,
-                                                   sample_uniform(p, light_words.x), sample_uniform(p, light_words.y),
-                                                   sample_uniform(p, light_words.z));
         if (!light.valid) {
             path.status = S_ARITHMETIC;
             return kEventFinished;
@@ -1194,7 +1261,7 @@ RP_DEV bool scalar_ray_valid(const ScalarPath &path) {
     return finite3(path.o) && finite3(path.d) && isfinite(path.throughput) && isfinite(path.radiance);
 }
 
-// Whether shade_event will take its medium-scattering branch for this hit: the same medium
+// Whether shade_begin will take its medium-scattering branch for this hit: the same medium
 // lookup and free-flight draw, without consuming the draw.  Only groups the step warps; the
 // step itself decides.
 RP_DEV bool predicts_medium_scatter(const DeviceScene &s, const WaveParams &p, const ScalarPath &path, const Hit &hit) {
@@ -1367,10 +1434,14 @@ __global__ void k_scalar_slots_init(u32 *mode, u32 count) {
 // lanes for the finished ones (one atomic per warp).  parity >= 0: the slots the walk of this
 // trip queued, connection steps first, then medium-scattering path events, null-interface
 // events and the other path events; parity < 0: every slot (the wave's first fill, and geometry-free scenes, which
-// take no walk).  Four blocks of 128 per SM (128 registers, a few spilled) hide more of the
-// slot loads' latency than three at 154 registers: 133 against 143 ms on the fog box.
+// take no walk).  512 threads per SM (128 registers, a few spilled) hide more of the slot loads'
+// latency than three blocks of 128 at 154 registers: 133 against 143 ms on the fog box at 1024x1024.
+// Two blocks of 256, whose warps meet before an event and around its light sample in scenes with
+// media, fetch the divergent code's instructions once for eight warps: fog box 512x512, 16 spp
+// 35.3 ms with four blocks of 128, 32.6 meeting once a trip, 31.8 also around the light sample.
+constexpr int kStepBlock = 256;
 template <bool Full>
-__global__ void __launch_bounds__(kTraceBlock, 4) k_scalar_step(const __grid_constant__ DeviceScene s,
+__global__ void __launch_bounds__(kStepBlock, 512 / kStepBlock) k_scalar_step(const __grid_constant__ DeviceScene s,
                                                              const __grid_constant__ WaveParams p, ScalarParams q,
                                                              ScalarSlots w, int parity) {
     const int lane_in_warp = threadIdx.x & 31;
@@ -1389,6 +1460,9 @@ __global__ void __launch_bounds__(kTraceBlock, 4) k_scalar_step(const __grid_con
     const u32 trips = (total + stride - 1) / stride;
     for (u32 trip = 0; trip < trips; ++trip) {
         const u32 k = trip * stride + blockIdx.x * blockDim.x + threadIdx.x;
+        const bool sync = s.media_enabled; // the block's warps share the lines of instructions they fetch
+        if (sync)
+            __syncthreads();
         u32 i = k;
         if (parity >= 0 && k < total)
             i = k < n_connect     ? w.queue_connect[parity][k]
@@ -1396,15 +1470,20 @@ __global__ void __launch_bounds__(kTraceBlock, 4) k_scalar_step(const __grid_con
                 : k < n_interface ? w.queue_interface[parity][k - n_medium]
                                   : w.queue_path[parity][k - n_interface];
         u32 mode = kEventFinished;
-        bool finished_now = false;
+        bool finished_now = false, active = false;
+        ScalarPath path;
+        // a connection in flight is read only by its steps, and a path event that begins one
+        // sets it up whole (connection_begin and the event's weights)
+        Connection c;
+        Hit hit;
+        ScalarEvent ev;
+        ev.wants_light = false;
         if (k < total) {
             const u32 m = w.mode[i];
             mode = m & 0xffu;
-            if (mode != kEventFinished) {
-                ScalarPath path = w.path[i];
-                // a connection in flight is read only by its steps, and a path event that
-                // begins one sets it up whole (connection_begin and the event's weights)
-                Connection c;
+            active = mode != kEventFinished;
+            if (active) {
+                path = w.path[i];
                 if (mode == kEventConnect)
                     c = w.conn[i];
                 if (s.instance_count == 0) {
@@ -1414,21 +1493,33 @@ __global__ void __launch_bounds__(kTraceBlock, 4) k_scalar_step(const __grid_con
                     path.status = S_ARITHMETIC;
                     mode = kEventFinished;
                 } else {
-                    const Hit hit = w.hit[i];
+                    hit = w.hit[i];
                     const bool ok = (m & kWalkOk) != 0;
-                    mode = mode == kEventPath ? shade_event<Full>(s, p, q, path, ok, hit, c)
+                    mode = mode == kEventPath ? shade_begin<Full>(s, p, q, path, ok, hit, ev)
                                               : connection_step(s, q, path, c, ok, hit);
                 }
-                if (mode == kEventFinished) {
-                    q.out[path.lane] = scalar_record(path);
-                    finished_now = true;
-                } else {
-                    w.path[i] = path;
-                    if (mode == kEventConnect)
-                        w.conn[i] = c;
-                }
-                w.mode[i] = mode;
             }
+        }
+        if (sync)
+            __syncthreads();
+        if (mode == kEventLight) {
+            Incident light;
+            light.valid = true;
+            light.pdf = light.radiance = 0;
+            if (ev.wants_light)
+                light = scalar_light_sample(s, path.wavelength, ev.position, ev.normal, ev.selection, ev.ux, ev.uy);
+            mode = shade_end<Full>(s, p, path, hit, ev, light, c);
+        }
+        if (active) {
+            if (mode == kEventFinished) {
+                q.out[path.lane] = scalar_record(path);
+                finished_now = true;
+            } else {
+                w.path[i] = path;
+                if (mode == kEventConnect)
+                    w.conn[i] = c;
+            }
+            w.mode[i] = mode;
         }
         // records written this trip
         const u32 done = __ballot_sync(0xffffffffu, finished_now);
