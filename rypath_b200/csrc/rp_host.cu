@@ -1524,8 +1524,16 @@ void attach_draw_tables(rp_scene *s, WaveParams &p) {
     p.draw_blocks = blocks;
 }
 
-// Waves of at most this many lanes run as whole paths (k_paths).
-constexpr u32 kWholePathLanes = 32768;
+// Waves of so few lanes that whole paths (k_paths) beat the launches of their events: 512 lanes an
+// event, 2,048 in scenes of one BSDF family, whose warps do not diverge over the families' code.
+// One sample a pixel, whole paths against the wavefront, ms: Cornell box (one family, 9 events)
+// 0.59 / 1.10 at 6,144 lanes, 1.01 / 1.14 at 19,200, 1.75 / 1.17 at 49,152; the box with glass and
+// a conductor 1.19 / 1.18 at 6,144, 2.22 / 1.20 at 19,200; mixed scene (17 events) 1.40 / 3.12 at
+// 6,144, 2.07 / 3.53 at 19,200, 4.72 / 4.17 at 76,800.
+bool whole_paths(const rp_scene *s, u32 lanes) {
+    const bool one_family = (s->family_mask & (s->family_mask - 1)) == 0;
+    return u64(lanes) <= u64(s->ds.max_depth + 1) * (one_family ? 2048u : 512u);
+}
 void launch_paths(rp_scene *s, const WaveParams &p, const PathPool &pool) {
     const unsigned grid = grid_for(s->sm_count, p.lanes, kPathBlock, 64);
     const bool img = s->ds.img.textured || s->ds.img.env_image != kNone, deep = s->wide_levels > u32(kShortStack);
@@ -1560,7 +1568,7 @@ void run_wave(rp_scene *s, const WaveParams &request_params, size_t adjoint_smem
     RP_CHECK(cudaMemsetAsync(pool.counters, 0, 64 * sizeof(u32), s->stream));
     k_raygen<<<grid_for(sms, p.lanes, 256, 16), 256, 0, s->stream>>>(s->ds, p, pool);
     s->done();
-    if (p.lanes <= kWholePathLanes && !s->resolve && !s->counting && !pool.hist) {
+    if (whole_paths(s, p.lanes) && !s->resolve && !s->counting && !pool.hist) {
         s->mark(2);
         launch_paths(s, p, pool);
         s->done();

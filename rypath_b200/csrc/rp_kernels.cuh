@@ -983,11 +983,12 @@ __global__ void __launch_bounds__(Block, walk_blocks(Block, Stack, Stream))
     }
 }
 
-// Whole paths, one thread each: every event of a wave's paths, each the closest hit, the event, its light sample and that sample's visibility in turn, on the
-// same path state as the wavefront kernels (so every lane's result is theirs).  A wave of few
-// lanes is bound by the launches of its events (about eleven kernels each), not by their work:
-// one launch runs it instead.  Its warps diverge over the families, so it is for waves of at
-// most kWholePathLanes lanes; scenes whose hits resolve before shading take the wavefront.
+// Whole paths, one thread each: every event of a wave's paths, each the closest hit, the event,
+// its light sample and that sample's visibility in turn, on the same path state as the wavefront
+// kernels (so every lane's result is theirs).  A wave of few lanes is bound by the launches and
+// the latencies of its events' kernels, not by their work: one launch runs it instead
+// (whole_paths says when: its warps diverge over the families).  Scenes whose hits resolve before
+// shading take the wavefront.
 constexpr int kPathBlock = 64;
 template <int Stack, bool Img>
 __global__ void __launch_bounds__(kPathBlock, 6) k_paths(const __grid_constant__ DeviceScene s,
