@@ -1479,8 +1479,8 @@ void launch_shade(rp_scene *s, const WaveParams &p, const PathPool &pool, int in
 // Sobol sampler with Owen randomisation: attaches the tables of the draw blocks of the scene's
 // transport, building them on the scene stream when the seed or depth changed.  Hero: the
 // continuation and light-sample blocks [4, 4 + n) and [133, 133 + n), one of each per vertex up
-// to the maximum depth; scalar: blocks [1, 1 + n), two per vertex.  Every word drawn through
-// them equals the fully computed word.
+// to the maximum depth; scalar: blocks [1, 1 + n), two per vertex; both: block 0, the camera's.
+// Every word drawn through them equals the fully computed word.
 void attach_draw_tables(rp_scene *s, WaveParams &p) {
     p.owen_prefix = nullptr;
     p.draw_bytes = nullptr;
@@ -1491,7 +1491,7 @@ void attach_draw_tables(rp_scene *s, WaveParams &p) {
     const bool hero = s->transport == RP_TRANSPORT_HERO;
     const u32 depth = std::max<u32>(s->ds.max_depth, 1);
     const u32 blocks = hero ? std::min<u32>(depth, 129) : 2 * std::min<u32>(depth, 127);
-    const u32 tables = hero ? 2 * blocks : blocks, first = hero ? 4 : 1;
+    const u32 tables = (hero ? 2 * blocks : blocks) + 1, first = hero ? 4 : 1;
     const size_t products = size_t(tables) * kIndexBytes * 256 * sizeof(uint4);
     const size_t prefixes = size_t(tables) * 4 * kOwenPrefixEntries * sizeof(unsigned short);
     if (s->draw_capacity < tables) {

@@ -37,11 +37,7 @@ RP_DEV void raygen_lane(const DeviceScene &s, const RasterCam &cam, const WavePa
         pool.index(slot) = make_uint4(u32(b.index), u32(b.index >> 32), 0, 0);
         pool.lambda(slot) = to_float4(lambda);
         pool.lambda_pdf(slot) = to_float4(pdf);
-        pool.beta(slot) = make_float4(1, 1, 1, 1);
         pool.radiance(slot) = make_float4(0, 0, 0, 0);
-        pool.dens_f(0, slot) = make_float4(.5f, .5f, .5f, .5f); // read before [1] is
-        pool.dens_e(0, slot) = make_int4(1, 1, 1, 1);
-        pool.eta_scale(slot) = make_float4(1, 1, 1, 1);
         pool.ray_o(0, slot) = make_float4(o.x, o.y, o.z, 0);
         pool.ray_d(0, slot) = make_float4(d.x, d.y, d.z, 0);
         pool.vertex(0, slot)[0] = make_float4(o.x, o.y, o.z, 0);
@@ -268,11 +264,13 @@ RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool
         const u64 index = (u64(index2.y) << 32) | index2.x;
         u32 cnt = event_index + 1; // vertices so far, the camera's included
         const V4 lambda = from_float4(pool.lambda(path));
-        V4 beta = from_float4(pool.beta(path));
-        Density density = load_density(pool.dens_f(in, path), pool.dens_e(in, path));
-        V4 eta_scale = v4(1);
-        if (event_index)
+        // at the first event the throughput, eta scale and density are the initial ones
+        V4 beta = v4(1), eta_scale = v4(1);
+        if (event_index) {
+            beta = from_float4(pool.beta(path));
             eta_scale = from_float4(pool.eta_scale(path));
+        }
+        Density density = event_density(pool, in, path, event_index);
         bool roulette = (flags & F_ROULETTE) != 0;
         u32 active_mask = flags & F_MASK;
         const float4 ro4 = pool.ray_o(in, path), rd4 = pool.ray_d(in, path);
@@ -510,7 +508,7 @@ RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool
                     latest.param = from_float4(vertex[2]);
                     latest.k = latest.kind == 1 ? from_float4(vertex[3]) : v4(0);
                     const float4 pre = pool.vertex(in ^ 1, path)[0]; // the vertex before it
-                    const Density previous_density = load_density(pool.dens_f(in ^ 1, path), pool.dens_e(in ^ 1, path));
+                    const Density previous_density = event_density(pool, in ^ 1, path, event_index - 1);
                     bool ok;
                     const V4 bsdf_pdf = represented_pdf<-1>(latest_bsdf(latest), latest.shading_normal, latest.position,
                                                         v3(pre.x, pre.y, pre.z), ctype == kEnvironment,
@@ -603,7 +601,7 @@ RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool
             store_density(density, f, e);
             pool.dens_f(in ^ 1, path) = f;
             pool.dens_e(in ^ 1, path) = e;
-            if (F == 2)
+            if (F == 2 || event_index == 0)
                 pool.eta_scale(path) = to_float4(eta_scale); // only transmission changes it
             pool.ray_o(in ^ 1, path) = make_float4(ro.x, ro.y, ro.z, 0);
             pool.ray_d(in ^ 1, path) = make_float4(rd.x, rd.y, rd.z, 0);
@@ -613,10 +611,9 @@ RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool
 }
 // shade_path of the paths in the bin of family F.
 // Adjoint: the path-replay adjoint hooks are compiled in (the plain forward kernel carries none
-// of their registers).  The minimum of 512 resident threads per SM caps registers at 128, so
-// four 128-thread blocks fit an SM; the escape kernel (F = 3) fits without spilling, the
-// other families spill about 500 bytes to L1 and still run a little faster than three blocks
-// at 168 registers (113.5 against 115.0 ms per 1080p 16-spp frame of the mixed scene).
+// of their registers).  512 resident threads per SM cap the registers at 128, which the plain
+// forms keep to without spilling (200 to 300 bytes a thread before the event's state was cut:
+// mixed scene 1080p, 16 spp 91.9 against 84.5 ms).
 // Img: the scene has image reflectance or an environment image (their code is compiled out of
 // the plain kernels).
 template <int F, int Block = 128, bool Adjoint = false, bool Img = true>
@@ -675,7 +672,7 @@ RP_DEV void nee_path(const DeviceScene &s, const WaveParams &p, const PathPool &
     V3 cwo, previous;
     V4 direct_beta;
     Density direct_density;
-    read_nee_request<F>(pool, in, path, ident.w, cp, cbsdf, cwo, previous, direct_beta, direct_density);
+    read_nee_request<F>(pool, in, event_index, path, ident.w, cp, cbsdf, cwo, previous, direct_beta, direct_density);
     u32 status = 0;
     // the light-sample draw: its first word selects the light; the next two, a point on an
     // area light, are drawn only when an area light was selected (the same words either way)
@@ -1161,14 +1158,18 @@ __global__ void k_count_failures(PathPool pool, u32 lanes) {
     }
 }
 // Every sample of a wave reduced per pixel in canonical (absolute sample, pixel) order.
-// The DrawTables of the draw blocks [first, first + blocks), then [133, ...), `tables` in all.
+// The DrawTables of the draw blocks [first, first + blocks), for the hero transport [133, 133 +
+// blocks), and block 0: `tables` in all.
+RP_DEV u32 draw_block_of(u32 slot, u32 first, u32 blocks, u32 tables) {
+    return slot == tables - 1 ? 0 : slot < blocks ? first + slot : 133 + (slot - blocks);
+}
 __global__ void k_draw_tables(SobolTables sobol, unsigned short *prefix, uint4 *bytes, u32 *hash, u32 first, u32 blocks,
                               u32 tables, u32 seed) {
     const u32 prefixes = tables * 4 * kOwenPrefixEntries, products = tables * kIndexBytes * 256;
     const u32 stride = gridDim.x * blockDim.x, begin = blockIdx.x * blockDim.x + threadIdx.x;
     for (u32 e = begin; e < prefixes; e += stride) {
         const u32 slot = e / (4 * kOwenPrefixEntries), k = (e / kOwenPrefixEntries) & 3u;
-        const u32 block = slot < blocks ? first + slot : 133 + (slot - blocks);
+        const u32 block = draw_block_of(slot, first, blocks, tables);
         const u32 h = sobol_dimension_hash(4 * block + k, seed);
         prefix[e] = (unsigned short)owen_prefix_rounds(e % kOwenPrefixEntries, h);
         if (e % kOwenPrefixEntries == 0)
@@ -1176,7 +1177,7 @@ __global__ void k_draw_tables(SobolTables sobol, unsigned short *prefix, uint4 *
     }
     for (u32 e = begin; e < products; e += stride) {
         const u32 slot = e / (kIndexBytes * 256), byte = (e >> 8) % kIndexBytes, value = e & 0xffu;
-        const u32 block = slot < blocks ? first + slot : 133 + (slot - blocks);
+        const u32 block = draw_block_of(slot, first, blocks, tables);
         u32 v[4] = {0, 0, 0, 0};
         for (u32 bit = 0; bit < 8 && 8 * byte + bit < kSobolMatrix; ++bit)
             if (value >> bit & 1u)

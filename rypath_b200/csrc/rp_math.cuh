@@ -180,6 +180,20 @@ struct DrawTable {
     const uint4 *bytes;           // [kIndexBytes][256]
     const u32 *hash;              // [4]
 };
+// The generator products of a block's four dimensions.
+RP_DEV uint4 sobol_products(const DrawTable &table, u64 index) {
+    const uint4 *e = table.bytes;
+    uint4 v = make_uint4(0, 0, 0, 0);
+#pragma unroll 1
+    for (u32 byte = 0; index && byte < kIndexBytes; ++byte, index >>= 8, e += 256) {
+        const uint4 w = __ldg(e + (u32(index) & 0xffu));
+        v.x ^= w.x;
+        v.y ^= w.y;
+        v.z ^= w.z;
+        v.w ^= w.w;
+    }
+    return v;
+}
 RP_DEV u32 word_of(const uint4 &v, int k) { return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w; }
 // mix_bits after its first step, whose shift by 31 of a 32-bit value only carries its top bit
 // into bit 0: constant over the rounds of a word, so sobol_words folds it into the hash.
@@ -203,14 +217,10 @@ RP_DEV void sobol_words(const SobolTables &t, u64 index, u32 dimension, u32 mode
     u32 v[N] = {}, h[N];
     const bool tabled = table.prefix != nullptr;
     if (tabled) {
-        const uint4 *e = table.bytes;
-#pragma unroll 1
-        for (u32 byte = 0; index && byte < kIndexBytes; ++byte, index >>= 8, e += 256) {
-            const uint4 w = __ldg(e + (u32(index) & 0xffu));
+        const uint4 w = sobol_products(table, index);
 #pragma unroll
-            for (int k = 0; k < N; ++k)
-                v[k] ^= word_of(w, dim[k]);
-        }
+        for (int k = 0; k < N; ++k)
+            v[k] = word_of(w, dim[k]);
 #pragma unroll
         for (int k = 0; k < N; ++k)
             h[k] = __ldg(table.hash + dim[k]);

@@ -105,8 +105,8 @@ struct WaveParams {
     u32 log_spp;        // ZSobol: log2 of the total sample budget
     u32 boundary_limit; // pass-through crossings allowed between two vertices
     // Sobol sampler with Owen randomisation: tables (DrawTable) of the draw blocks [draw_first,
-    // draw_first + draw_blocks) and, for the hero transport (draw_first 4), [133, 133 +
-    // draw_blocks); null: none
+    // draw_first + draw_blocks), for the hero transport (draw_first 4) [133, 133 + draw_blocks),
+    // and block 0, the camera's, in the last slot; null: none
     const unsigned short *owen_prefix;
     const uint4 *draw_bytes;
     const u32 *draw_hash;
@@ -117,7 +117,9 @@ RP_DEV DrawTable draw_table(const WaveParams &p, u32 block) {
     if (p.owen_prefix && p.randomization == 3) {
         u32 slot = block - p.draw_first;
         if (slot >= p.draw_blocks)
-            slot = p.draw_first == 4u && block - 133u < p.draw_blocks ? p.draw_blocks + block - 133u : ~0u;
+            slot = block == 0                                                 ? p.draw_blocks * (p.draw_first == 4u ? 2u : 1u)
+                   : p.draw_first == 4u && block - 133u < p.draw_blocks ? p.draw_blocks + block - 133u
+                                                                              : ~0u;
         if (slot != ~0u)
             return {p.owen_prefix + size_t(slot) * 4 * kOwenPrefixEntries, p.draw_bytes + size_t(slot) * kIndexBytes * 256,
                     p.draw_hash + 4 * slot};
@@ -240,9 +242,18 @@ RP_DEV BeginSample begin_sample_at(const DeviceScene &s, const WaveParams &p, u3
     if (p.sampler == 1) {
         const u64 sample = (u64(r.sample_high) << 32) | r.sample_low;
         r.index = sobol_index(s.sobol, p.m, r.pixel % p.width, r.pixel / p.width, sample);
-        r.words = make_uint4(sobol_word(s.sobol, r.index, 0, 0, 0), sobol_word(s.sobol, r.index, 1, 0, 0),
-                             sobol_word(s.sobol, r.index, 2, p.randomization, p.seed_low),
-                             sobol_word(s.sobol, r.index, 3, p.randomization, p.seed_low));
+        const DrawTable table = draw_table(p, 0);
+        if (table.prefix) {
+            u32 z[4], w[4];
+            sobol_words<-1, 2>(s.sobol, r.index, 0, p.randomization, p.seed_low, table, z);
+            sobol_words<-1, 3>(s.sobol, r.index, 0, p.randomization, p.seed_low, table, w);
+            const uint4 raw = sobol_products(table, r.index);
+            r.words = make_uint4(raw.x, raw.y, z[2], w[3]);
+        } else {
+            r.words = make_uint4(sobol_word(s.sobol, r.index, 0, 0, 0), sobol_word(s.sobol, r.index, 1, 0, 0),
+                                 sobol_word(s.sobol, r.index, 2, p.randomization, p.seed_low),
+                                 sobol_word(s.sobol, r.index, 3, p.randomization, p.seed_low));
+        }
     } else if (p.sampler == 2) {
         const u64 sample = (u64(r.sample_high) << 32) | r.sample_low;
         r.index = halton_index(p.width, p.height, r.pixel % p.width, r.pixel / p.width, sample);
@@ -694,9 +705,13 @@ RP_DEV void store_density(const Density &d, float4 &f, int4 &e) {
     e = make_int4(d.lane[0].exponent, d.lane[1].exponent, d.lane[2].exponent, d.lane[3].exponent);
 }
 
+// The density at the start of an event: at the first one the initial density, which is not stored.
+RP_DEV Density event_density(const PathPool &pool, int in, u32 path, u32 event_index) {
+    return event_index ? load_density(pool.dens_f(in, path), pool.dens_e(in, path)) : initial_density();
+}
 // The light-sample request of a path's event, a vertex of family F.
 template <int F>
-RP_DEV void read_nee_request(const PathPool &pool, int in, u32 path, u32 flags, SurfacePoint &cp, HeroBsdf &b, V3 &wo,
+RP_DEV void read_nee_request(const PathPool &pool, int in, u32 event_index, u32 path, u32 flags, SurfacePoint &cp, HeroBsdf &b, V3 &wo,
                              V3 &previous, V4 &beta, Density &density) {
     const float4 *vertex = pool.vertex(in ^ 1, path), *request = pool.request(path);
     const float4 pp = vertex[0], n = vertex[1], pa = vertex[2], g = request[0], e = request[1];
@@ -725,7 +740,7 @@ RP_DEV void read_nee_request(const PathPool &pool, int in, u32 path, u32 flags, 
     wo = -v3(w.x, w.y, w.z);
     previous = v3(v.x, v.y, v.z);
     beta = from_float4(request[2]);
-    density = load_density(pool.dens_f(in, path), pool.dens_e(in, path));
+    density = event_density(pool, in, path, event_index);
 }
 
 // shaders/packet_transport.h:77-83

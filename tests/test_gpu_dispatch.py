@@ -1,12 +1,15 @@
 """The forms of a kernel that a launch rule chooses between give identical lanes.
 
-Waves of few lanes run as whole paths, larger ones as the wavefront, compared bit for bit.
+Waves of few lanes run as whole paths, larger ones as the wavefront; rays of deep trees stream
+over a warp's lanes after the first event, except in counting runs; evenly spaced knots guess
+their segment, others are searched.  Each pair is compared bit for bit, or with the oracle.
 """
 
 import numpy as np
 import pytest
 
 from rypath_b200 import abi, renderer, scenes
+from tests.oracle_lib import OracleScene, request
 
 pytestmark = pytest.mark.gpu
 
@@ -46,4 +49,70 @@ def test_whole_paths_equal_the_wavefront(kind, limit, sampler):
         part = rs.sample(renderer.RenderRequest(257, 129, sampler=sampler, pixel_begin=begin, pixel_count=count))
         assert part.status == abi.RP_SUCCESS, part.diagnostic
         assert_same(part.packet_samples, whole.packet_samples[begin:begin + count])
+    rs.close()
+
+
+@pytest.mark.parametrize("width,height,spp", [(257, 129, 1), (200, 170, 3)])
+def test_streamed_walks_equal_a_ray_a_thread(width, height, spp):
+    rs = build(scenes.mixed_scene(width, height, spp, 16, subdivisions=5, sphere_count=8))
+    req = renderer.RenderRequest(width, height, sample_count=spp)
+    streamed = rs.sample(req)
+    assert streamed.status == abi.RP_SUCCESS, streamed.diagnostic
+    rs.set_counting(True)  # counting runs walk a ray a thread
+    counted = rs.sample(req)
+    rs.set_counting(False)
+    assert_same(streamed.packet_samples, counted.packet_samples)
+    rs.close()
+
+
+@pytest.mark.parametrize("spp", [4736, 4737])
+def test_scalar_waves_at_the_slot_count(spp):
+    # 64 lanes a sample: as many lanes as the slots of 148 SMs, then more, the last ones in slots
+    # that others left
+    rs = build(scenes.cornell_fog(8, 8, 1, 8))
+    whole = rs.sample_scalar(renderer.RenderRequest(8, 8, sample_count=spp)).samples
+    part = rs.sample_scalar(renderer.RenderRequest(8, 8, sample_begin=spp - 1, sample_count=1)).samples
+    assert whole.tobytes()[-part.nbytes:] == part.tobytes()
+    rs.close()
+
+
+def uneven(scene, kind):
+    """The scene with its sampled spectra on two knots, on uneven ones, or inside the visible range
+    (the values outside are zero, or the ends' for optical constants)."""
+    w = {"two": [360.0, 830.0], "uneven": [360.0, 365.0, 400.0, 612.5, 613.0, 830.0],
+         "inside": [420.0, 500.0, 580.0, 660.0]}[kind]
+    knots, ranges = [], {}
+    old = np.asarray(scene.knots)
+
+    def moved(begin, count):
+        if count < 2:
+            return begin, count
+        if begin not in ranges:
+            k = old[begin:begin + count]
+            ranges[begin] = sum(len(x) for x in knots)
+            knots.append(np.stack([np.float32(w), np.interp(w, k[:, 0], k[:, 1]).astype(np.float32)], 1))
+        return ranges[begin], len(w)
+
+    for m in scene.materials:
+        m.knot_begin, m.knot_count = moved(m.knot_begin, m.knot_count)
+        m.eta_begin, m.eta_count = moved(m.eta_begin, m.eta_count)
+        m.k_begin, m.k_count = moved(m.k_begin, m.k_count)
+    scene.knots = np.concatenate(knots).astype(np.float32)
+    return scene
+
+
+@pytest.mark.parametrize("kind", ["two", "uneven", "inside"])
+@pytest.mark.parametrize("transport", [abi.TRANSPORT_HERO, abi.TRANSPORT_SCALAR])
+def test_sampled_spectra_on_other_knots(kind, transport):
+    scene = uneven(scenes.cornell_microfacets(32, 32, 4, 8, transport=transport), kind)
+    rs, oracle, q = build(scene), OracleScene(scene), request(32, 32, 4)
+    if transport == abi.TRANSPORT_HERO:
+        got, ref = rs.sample(renderer.RenderRequest(32, 32, sample_count=4)).packet_samples, oracle.sample(q)
+    else:
+        got, ref = rs.sample_scalar(renderer.RenderRequest(32, 32, sample_count=4)).samples, oracle.sample_scalar(q)
+    np.testing.assert_array_equal(got["status"], ref["status"])
+    # the lane gate of the transports' parity tests: relative 1e-3 for at least 97% of the lanes
+    g, r = got["radiance"].reshape(len(got), -1), ref["radiance"].reshape(len(ref), -1)
+    close = np.all(np.abs(g - r) <= 1e-3 * np.maximum(np.abs(r), 1e-6) + 1e-7, axis=1)
+    assert close.mean() >= 0.97
     rs.close()
