@@ -1759,6 +1759,15 @@ template <class F> rp_status guarded(char *diag, size_t cap, F &&f) {
     }
 }
 
+// The status of a call whose lanes are on the host, from count_failed's words.
+template <class T> rp_status report_failed(const u32 (&failed)[2], const T *out, char *diag, size_t cap) {
+    if (!failed[1])
+        return RP_SUCCESS;
+    const u32 lane = ~failed[0];
+    set_diag(diag, cap, "Metal render sample failed with status %u at lane %u", out[lane].status, lane);
+    return RP_FAILURE;
+}
+
 // First half of the LBVH build, launched as soon as the triangles are on the device: the
 // build storage, then world-space triangles, their boxes, and the centroid and vertex bounds
 // (read back by build_bounds).  The light tables are built on the host meanwhile.
@@ -2589,10 +2598,12 @@ static rp_status sample_impl(rp_scene *s, const rp_request *request, rp_packet_r
             dst = staging;
         }
         s->mark(3);
-        k_results<<<grid_for(s->sm_count, p.lanes, 256, 16), 256, 0, s->stream>>>(s->pool, p.lanes, s->ds.filter_weight, dst);
+        k_results<<<grid_for(s->sm_count, p.lanes, 256, 16), 256, 0, s->stream>>>(s->pool, p.lanes, s->ds.filter_weight, dst,
+                                                                                 host ? s->pool.counters + kFailedLanes : nullptr);
         s->done();
-        u32 failures = 0;
+        u32 failed[2] = {0, 0};
         if (host) {
+            RP_CHECK(cudaMemcpyAsync(failed, s->pool.counters + kFailedLanes, sizeof(failed), cudaMemcpyDeviceToHost, s->stream));
             RP_CHECK(cudaMemcpyAsync(out, staging, size_t(p.lanes) * sizeof(PacketResult), cudaMemcpyDeviceToHost, s->stream));
             RP_CHECK(cudaFreeAsync(staging, s->stream));
         }
@@ -2616,15 +2627,7 @@ static rp_status sample_impl(rp_scene *s, const rp_request *request, rp_packet_r
             s->timing.shadow_nodes_visited = st[4];
             s->timing.shadow_triangles_tested = st[5];
         }
-        if (host) {
-            for (u32 i = 0; i < p.lanes; ++i)
-                if (out[i].status != RP_SAMPLE_SUCCESS) {
-                    if (!failures)
-                        set_diag(diag, cap, "Metal render sample failed with status %u at lane %u", out[i].status, i);
-                    ++failures;
-                }
-        }
-        return failures ? RP_FAILURE : RP_SUCCESS;
+        return report_failed(failed, out, diag, cap);
     });
 }
 
@@ -2666,8 +2669,10 @@ rp_status rp_cuda_sample_scalar(rp_scene *s, const rp_request *request, rp_scala
         RP_CHECK(cudaMallocAsync(reinterpret_cast<void **>(&staging), size_t(p.lanes) * sizeof(ScalarResult), s->stream));
         s->mark(3);
         k_scalar_results<<<grid_for(s->sm_count, p.lanes, 256, 16), 256, 0, s->stream>>>(s->ds, p, s->scalar_records,
-                                                                                          staging);
+                                                                                          staging, s->scalar_counters + 14);
         s->done();
+        u32 failed[2];
+        RP_CHECK(cudaMemcpyAsync(failed, s->scalar_counters + 14, sizeof(failed), cudaMemcpyDeviceToHost, s->stream));
         RP_CHECK(cudaMemcpyAsync(out, staging, size_t(p.lanes) * sizeof(ScalarResult), cudaMemcpyDeviceToHost,
                                  s->stream));
         RP_CHECK(cudaFreeAsync(staging, s->stream));
@@ -2689,14 +2694,7 @@ rp_status rp_cuda_sample_scalar(rp_scene *s, const rp_request *request, rp_scala
             s->timing.shadow_nodes_visited = st[4];
             s->timing.shadow_triangles_tested = st[5];
         }
-        u32 failures = 0;
-        for (u32 i = 0; i < p.lanes; ++i)
-            if (out[i].status != RP_SAMPLE_SUCCESS) {
-                if (!failures)
-                    set_diag(diag, cap, "Metal render sample failed with status %u at lane %u", out[i].status, i);
-                ++failures;
-            }
-        return failures ? RP_FAILURE : RP_SUCCESS;
+        return report_failed(failed, out, diag, cap);
     });
 }
 
@@ -4052,7 +4050,7 @@ rp_status rp_cuda_sample_device_static(rp_scene *s, const rp_request *request, r
             in ^= 1;
         }
         k_results<<<grid_for(sms, p.lanes, 256, 16), 256, 0, st>>>(pool, p.lanes, s->ds.filter_weight,
-                                                                   reinterpret_cast<PacketResult *>(device_results));
+                                                                   reinterpret_cast<PacketResult *>(device_results), nullptr);
         RP_CHECK(cudaGetLastError());
         return RP_SUCCESS;
     });

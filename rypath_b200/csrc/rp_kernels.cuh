@@ -1043,12 +1043,21 @@ struct PacketResult {
     float filter_weight;
     u32 reserved[2];
 };
-__global__ void k_results(PathPool pool, u32 lanes, float filter_weight, PacketResult *out) {
+// failed (null: not wanted; zero before): the complement of the first failed lane, [1] their
+// number, so that the host need not read every lane's status (0.4 ms of 20 MB of lanes).
+RP_DEV void count_failed(u32 *failed, u32 lane, u32 status) {
+    if (failed && status) {
+        atomicMax(failed, ~lane);
+        atomicAdd(failed + 1, 1u);
+    }
+}
+__global__ void k_results(PathPool pool, u32 lanes, float filter_weight, PacketResult *out, u32 *failed) {
     for (u32 lane = blockIdx.x * blockDim.x + threadIdx.x; lane < lanes; lane += gridDim.x * blockDim.x) {
         const uint4 id = pool.ident(lane);
         const float4 l = pool.lambda(lane), pdf = pool.lambda_pdf(lane), r = pool.radiance(lane);
         PacketResult res;
         res.status = (id.w & F_COMPLETE) ? get_status(id.w) : 2u;
+        count_failed(failed, lane, res.status);
         res.pixel = id.x;
         res.sample_low = id.y;
         res.sample_high = id.z;

@@ -64,7 +64,8 @@ struct PathPool {
     RP_DEV float4 *request(u32 path) const { return requests + 4 * size_t(path); }
     // queues
     u32 *queue[2];
-    u32 *counters; // [0] queue0, [1] queue1, [3] failures, then the two event sets
+    u32 *counters; // [0] queue0, [1] queue1, [3] failures, [4] [5] failed lanes of results (count_failed),
+                   // then the two event sets from [16] on
     u32 *bins;     // 4 family bins of bin_capacity path ids each
     u32 bin_capacity;
     float4 *sh_o;  // shadow origin, tmax
@@ -95,6 +96,7 @@ struct PathPool {
     // clears the other set; its closest-hit kernel clears the queue it will fill.
     RP_DEV u32 *event(int in) const { return counters + 16 + 16 * in; }
 };
+constexpr u32 kFailedLanes = 4;
 enum : u32 { kBinCount = 0, kNeeCount = 4, kShadowCount = 7, kTraceNext = 8, kShadowNext = 9, kEventCounters = 10 };
 
 // sampler: 0 independent, 1 Sobol, 2 Halton, 3 ZSobol (src/render_wire.h:41)

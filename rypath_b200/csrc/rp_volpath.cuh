@@ -941,7 +941,6 @@ RP_DEV int shade_begin(const DeviceScene &s, const WaveParams &p, const ScalarPa
             return kEventFinished;
     }
     const bool dirac = microfacet && bsdf.g.smooth; // delta_only (shaders/scattering.h:25-28)
-    const bool both_hemispheres = microfacet && bsdf.kind == 2;
     const V3 context_normal = microfacet ? frame.z : point.shading_normal;
     const bool directional_offset = authored_normals;
     const V3 area_reference = directional_offset ? point.position : spawn_origin(path.o, path.d, hit.t, point, n);
@@ -1551,12 +1550,13 @@ struct ScalarResult {
     u32 random_words[4];
 };
 __global__ void k_scalar_results(const __grid_constant__ DeviceScene s, const __grid_constant__ WaveParams p,
-                                 const uint4 *records, ScalarResult *out) {
+                                 const uint4 *records, ScalarResult *out, u32 *failed) {
     for (u32 lane = blockIdx.x * blockDim.x + threadIdx.x; lane < p.lanes; lane += gridDim.x * blockDim.x) {
         const BeginSample b = begin_sample(s, p, lane);
         const uint4 r = records[lane];
         ScalarResult o;
         o.status = r.x;
+        count_failed(failed, lane, r.x);
         o.pixel = b.pixel;
         o.sample_low = b.sample_low;
         o.sample_high = b.sample_high;

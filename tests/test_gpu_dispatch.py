@@ -116,3 +116,35 @@ def test_sampled_spectra_on_other_knots(kind, transport):
     close = np.all(np.abs(g - r) <= 1e-3 * np.maximum(np.abs(r), 1e-6) + 1e-7, axis=1)
     assert close.mean() >= 0.97
     rs.close()
+
+
+@pytest.mark.parametrize("transport", [abi.TRANSPORT_HERO, abi.TRANSPORT_SCALAR])
+@pytest.mark.parametrize("limit", [1, 4096])
+def test_failed_lanes_are_reported(transport, limit):
+    # two panes in a row: camera rays through both exceed a limit of one crossing
+    scene = scenes.cornell_pass_through(16, 16, 2, 8, invisible_light=False, mixes=False)
+    scene.transport = transport
+    second = scenes.identity_instance(scene.positions.shape[0], scene.triangles.shape[0], 2,
+                                      scene.instances[-1].material)
+    scene.positions = np.concatenate([scene.positions, scene.positions[-4:] + np.float32([0, 0, 0.1])])
+    scene.triangles = np.concatenate([scene.triangles, scene.triangles[-2:]])
+    scene.instances.append(second)
+    rs = build(scene)
+
+    def sample(**more):
+        req = renderer.RenderRequest(16, 16, sample_count=2, boundary_limit=limit, **more)
+        if transport == abi.TRANSPORT_HERO:
+            res = rs.sample(req)
+            return res, res.packet_samples
+        res = rs.sample_scalar(req)
+        return res, res.samples
+
+    res, lanes = sample()
+    failed = np.flatnonzero(lanes["status"])
+    assert (len(failed) > 0) == (limit == 1)
+    assert res.status == (abi.RP_FAILURE if len(failed) else abi.RP_SUCCESS)
+    if len(failed):
+        assert res.diagnostic.endswith(f"failed with status {lanes['status'][failed[0]]} at lane {failed[0]}")
+    refused, lanes = sample(pixel_begin=1, pixel_count=256)
+    assert refused.status == abi.RP_INVALID_ARGUMENT and not lanes.tobytes().strip(b"\0")
+    rs.close()
