@@ -1240,10 +1240,14 @@ RP_DEV uint4 scalar_record(const ScalarPath &path) {
 // event or connection step and hands finished slots the wave's next lanes.  Each lane's path
 // depends only on its own indices, so its record does not depend on the slot or trip that
 // ran it.
+//
+// paired: scenes without media, whose connection is one vacuum query.  The walk then takes a
+// slot's connection and, unless the path ends with it, the continuation's ray together, and the
+// step applies the connection before the continuation's event: one trip an event instead of two.
 struct ScalarSlots {
     ScalarPath *path;
     Connection *conn;
-    u32 *mode;      // kEvent* in the low byte; bit 8: the walk of this trip succeeded
+    u32 *mode;      // kEvent* in the low byte, kWalkOk, and of a paired connection kConnection*
     Hit *hit;       // the walk's hit
     u32 count;      // slots
     u32 *remaining; // lanes of the wave whose record is not written yet
@@ -1253,8 +1257,10 @@ struct ScalarSlots {
     u32 *queue_connect[2], *queue_medium[2], *queue_interface[2], *queue_path[2];
     u32 *qcount;
     u32 *next_slot; // [parity] the walk's next slot
+    bool paired;
 };
-constexpr u32 kWalkOk = 1u << 8;
+// the walk of this trip succeeded; the paired connection's did; it is occluded
+constexpr u32 kWalkOk = 1u << 8, kConnectionOk = 1u << 9, kConnectionHit = 1u << 10;
 
 RP_DEV bool scalar_ray_valid(const ScalarPath &path) {
     return finite3(path.o) && finite3(path.d) && isfinite(path.throughput) && isfinite(path.radiance);
@@ -1369,35 +1375,34 @@ __global__ void __launch_bounds__(kTraceBlock, walk_blocks(kTraceBlock, Stack, S
     for (u32 trip = 0; trip < trips; ++trip) {
         const u32 i = trip * stride + blockIdx.x * blockDim.x + threadIdx.x;
         u32 mode = kEventFinished;
-        bool scatter = false, interface = false;
+        bool scatter = false, interface = false, ends = false; // ends: the step runs a connection only
         if (i < w.count) {
             mode = w.mode[i] & 0xffu;
             if (mode != kEventFinished) {
-                V3 ro, rd;
-                float tmax;
-                bool walk = true;
                 const ScalarPath &path = w.path[i];
-                if (mode == kEventPath) {
-                    ro = path.o;
-                    rd = path.d;
-                    walk = scalar_ray_valid(path); // else the step kernel records the failure
-                    tmax = finf();
-                } else {
-                    const Connection &c = w.conn[i];
-                    ro = c.o;
-                    rd = c.d;
-                    tmax = c.remaining;
-                }
-                if (walk) {
+                const Connection &c = w.conn[i];
+                bool connection = mode == kEventConnect;
+                u32 state = mode;
+                ends = connection;
+                for (;;) { // the connection, the path's ray, or (paired) both in turn
+                    V3 ro, rd;
+                    float tmax;
+                    if (connection) {
+                        ro = c.o;
+                        rd = c.d;
+                        tmax = c.remaining;
+                    } else {
+                        if (!scalar_ray_valid(path)) // the step kernel records the failure
+                            break;
+                        ro = path.o;
+                        rd = path.d;
+                        tmax = finf();
+                    }
                     Hit hit;
                     u32 nodes = 0, tris = 0;
                     const bool ok =
                         walk_closest<Count, Stack, Proc>(s, ro, rd, tmax, hit, stack + threadIdx.x, kTraceBlock, nodes, tris);
-                    w.hit[i] = hit;
-                    w.mode[i] = mode | (ok ? kWalkOk : 0u);
-                    scatter = ok && mode == kEventPath && predicts_medium_scatter(s, p, path, hit);
-                    interface = ok && mode == kEventPath && !scatter && hits_interface(s, hit);
-                    if (Count && mode == kEventPath) {
+                    if (Count && !connection) {
                         counts[0] += nodes;
                         counts[1] += tris;
                         counts[2] += 1;
@@ -1406,13 +1411,31 @@ __global__ void __launch_bounds__(kTraceBlock, walk_blocks(kTraceBlock, Stack, S
                         counts[4] += nodes;
                         counts[5] += tris;
                     }
+                    if (connection && w.paired) {
+                        state |= (ok ? kConnectionOk : 0u) | (hit.prim != kNone ? kConnectionHit : 0u);
+                        if (!ok || c.after != kAfterContinue)
+                            break;
+                        connection = ends = false;
+                        continue;
+                    }
+                    w.hit[i] = hit;
+                    state |= ok ? kWalkOk : 0u;
+                    if (w.paired) { // escapes apart from surfaces
+                        interface = ok && hit.prim == kNone;
+                    } else {
+                        scatter = ok && mode == kEventPath && predicts_medium_scatter(s, p, path, hit);
+                        interface = ok && mode == kEventPath && !scatter && hits_interface(s, hit);
+                    }
+                    break;
                 }
+                w.mode[i] = state;
             }
         }
-        slot_append(w.queue_connect[parity], w.qcount + 4 * parity, mode == kEventConnect, i);
-        slot_append(w.queue_medium[parity], w.qcount + 4 * parity + 1, mode == kEventPath && scatter, i);
-        slot_append(w.queue_interface[parity], w.qcount + 4 * parity + 2, mode == kEventPath && interface, i);
-        slot_append(w.queue_path[parity], w.qcount + 4 * parity + 3, mode == kEventPath && !scatter && !interface, i);
+        const u32 kind = mode == kEventFinished ? 4u : ends ? 0u : scatter ? 1u : interface ? 2u : 3u;
+        slot_append(w.queue_connect[parity], w.qcount + 4 * parity, kind == 0, i);
+        slot_append(w.queue_medium[parity], w.qcount + 4 * parity + 1, kind == 1, i);
+        slot_append(w.queue_interface[parity], w.qcount + 4 * parity + 2, kind == 2, i);
+        slot_append(w.queue_path[parity], w.qcount + 4 * parity + 3, kind == 3, i);
     }
     if (Count) {
         atomicAdd(stats + 0, (unsigned long long)counts[0]);
@@ -1483,19 +1506,31 @@ __global__ void __launch_bounds__(kStepBlock, 512 / kStepBlock) k_scalar_step(co
             active = mode != kEventFinished;
             if (active) {
                 path = w.path[i];
-                if (mode == kEventConnect)
-                    c = w.conn[i];
+                bool event = mode == kEventPath;
                 if (s.instance_count == 0) {
+                    event = false;
                     if (scalar_sky_step(s, p, path))
                         mode = kEventFinished;
-                } else if (mode == kEventPath && !scalar_ray_valid(path)) {
-                    path.status = S_ARITHMETIC;
-                    mode = kEventFinished;
-                } else {
-                    hit = w.hit[i];
-                    const bool ok = (m & kWalkOk) != 0;
-                    mode = mode == kEventPath ? shade_begin<Full>(s, p, q, path, ok, hit, ev)
-                                              : connection_step(s, q, path, c, ok, hit);
+                } else if (mode == kEventConnect) {
+                    c = w.conn[i];
+                    bool ok = (m & kWalkOk) != 0;
+                    if (w.paired) {
+                        ok = (m & kConnectionOk) != 0;
+                        hit.prim = m & kConnectionHit ? 0u : kNone; // all that a vacuum query reads
+                    } else {
+                        hit = w.hit[i];
+                    }
+                    mode = connection_step(s, q, path, c, ok, hit);
+                    event = w.paired && mode == kEventPath;
+                }
+                if (event) {
+                    if (!scalar_ray_valid(path)) {
+                        path.status = S_ARITHMETIC;
+                        mode = kEventFinished;
+                    } else {
+                        hit = w.hit[i];
+                        mode = shade_begin<Full>(s, p, q, path, (m & kWalkOk) != 0, hit, ev);
+                    }
                 }
             }
         }

@@ -148,3 +148,16 @@ def test_failed_lanes_are_reported(transport, limit):
     refused, lanes = sample(pixel_begin=1, pixel_count=256)
     assert refused.status == abi.RP_INVALID_ARGUMENT and not lanes.tobytes().strip(b"\0")
     rs.close()
+
+
+@pytest.mark.parametrize("subdivisions", [1, 5])  # a tree whose scalar walks pair, one whose walks stream
+def test_scalar_walks_match_the_oracle(subdivisions):
+    scene = scenes.mixed_scene(32, 32, 4, 8, subdivisions=subdivisions, sphere_count=3)
+    scene.transport = abi.TRANSPORT_SCALAR
+    rs = build(scene)
+    got = rs.sample_scalar(renderer.RenderRequest(32, 32, sample_count=4)).samples
+    ref = OracleScene(scene).sample_scalar(request(32, 32, 4))
+    np.testing.assert_array_equal(got["status"], ref["status"])
+    close = np.abs(got["radiance"] - ref["radiance"]) <= 1e-3 * np.maximum(np.abs(ref["radiance"]), 1e-6) + 1e-7
+    assert close.mean() >= 0.97
+    rs.close()
