@@ -1366,7 +1366,9 @@ void launch_scalar_step(const rp_scene *s, unsigned grid, const WaveParams &p, c
 }
 
 // Whether walks of this scene's tree stream (rp_walk.cuh): where rays visit about six nodes or
-// more, so that what the longest of 32 waits for outweighs the streaming's own bookkeeping.
+// more, so that what the longest of 32 waits for outweighs the streaming's own bookkeeping: the
+// mixed scenes (7 to 11 nodes a ray) gain 2 to 3%; the fog box, of 38 triangles, lost 6 of 38 ms,
+// the demonstration scene, of 26, 2 of 10.
 bool use_stream(const rp_scene *s) { return s->wide_levels >= kStreamLevels; }
 // The closest-hit and shadow kernels with the traversal stack the built tree needs, resolving
 // pass-through and mix-root hits when the scene has them.  Stream: the streaming form.
@@ -1663,9 +1665,13 @@ constexpr u32 kScalarSlotsPerSm = 2048;
 constexpr int kScalarTripsPerCheck = 8;
 
 // Whether a scalar wave's walk takes a path's connection and its continuation together: without
-// media, where a connection is one query: demonstration scene 256x192, 128 spp 9.5 ms against 10.3
-// of two trips an event.  Streamed walks hold one ray a slot.
-bool pairs(const rp_scene *s) { return !s->ds.media_enabled && !(use_stream(s) && s->wide_levels <= u32(kShortStack)); }
+// media, where a connection is one query, which then ends at its first hit.  Demonstration scene
+// 256x192, 128 spp: 10.3 ms with two trips an event, 9.5 in one, 9.3 ending at the first hit.
+// Streamed walks hold one ray a slot; a tree deeper than any stack keeps the walk that reports it.
+bool pairs(const rp_scene *s) {
+    return !s->ds.media_enabled && s->wide_levels <= u32(kStackDepth) &&
+           !(use_stream(s) && s->wide_levels <= u32(kShortStack));
+}
 
 // One wave of the scalar transport, one record per lane in s->scalar_records: camera rays,
 // then walk / step trips over the slots until every lane's record is written.

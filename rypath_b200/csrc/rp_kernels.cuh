@@ -52,6 +52,9 @@ RP_DEV void raygen_lane(const DeviceScene &s, const RasterCam &cam, const WavePa
         }
     }
 }
+// Issue-bound by the draw words.  The first event uses constants for the initial throughput, eta
+// scale and density, which are not written: mixed scene 1080p, 16 spp 81.8 -> 80.3 ms, with the
+// camera's draw block from a table.
 __global__ void k_raygen(const __grid_constant__ DeviceScene s, const __grid_constant__ WaveParams p, PathPool pool) {
     const RasterCam cam{s.origin, s.forward, s.right, s.up};
     if (blockIdx.x == 0 && threadIdx.x == 0)
@@ -1044,7 +1047,7 @@ struct PacketResult {
     u32 reserved[2];
 };
 // failed (null: not wanted; zero before): the complement of the first failed lane, [1] their
-// number, so that the host need not read every lane's status (0.4 ms of 20 MB of lanes).
+// number, so that the host need not read every lane's status (1.3 ms of 20 MB of lanes).
 RP_DEV void count_failed(u32 *failed, u32 lane, u32 status) {
     if (failed && status) {
         atomicMax(failed, ~lane);

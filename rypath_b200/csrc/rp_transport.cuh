@@ -29,7 +29,8 @@ RP_DEV u32 set_status(u32 f, u32 s) { return (f & ~(7u << F_STATUS_SHIFT)) | (s 
 // Path pool: one slot per lane of the wave.  What a kernel reads or writes together lies
 // together in records of 32 or 64 bytes, whole 32-byte sectors: after the first event the bins
 // list their paths out of order, and sixteen bytes of one array at a time would fetch two
-// sectors for the bytes of one.
+// sectors for the bytes of one (textured box 640x480, 16 spp 13.7 -> 13.4 ms, mixed scene 84.5 ->
+// 83.9).
 struct PathPool {
     uint4 *ident_index; // 2: pixel, sample_low, sample_high, flags; Sobol index lo, hi
     float4 *spectrum;   // 2: lambda, lambda pdf

@@ -1401,7 +1401,8 @@ __global__ void __launch_bounds__(kTraceBlock, walk_blocks(kTraceBlock, Stack, S
                     Hit hit;
                     u32 nodes = 0, tris = 0;
                     const bool ok =
-                        walk_closest<Count, Stack, Proc>(s, ro, rd, tmax, hit, stack + threadIdx.x, kTraceBlock, nodes, tris);
+                        walk_closest<Count, Stack, Proc>(s, ro, rd, tmax, hit, stack + threadIdx.x, kTraceBlock, nodes,
+                                                         tris, connection && w.paired);
                     if (Count && !connection) {
                         counts[0] += nodes;
                         counts[1] += tris;
