@@ -9,8 +9,8 @@
 // until kLeafLanes lanes have some (or no lane can visit a node); results leave through
 // per-warp queues in shared memory that append 32 entries at a time.  A ray's hits do not
 // depend on any of this: the visits of one ray and its tests are those of walk_closest and
-// walk_any, in the same order.  Mixed scene 1080p, 16 spp: 9 of 32 lanes active an instruction
-// before, 17 so; 83.9 -> 81.6 ms.  Refill / leaf thresholds 4/8, 16/12, 8/14 and 14/14 were slower
+// walk_any, in the same order.  Mixed scene, event 1: 9.5 of 32 lanes active an instruction
+// before, 12.7 so; 1080p, 16 spp 83.9 -> 81.6 ms.  Refill / leaf thresholds 4/8, 16/12, 8/14 and 14/14 were slower
 // than 12/10.
 #pragma once
 
