@@ -232,18 +232,26 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_hist(const u64 *keys, u3
     __syncthreads();
     hist[threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
 }
-// exclusive scan of hist (digit-major) in one block
+// Exclusive scan of hist (digit-major; total is a multiple of 256) in one block: a chain of
+// barriers, bound by their latency, so each thread takes sixteen entries between two of them.
+// One entry a thread took 163 us for 180,224 entries (1.44M triangles), eight scans a build; a scene
+// of 458,754 triangles builds in 2.68 ms, 2.87 so.
+constexpr u32 kScanItems = 16;
 __global__ void __launch_bounds__(1024) k_radix_scan(u32 *hist, u32 total) {
     __shared__ u32 warp_sums[32];
-    __shared__ u32 carry;
-    if (threadIdx.x == 0)
-        carry = 0;
-    __syncthreads();
-    for (u32 base = 0; base < total; base += 1024) {
-        const u32 i = base + threadIdx.x;
-        const u32 v = i < total ? hist[i] : 0;
-        u32 x = v;
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    u32 carry = 0;
+    for (u32 base = 0; base < total; base += 1024 * kScanItems) {
+        const u32 i = base + kScanItems * threadIdx.x;
+        uint4 v[kScanItems / 4] = {};
+        u32 sum = 0;
+        if (i < total)
+#pragma unroll
+            for (u32 k = 0; k < kScanItems / 4; ++k) {
+                v[k] = reinterpret_cast<const uint4 *>(hist + i)[k];
+                sum += v[k].x + v[k].y + v[k].z + v[k].w;
+            }
+        u32 x = sum;
         for (int o = 1; o < 32; o <<= 1) {
             const u32 y = __shfl_up_sync(0xffffffffu, x, o);
             if (lane >= o)
@@ -262,13 +270,20 @@ __global__ void __launch_bounds__(1024) k_radix_scan(u32 *hist, u32 total) {
             warp_sums[lane] = w;
         }
         __syncthreads();
-        const u32 incl = x + (warp > 0 ? warp_sums[warp - 1] : 0) + carry;
+        u32 before = carry + (warp > 0 ? warp_sums[warp - 1] : 0) + x - sum;
+        carry += warp_sums[31];
         if (i < total)
-            hist[i] = incl - v;
-        __syncthreads();
-        if (threadIdx.x == 1023)
-            carry = incl;
-        __syncthreads();
+#pragma unroll
+            for (u32 k = 0; k < kScanItems / 4; ++k) {
+                uint4 e;
+                e.x = before;
+                e.y = e.x + v[k].x;
+                e.z = e.y + v[k].y;
+                e.w = e.z + v[k].z;
+                before = e.w + v[k].w;
+                reinterpret_cast<uint4 *>(hist + i)[k] = e;
+            }
+        __syncthreads(); // warp_sums is written again
     }
 }
 __global__ void __launch_bounds__(kSortThreads) k_radix_scatter(const u64 *kin, const u32 *vin, u64 *kout, u32 *vout,

@@ -9,7 +9,8 @@ import numpy as np
 import pytest
 
 from rypath_b200 import abi, renderer, scenes
-from tests.oracle_lib import OracleScene, request
+from tests.oracle_lib import OracleScene, oracle, request
+from tests.test_gpu_parity import _soup
 
 pytestmark = pytest.mark.gpu
 
@@ -105,11 +106,11 @@ def uneven(scene, kind):
 @pytest.mark.parametrize("transport", [abi.TRANSPORT_HERO, abi.TRANSPORT_SCALAR])
 def test_sampled_spectra_on_other_knots(kind, transport):
     scene = uneven(scenes.cornell_microfacets(32, 32, 4, 8, transport=transport), kind)
-    rs, oracle, q = build(scene), OracleScene(scene), request(32, 32, 4)
+    rs, ref_scene, q = build(scene), OracleScene(scene), request(32, 32, 4)
     if transport == abi.TRANSPORT_HERO:
-        got, ref = rs.sample(renderer.RenderRequest(32, 32, sample_count=4)).packet_samples, oracle.sample(q)
+        got, ref = rs.sample(renderer.RenderRequest(32, 32, sample_count=4)).packet_samples, ref_scene.sample(q)
     else:
-        got, ref = rs.sample_scalar(renderer.RenderRequest(32, 32, sample_count=4)).samples, oracle.sample_scalar(q)
+        got, ref = rs.sample_scalar(renderer.RenderRequest(32, 32, sample_count=4)).samples, ref_scene.sample_scalar(q)
     np.testing.assert_array_equal(got["status"], ref["status"])
     # the lane gate of the transports' parity tests: relative 1e-3 for at least 97% of the lanes
     g, r = got["radiance"].reshape(len(got), -1), ref["radiance"].reshape(len(ref), -1)
@@ -161,3 +162,16 @@ def test_scalar_walks_match_the_oracle(subdivisions):
     close = np.abs(got["radiance"] - ref["radiance"]) <= 1e-3 * np.maximum(np.abs(ref["radiance"]), 1e-6) + 1e-7
     assert close.mean() >= 0.97
     rs.close()
+
+
+@pytest.mark.parametrize("n", [2, 2049, 131072, 131073, 270001])  # tiles of 2,048, scan passes of 64 tiles
+def test_sorted_order_is_the_oracles(n):
+    scene = _soup(n, 9)
+    rs, oracle_scene = build(scene), OracleScene(scene)
+    nodes, order, keys, bounds = rs.export_bvh(n)
+    rs.close()
+    ref = [np.zeros((n - 1, 3), np.uint32), np.zeros(n, np.uint32), np.zeros(n, np.uint64),
+           np.zeros((2 * n - 1, 6), np.float32)]
+    assert oracle().or_export_bvh(oracle_scene.handle, *(a.ctypes.data for a in ref), n) == n
+    np.testing.assert_array_equal(keys, ref[2])
+    np.testing.assert_array_equal(order, ref[1])
