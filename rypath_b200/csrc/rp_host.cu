@@ -1088,6 +1088,11 @@ struct rp_scene {
     }
     void done_family(cudaStream_t on) { RP_CHECK(cudaEventRecord(family_events[2 * family_kind.size() - 1], on)); }
     void collect() {
+        // the recorded pairs end with this call, also when reading one fails
+        struct Discard {
+            rp_scene *s;
+            ~Discard() { s->discard_marks(); }
+        } discard{this};
         RP_CHECK(cudaStreamSynchronize(stream));
         double sums[4] = {0, 0, 0, 0};
         uint64_t counts[4] = {0, 0, 0, 0};
@@ -1104,7 +1109,6 @@ struct rp_scene {
             RP_CHECK(cudaEventElapsedTime(&ms, family_events[2 * i], family_events[2 * i + 1]));
             timing.shade_family_ms[family_kind[i]] += ms;
         }
-        family_kind.clear();
         timing.trace_launches = counts[0];
         timing.shadow_launches = counts[1];
         timing.shade_launches = counts[2];
@@ -1114,9 +1118,6 @@ struct rp_scene {
         timing.shade_ms = sums[2];
         timing.other_ms = sums[3];
         timing.kernel_launches = launches;
-        launches = 0;
-        event_kind.clear();
-        event_cursor = 0;
     }
 
     void ensure_scalar(u32 lanes) {
@@ -1425,29 +1426,31 @@ void launch_shadow(const rp_scene *s, const PathPool &pool, int in, unsigned gri
 constexpr int kShadeBlock = 256;
 template <int F, int Block, bool Adjoint, bool Img>
 void launch_family(rp_scene *s, const WaveParams &p, const PathPool &pool, int in, u32 event, unsigned grid, size_t smem,
-                   cudaStream_t st) {
-    // counting runs time each family kernel alone: all run one after another on the scene
-    // stream, so each one's events bracket its own work (side by side they share the SMs)
-    if (s->counting)
+                   cudaStream_t st, bool timed) {
+    if (timed)
         s->mark_family(F, st);
     k_shade<F, Block, Adjoint, Img><<<grid, Block, smem, st>>>(s->ds, p, pool, in, event);
     if constexpr (F != 3)
         k_nee<F, Block, Img><<<grid, Block, 0, st>>>(s->ds, p, pool, in, event);
-    if (s->counting)
+    if (timed)
         s->done_family(st);
 }
+// timed (counting runs): each family kernel is timed alone, so all run one after another on the
+// scene stream and each one's events bracket its own work (side by side they share the SMs).  A
+// batch never is: its launches may be captured, and events recorded in a capture have no time.
 template <int Block, bool Adjoint, bool Img>
-void launch_families(rp_scene *s, const WaveParams &p, const PathPool &pool, int in, u32 event, unsigned grid, size_t smem) {
+void launch_families(rp_scene *s, const WaveParams &p, const PathPool &pool, int in, u32 event, unsigned grid, size_t smem,
+                     bool timed) {
     const u32 mask = s->family_mask;
-    const bool fork = !s->counting && (mask & (mask - 1)) != 0;
+    const bool fork = !timed && (mask & (mask - 1)) != 0;
     if (!fork) {
-        launch_family<3, Block, Adjoint, Img>(s, p, pool, in, event, grid, smem, s->stream);
+        launch_family<3, Block, Adjoint, Img>(s, p, pool, in, event, grid, smem, s->stream, timed);
         if (mask & 1u)
-            launch_family<0, Block, Adjoint, Img>(s, p, pool, in, event, grid, smem, s->stream);
+            launch_family<0, Block, Adjoint, Img>(s, p, pool, in, event, grid, smem, s->stream, timed);
         if (mask & 2u)
-            launch_family<1, Block, Adjoint, Img>(s, p, pool, in, event, grid, smem, s->stream);
+            launch_family<1, Block, Adjoint, Img>(s, p, pool, in, event, grid, smem, s->stream, timed);
         if (mask & 4u)
-            launch_family<2, Block, Adjoint, Img>(s, p, pool, in, event, grid, smem, s->stream);
+            launch_family<2, Block, Adjoint, Img>(s, p, pool, in, event, grid, smem, s->stream, timed);
         return;
     }
     const bool used[3] = {(mask & 2u) != 0, (mask & 4u) != 0, true};
@@ -1456,12 +1459,12 @@ void launch_families(rp_scene *s, const WaveParams &p, const PathPool &pool, int
         if (used[k])
             RP_CHECK(cudaStreamWaitEvent(s->family[k], s->forked, 0));
     if (mask & 1u)
-        launch_family<0, Block, Adjoint, Img>(s, p, pool, in, event, grid, smem, s->stream);
+        launch_family<0, Block, Adjoint, Img>(s, p, pool, in, event, grid, smem, s->stream, timed);
     if (mask & 2u)
-        launch_family<1, Block, Adjoint, Img>(s, p, pool, in, event, grid, smem, s->family[0]);
+        launch_family<1, Block, Adjoint, Img>(s, p, pool, in, event, grid, smem, s->family[0], timed);
     if (mask & 4u)
-        launch_family<2, Block, Adjoint, Img>(s, p, pool, in, event, grid, smem, s->family[1]);
-    launch_family<3, Block, Adjoint, Img>(s, p, pool, in, event, grid, smem, s->family[2]);
+        launch_family<2, Block, Adjoint, Img>(s, p, pool, in, event, grid, smem, s->family[1], timed);
+    launch_family<3, Block, Adjoint, Img>(s, p, pool, in, event, grid, smem, s->family[2], timed);
     for (int k = 0; k < 3; ++k)
         if (used[k]) {
             RP_CHECK(cudaEventRecord(s->family_done[k], s->family[k]));
@@ -1471,11 +1474,12 @@ void launch_families(rp_scene *s, const WaveParams &p, const PathPool &pool, int
 u32 family_kernels(const rp_scene *s) { return 2 * u32(__builtin_popcount(s->family_mask)) + 1; }
 // The plain shade kernels for scenes without images.
 template <int Block, bool Adjoint>
-void launch_shade(rp_scene *s, const WaveParams &p, const PathPool &pool, int in, u32 event, unsigned grid, size_t smem) {
+void launch_shade(rp_scene *s, const WaveParams &p, const PathPool &pool, int in, u32 event, unsigned grid, size_t smem,
+                  bool timed) {
     if (!s->ds.img.textured && s->ds.img.env_image == kNone)
-        launch_families<Block, Adjoint, false>(s, p, pool, in, event, grid, smem);
+        launch_families<Block, Adjoint, false>(s, p, pool, in, event, grid, smem, timed);
     else
-        launch_families<Block, Adjoint, true>(s, p, pool, in, event, grid, smem);
+        launch_families<Block, Adjoint, true>(s, p, pool, in, event, grid, smem, timed);
 }
 
 // Sobol sampler with Owen randomisation: attaches the tables of the draw blocks of the scene's
@@ -1596,9 +1600,9 @@ void run_wave(rp_scene *s, const WaveParams &request_params, size_t adjoint_smem
         const size_t smem = adjoint_smem;
         const unsigned shade_grid = grid_for(sms, p.lanes, kShadeBlock, 2048 / kShadeBlock);
         if (pool.hist)
-            launch_shade<kShadeBlock, true>(s, p, pool, in, e, shade_grid, smem);
+            launch_shade<kShadeBlock, true>(s, p, pool, in, e, shade_grid, smem, s->counting);
         else
-            launch_shade<kShadeBlock, false>(s, p, pool, in, e, shade_grid, 0);
+            launch_shade<kShadeBlock, false>(s, p, pool, in, e, shade_grid, 0, s->counting);
         s->done();
         RP_CHECK(cudaEventRecord(s->forked, s->stream));
         RP_CHECK(cudaStreamWaitEvent(s->side, s->forked, 0));
@@ -3121,7 +3125,7 @@ void batch_wave_kernels(rp_scene *s, const WaveParams &p, const Batch &b, u32 wa
             RP_CHECK(cudaStreamWaitEvent(st, s->joined, 0));
             shadow_pending = false;
         }
-        launch_shade<SB, false>(s, p, pool, in, e, shade_grid, 0);
+        launch_shade<SB, false>(s, p, pool, in, e, shade_grid, 0, false);
         RP_CHECK(cudaEventRecord(s->forked, st));
         RP_CHECK(cudaStreamWaitEvent(s->side, s->forked, 0));
         launch_shadow<false, TB, false>(s, pool, in, trace_grid, 0, s->side, p.boundary_limit);

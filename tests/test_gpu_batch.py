@@ -112,3 +112,26 @@ def test_batch_validation():
     with pytest.raises(RuntimeError, match="trace block"):
         rs.render_views_device(views, renderer.BatchRequest(wave_lanes=1000, trace_block=96, shade_block=128,
                                                             blocks_per_sm=8), film.data_ptr())
+
+
+@pytest.mark.parametrize("use_graph", [1, 2])
+def test_a_batch_of_a_counting_scene_leaves_no_timing_behind(use_graph):
+    """Counting runs time each family's shade kernel; a batch, whose launches may be captured, does
+    not, and the calls after it work and report their own times."""
+    torch = pytest.importorskip("torch")
+    base, views = scenes.cornell_features("cauchy", 16, 16, 2), cornell_views()[1]
+    rs = build(base)
+    plains = per_view_plain(base, views)
+    req = renderer.RenderRequest(16, 16, sample_count=2)
+    before = rs.sample(req)
+    assert before.status == abi.RP_SUCCESS, before.diagnostic
+    rs.set_counting(True)
+    film, _ = batch_film(rs, views, renderer.BatchRequest(wave_lanes=4096, trace_block=128, shade_block=128,
+                                                          blocks_per_sm=8, use_graph=use_graph), torch)
+    rs.set_counting(False)
+    assert_same(film, plains, views)
+    after = rs.sample(req)
+    assert after.status == abi.RP_SUCCESS, after.diagnostic
+    assert after.packet_samples.tobytes() == before.packet_samples.tobytes()
+    assert list(rs.timing().shade_family_ms) == [0, 0, 0, 0]
+    rs.close()
