@@ -140,11 +140,20 @@ def pack_views(views):
     return offset
 
 
-def _written(status, diag, lanes):
-    """The lanes of a sample call: all written when it succeeds or reports a failed lane, else zeros.
+UNWRITTEN = 0xffffffff  # no lane's status
 
-    (Zeroed beforehand they cost 1 ms for 20 MB of lanes that the call then overwrites.)"""
-    if status != abi.RP_SUCCESS and not diag.value.startswith(b"Metal render sample failed"):
+
+def _lanes(count, dtype):
+    """Lanes for a sample call to write, the last one marked (see _written).  Zeroed beforehand they
+    cost 1 ms for 20 MB of lanes that the call then overwrites."""
+    lanes = np.empty(count, dtype)
+    lanes["status"][-1:] = UNWRITTEN
+    return lanes
+
+
+def _written(lanes):
+    """The lanes of a sample call, which writes all of them or none: zeros if none."""
+    if (lanes["status"][-1:] == UNWRITTEN).any():
         lanes.view(np.uint8)[:] = 0
     return lanes
 
@@ -170,19 +179,19 @@ class CudaRenderScene:
     def sample(self, request: RenderRequest) -> RenderSamplesResult:
         q = request.to_c()
         lanes = q.pixel_count * q.sample_count
-        out = np.empty(lanes, abi.packet_dtype())
+        out = _lanes(lanes, abi.packet_dtype())
         diag = C.create_string_buffer(512)
         st = native.lib().rp_cuda_sample(self._handle, C.byref(q), out.ctypes.data, lanes, diag, 512)
-        return RenderSamplesResult(st, diag.value.decode(errors="replace"), _written(st, diag, out))
+        return RenderSamplesResult(st, diag.value.decode(errors="replace"), _written(out))
 
     def sample_scalar(self, request: RenderRequest) -> RenderSamplesResult:
         """Scalar-transport lanes (``samples``): scenes built with ``transport=TRANSPORT_SCALAR``."""
         q = request.to_c()
         lanes = q.pixel_count * q.sample_count
-        out = np.empty(lanes, abi.scalar_dtype())
+        out = _lanes(lanes, abi.scalar_dtype())
         diag = C.create_string_buffer(512)
         st = native.lib().rp_cuda_sample_scalar(self._handle, C.byref(q), out.ctypes.data, lanes, diag, 512)
-        return RenderSamplesResult(st, diag.value.decode(errors="replace"), None, _written(st, diag, out))
+        return RenderSamplesResult(st, diag.value.decode(errors="replace"), None, _written(out))
 
     def sample_device(self, request: RenderRequest, device_ptr: int, capacity: int, stream: int = 0) -> int:
         q = request.to_c()
