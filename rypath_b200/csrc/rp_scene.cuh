@@ -1004,12 +1004,13 @@ RP_DEV bool any_leaf(const DeviceScene &s, const WalkRay &r, float tmax, u32 ind
 // above the child's box), and the ray reaches it at t = (p - o) / d + q s / d.  With u = 2^-24,
 // inv = 1 / d rounded, D = (p - o) inv rounded, b = 2^15 s inv (exact) and Q = 1 + 2^-15 q, the
 // float whose bits are 0x3f80qq00 (one byte permute), t' = Q b + (D - b) in rounded arithmetic
-// is within 5.1 u |D| + 1.1 u |b| of t; taking 8 u |D| + 4 u |b| off the offset D - b for the
-// near planes and adding it for the far ones (each another u (|D| + |b|)) bounds t on either
-// side, about 2^-7 of a quantization step wider than t' itself.  A direction component of zero
-// (or one whose reciprocal overflows) makes that axis's bounds NaN or infinite in the direction
-// that leaves the axis unconstrained; the NaN-ignoring min and max then skip it, which is
-// conservative.  The bounds' multiplications and additions run on the FMA pipe: the walk is
+// is within 5.1 u |D| + 1.1 u |b| of t.  Taking 12 u |D| + 4 u |D - b| off the offset D - b for
+// the near planes and adding it for the far ones (each another u (|D| + |b|)) bounds t on either
+// side, for |b| is at most |D| + |D - b|: about 2^-7 of a quantization step wider than t' itself.
+// Where a direction component is zero, or so small that its reciprocal, D, b or the offset
+// overflows, the margin is infinite or NaN with the offset, which leaves the axis's bounds NaN or
+// infinite in the direction that does not constrain it; the NaN-ignoring min and max then skip
+// it, which is conservative.  The bounds' multiplications and additions run on the FMA pipe: the walk is
 // bound by issue and by the ALU pipe, which the permutes, minima and maxima fill.  Mixed scene
 // 1080p, 16 spp 91.9 ms, against 96.9 with one directed-rounding FMA a plane and comparisons that
 // select; packed two-wide FMAs were slower (the walk 46 to 50 ms instead of 43).
@@ -1051,7 +1052,7 @@ RP_DEV void wide_children(const WNode *np, float4 origin, uint4 links, V3 o, con
         const float D = (p[a] - oo[a]) * w.inv[a];
         b[a] = (s * 32768.0f) * w.inv[a];
         const float offset = D - b[a];
-        const float margin = fmaf(fabsf(D), 0x1p-21f, fmaf(fabsf(b[a]), 0x1p-22f, kFltMin));
+        const float margin = fmaf(fabsf(D), 0x1.8p-21f, fmaf(fabsf(offset), 0x1p-22f, kFltMin));
         a_near[a] = offset - margin;
         a_far[a] = offset + margin;
         const uint2 near = __ldg(rows + (neg ? 3 + a : a)), far = __ldg(rows + (neg ? a : 3 + a));
