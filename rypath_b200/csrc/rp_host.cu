@@ -1369,8 +1369,9 @@ void launch_scalar_step(const rp_scene *s, unsigned grid, const WaveParams &p, c
 // Whether walks of this scene's tree stream (rp_walk.cuh): where rays visit about six nodes or
 // more, so that what the longest of 32 waits for outweighs the streaming's own bookkeeping: the
 // mixed scenes (7 to 11 nodes a ray) gain 2 to 3%; the fog box, of 38 triangles, lost 6 of 38 ms,
-// the demonstration scene, of 26, 2 of 10.
-bool use_stream(const rp_scene *s) { return s->wide_levels >= kStreamLevels; }
+// the demonstration scene, of 26, 2 of 10.  A tree deeper than any stack keeps the plain walks: a
+// query that runs out of entries has then tested the leaves of its last node, which may end it.
+bool use_stream(const rp_scene *s) { return s->wide_levels >= kStreamLevels && s->wide_levels <= u32(kStackDepth); }
 // The closest-hit and shadow kernels with the traversal stack the built tree needs, resolving
 // pass-through and mix-root hits when the scene has them.  Stream: the streaming form.
 template <bool Count, int Block, int Stack>
