@@ -1655,7 +1655,6 @@ ScalarSlots scalar_slots(rp_scene *s, u32 count) {
     w.count = count;
     w.remaining = s->scalar_counters + 2;
     w.qcount = s->scalar_counters + 4; // zeroed with the wave's counters
-    w.next_slot = s->scalar_counters + 12;
     w.paired = false;
     return w;
 }
@@ -1672,11 +1671,10 @@ constexpr int kScalarTripsPerCheck = 8;
 // Whether a scalar wave's walk takes a path's connection and its continuation together: without
 // media, where a connection is one query, which then ends at its first hit.  Demonstration scene
 // 256x192, 128 spp: 10.3 ms with two trips an event, 9.5 in one, 9.3 ending at the first hit.
-// Streamed walks hold one ray a slot; a tree deeper than any stack keeps the walk that reports it.
-bool pairs(const rp_scene *s) {
-    return !s->ds.media_enabled && s->wide_levels <= u32(kStackDepth) &&
-           !(use_stream(s) && s->wide_levels <= u32(kShortStack));
-}
+// Also in deep trees, where the hero walks stream instead (a ray a slot, two trips an event): mixed
+// scenes 512x384, 8 spp, pairing against streaming 8.0 / 12.5 ms with 53,250 triangles, 12.7 / 18.2
+// with 458,754; neither, 10.1 / 14.3.  A tree deeper than any stack keeps the walk that reports it.
+bool pairs(const rp_scene *s) { return !s->ds.media_enabled && s->wide_levels <= u32(kStackDepth); }
 
 // One wave of the scalar transport, one record per lane in s->scalar_records: camera rays,
 // then walk / step trips over the slots until every lane's record is written.
@@ -1739,8 +1737,6 @@ void run_scalar_wave(rp_scene *s, const WaveParams &request_params, u32 boundary
                 k_scalar_walk<true, kShortStack><<<walk_grid, kTraceBlock, 0, s->stream>>>(s->ds, p, w, parity, s->stats);
             else if (s->counting)
                 k_scalar_walk<true, kStackDepth><<<walk_grid, kTraceBlock, 0, s->stream>>>(s->ds, p, w, parity, s->stats);
-            else if (short_stack && use_stream(s))
-                k_scalar_walk<false, kShortStack, false, true><<<walk_grid, kTraceBlock, 0, s->stream>>>(s->ds, p, w, parity, s->stats);
             else if (short_stack)
                 k_scalar_walk<false, kShortStack><<<walk_grid, kTraceBlock, 0, s->stream>>>(s->ds, p, w, parity, s->stats);
             else

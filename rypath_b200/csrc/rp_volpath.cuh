@@ -1256,7 +1256,6 @@ struct ScalarSlots {
     // at a null interface, other path events, counted in qcount[4 parity + 0 / 1 / 2 / 3]
     u32 *queue_connect[2], *queue_medium[2], *queue_interface[2], *queue_path[2];
     u32 *qcount;
-    u32 *next_slot; // [parity] the walk's next slot
     bool paired;
 };
 // the walk of this trip succeeded; the paired connection's did; it is occluded
@@ -1303,72 +1302,12 @@ RP_DEV void slot_append(u32 *queue, u32 *count, bool want, u32 slot) {
         queue[base + __popc(ballot & ((1u << lane) - 1))] = slot;
 }
 
-// The walk of every active slot: its path's ray, or the leg of its connection in flight.
-struct ScalarRays {
-    const DeviceScene &s;
-    const WaveParams &p;
-    const ScalarSlots &w;
-    int parity;
-    StagedAppend queues;
-    u32 slot, mode;
-
-    template <class W> RP_DEV bool load(u32 i, W &walk) {
-        slot = i;
-        mode = w.mode[i] & 0xffu;
-        if (mode == kEventFinished)
-            return false;
-        if (mode == kEventPath) {
-            const ScalarPath &path = w.path[i];
-            if (scalar_ray_valid(path)) {
-                walk.start(s, path.o, path.d, finf());
-            } else { // not walked: the step kernel records the failure
-                walk.skip();
-                walk.ok = false;
-            }
-        } else {
-            const Connection &c = w.conn[i];
-            walk.start(s, c.o, c.d, c.remaining);
-        }
-        return true;
-    }
-    template <class W> RP_DEV void finish(bool done, const W &walk) {
-        bool scatter = false, interface = false;
-        if (done) {
-            w.hit[slot] = walk.h;
-            w.mode[slot] = mode | (walk.ok ? kWalkOk : 0u);
-            if (walk.ok && mode == kEventPath) {
-                const ScalarPath &path = w.path[slot];
-                scatter = predicts_medium_scatter(s, p, path, walk.h);
-                interface = !scatter && hits_interface(s, walk.h);
-            }
-        }
-        const u32 q = !done ? 4u : mode == kEventConnect ? 0u : scatter ? 1u : interface ? 2u : 3u;
-        queues.push(0, q == 0, slot, w.qcount + 4 * parity, w.queue_connect[parity]);
-        queues.push(1, q == 1, slot, w.qcount + 4 * parity + 1, w.queue_medium[parity]);
-        queues.push(2, q == 2, slot, w.qcount + 4 * parity + 2, w.queue_interface[parity]);
-        queues.push(3, q == 3, slot, w.qcount + 4 * parity + 3, w.queue_path[parity]);
-    }
-    RP_DEV void flush() {
-        queues.flush(0, w.qcount + 4 * parity, w.queue_connect[parity]);
-        queues.flush(1, w.qcount + 4 * parity + 1, w.queue_medium[parity]);
-        queues.flush(2, w.qcount + 4 * parity + 2, w.queue_interface[parity]);
-        queues.flush(3, w.qcount + 4 * parity + 3, w.queue_path[parity]);
-    }
-};
-
 // Proc: the scene has procedural primitives.
-template <bool Count, int Stack = kStackDepth, bool Proc = false, bool Stream = false>
-__global__ void __launch_bounds__(kTraceBlock, walk_blocks(kTraceBlock, Stack, Stream))
-    k_scalar_walk(const __grid_constant__ DeviceScene s, const __grid_constant__ WaveParams p, ScalarSlots w,
-                  int parity, unsigned long long *stats) {
+template <bool Count, int Stack = kStackDepth, bool Proc = false>
+__global__ void __launch_bounds__(kTraceBlock, walk_blocks(kTraceBlock, Stack, false))
+    k_scalar_walk(const __grid_constant__ DeviceScene s, const __grid_constant__ WaveParams p,
+                  const __grid_constant__ ScalarSlots w, int parity, unsigned long long *stats) {
     __shared__ uint2 stack[Stack * kTraceBlock];
-    if constexpr (Stream) {
-        static_assert(!Count);
-        __shared__ u32 stage[kTraceBlock / 32 * 4 * kStageEntries];
-        ScalarRays io{s, p, w, parity, {stage + (threadIdx.x >> 5) * 4 * kStageEntries, 0}, 0, 0};
-        walk_stream<Walker<false, Stack, Proc>>(s, w.count, w.next_slot + parity, stack + threadIdx.x, kTraceBlock, io);
-        return;
-    }
     u32 counts[6] = {0, 0, 0, 0, 0, 0};
     const u32 stride = gridDim.x * blockDim.x;
     const u32 trips = (w.count + stride - 1) / stride;
@@ -1466,7 +1405,7 @@ constexpr int kStepBlock = 256;
 template <bool Full>
 __global__ void __launch_bounds__(kStepBlock, 512 / kStepBlock) k_scalar_step(const __grid_constant__ DeviceScene s,
                                                              const __grid_constant__ WaveParams p, ScalarParams q,
-                                                             ScalarSlots w, int parity) {
+                                                             const __grid_constant__ ScalarSlots w, int parity) {
     const int lane_in_warp = threadIdx.x & 31;
     u32 n_connect = 0, n_medium = 0, n_interface = 0, total = w.count;
     if (parity >= 0) {
@@ -1476,8 +1415,6 @@ __global__ void __launch_bounds__(kStepBlock, 512 / kStepBlock) k_scalar_step(co
         total = n_interface + w.qcount[4 * parity + 3];
         if (blockIdx.x == 0 && threadIdx.x < 4)
             w.qcount[4 * (parity ^ 1) + threadIdx.x] = 0; // the next trip's walk appends there
-        if (blockIdx.x == 0 && threadIdx.x == 0)
-            w.next_slot[parity ^ 1] = 0;
     }
     const u32 stride = gridDim.x * blockDim.x;
     const u32 trips = (total + stride - 1) / stride;

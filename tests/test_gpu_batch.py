@@ -135,3 +135,26 @@ def test_a_batch_of_a_counting_scene_leaves_no_timing_behind(use_graph):
     assert after.packet_samples.tobytes() == before.packet_samples.tobytes()
     assert list(rs.timing().shade_family_ms) == [0, 0, 0, 0]
     rs.close()
+
+
+@pytest.mark.parametrize("kind,kernels", [("point", 5), ("cauchy", 9)])  # an event's: one BSDF family, three
+def test_a_batch_reports_its_launches(kind, kernels):
+    """Per wave the camera rays, the film and the step to the next wave, and per event two walks, the
+    escapes and each family's shading and light samples; a later call reports its own only."""
+    torch = pytest.importorskip("torch")
+    base, views = scenes.cornell_features(kind, 16, 16, 2, 8), cornell_views()[1]
+    rs = build(base)
+    lanes = sum(v.width * v.height * v.sample_count for v in views)
+    request = renderer.BatchRequest(wave_lanes=1000, trace_block=128, shade_block=128, blocks_per_sm=8)
+    req = renderer.RenderRequest(16, 16, sample_count=2)
+    assert rs.sample(req).status == abi.RP_SUCCESS
+    assert rs.sample(req).status == abi.RP_SUCCESS
+    plain = rs.timing().kernel_launches
+    for seed, tables in ((1, 0), (7, 1)):  # the draw tables are built once a seed
+        request.seed = seed
+        batch_film(rs, views, request, torch)
+        assert rs.timing().kernel_launches == tables + -(-lanes // 1000) * (3 + kernels * 9)
+    req.seed = 7
+    assert rs.sample(req).status == abi.RP_SUCCESS
+    assert rs.timing().kernel_launches == plain
+    rs.close()

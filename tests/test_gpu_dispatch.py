@@ -175,3 +175,16 @@ def test_sorted_order_is_the_oracles(n):
     assert oracle().or_export_bvh(oracle_scene.handle, *(a.ctypes.data for a in ref), n) == n
     np.testing.assert_array_equal(keys, ref[2])
     np.testing.assert_array_equal(order, ref[1])
+
+
+@pytest.mark.parametrize("subdivisions", [1, 3, 5])
+def test_scalar_walks_of_deep_trees_take_one_trip_an_event(subdivisions):
+    # without media a walk takes a path's connection together with its next ray: at most depth + 2
+    # trips of a walk and a step, in eights, beside the camera rays, the slots' two kernels, the draw
+    # tables and the lanes
+    scene = scenes.mixed_scene(128, 128, 1, 6, subdivisions=subdivisions, sphere_count=8)
+    scene.transport = abi.TRANSPORT_SCALAR
+    rs = build(scene)
+    assert rs.sample_scalar(renderer.RenderRequest(128, 128)).status == abi.RP_SUCCESS
+    assert rs.timing().kernel_launches <= 2 * 8 + 5
+    rs.close()
