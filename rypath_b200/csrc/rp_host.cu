@@ -3390,7 +3390,11 @@ rp_status rp_cuda_render_views_device(rp_scene *s, const rp_view *views, uint32_
         s->timing.build_bvh_ms = build.build_bvh_ms;
         s->timing.total_ms = ms;
         s->timing.samples = plan.lanes;
-        s->timing.kernel_launches = uint64_t(plan.waves.size()) * (3 + 6 * (s->ds.max_depth + 1));
+        // camera rays, film and the step to the next wave; two walks and the shade kernels an event;
+        // draw tables, if they were built
+        s->timing.kernel_launches =
+            uint64_t(plan.waves.size()) * (3 + uint64_t(2 + family_kernels(s)) * (s->ds.max_depth + 1)) + s->launches;
+        s->discard_marks();
         if (used)
             *used = c;
         if (failures) {
