@@ -259,26 +259,35 @@ template <int F, bool Adjoint, bool Img, bool Sync>
 RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool &pool, int in, u32 event_index,
                        bool active, u32 path, float *sgrad, bool &keep, bool &nee) {
     const u32 capacity = s.max_depth + 2;
-    uint4 ident = pool.ident(path);
+    uint4 ident = make_uint4(0, 0, 0, 0);
+    if (active)
+        ident = pool.ident(path);
     u32 flags = ident.w;
     active = active && !(flags & F_COMPLETE);
     {
-        const uint4 index2 = pool.index(path);
-        const u64 index = (u64(index2.y) << 32) | index2.x;
         u32 cnt = event_index + 1; // vertices so far, the camera's included
-        const V4 lambda = from_float4(pool.lambda(path));
         // at the first event the throughput, eta scale and density are the initial ones
-        V4 beta = v4(1), eta_scale = v4(1);
-        if (event_index) {
-            beta = from_float4(pool.beta(path));
-            eta_scale = from_float4(pool.eta_scale(path));
+        V4 lambda = v4(0), beta = v4(1), eta_scale = v4(1);
+        Density density = initial_density();
+        u64 index = 0;
+        V3 ro = v3(0, 0, 0), rd = v3(0, 0, 0);
+        float4 hit = make_float4(0, 0, 0, 0);
+        if (active) { // a thread without a path has no record to read: another's is written meanwhile
+            const uint4 index2 = pool.index(path);
+            index = (u64(index2.y) << 32) | index2.x;
+            lambda = from_float4(pool.lambda(path));
+            if (event_index) {
+                beta = from_float4(pool.beta(path));
+                eta_scale = from_float4(pool.eta_scale(path));
+                density = event_density(pool, in, path, event_index);
+            }
+            const float4 ro4 = pool.ray_o(in, path), rd4 = pool.ray_d(in, path);
+            ro = v3(ro4.x, ro4.y, ro4.z);
+            rd = v3(rd4.x, rd4.y, rd4.z);
+            hit = pool.hit(path);
         }
-        Density density = event_density(pool, in, path, event_index);
         bool roulette = (flags & F_ROULETTE) != 0;
         u32 active_mask = flags & F_MASK;
-        const float4 ro4 = pool.ray_o(in, path), rd4 = pool.ray_d(in, path);
-        V3 ro = v3(ro4.x, ro4.y, ro4.z), rd = v3(rd4.x, rd4.y, rd4.z);
-        const float4 hit = pool.hit(path);
         u32 status = get_status(flags);
         const Density direct_density = density;
         V4 direct_beta = beta;
@@ -666,16 +675,21 @@ __global__ void __launch_bounds__(Block, 512 / Block) k_shade(const __grid_const
 template <int F, bool Img, bool Sync>
 RP_DEV void nee_path(const DeviceScene &s, const WaveParams &p, const PathPool &pool, int in, u32 event_index, bool active,
                      u32 path, bool &shadow, float4 &sh_o, float4 &sh_d, float4 &sh_c, float4 &sh_t) {
-    uint4 ident = pool.ident(path);
-    const uint4 index2 = pool.index(path);
-    const u64 index = (u64(index2.y) << 32) | index2.x;
-    const V4 lambda = from_float4(pool.lambda(path));
+    uint4 ident;
+    u64 index;
+    V4 lambda;
     SurfacePoint cp;
     HeroBsdf cbsdf;
     V3 cwo, previous;
     V4 direct_beta;
     Density direct_density;
-    read_nee_request<F>(pool, in, event_index, path, ident.w, cp, cbsdf, cwo, previous, direct_beta, direct_density);
+    if (active) { // a thread without a path has no record to read: another's is written meanwhile
+        ident = pool.ident(path);
+        const uint4 index2 = pool.index(path);
+        index = (u64(index2.y) << 32) | index2.x;
+        lambda = from_float4(pool.lambda(path));
+        read_nee_request<F>(pool, in, event_index, path, ident.w, cp, cbsdf, cwo, previous, direct_beta, direct_density);
+    }
     u32 status = 0;
     // the light-sample draw: its first word selects the light; the next two, a point on an
     // area light, are drawn only when an area light was selected (the same words either way)
