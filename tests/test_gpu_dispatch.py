@@ -188,3 +188,33 @@ def test_scalar_walks_of_deep_trees_take_one_trip_an_event(subdivisions):
     assert rs.sample_scalar(renderer.RenderRequest(128, 128)).status == abi.RP_SUCCESS
     assert rs.timing().kernel_launches <= 2 * 8 + 5
     rs.close()
+
+
+@pytest.mark.parametrize("kind,limit", [("point", 18432), ("texture", 18432), ("cauchy", 4608), ("mixed", 8704)])
+def test_the_form_that_a_wave_takes(kind, limit):
+    # the pairs compared above are of two forms: whole paths launch no closest-hit kernel of their own
+    rs = build(small_scene(kind, 257, 129))
+    for count, wavefront in ((1, False), (limit, False), (limit + 1, True), (257 * 129, True)):
+        assert rs.sample(renderer.RenderRequest(257, 129, pixel_count=count)).status == abi.RP_SUCCESS
+        assert (rs.timing().trace_launches > 0) == wavefront
+    rs.close()
+
+
+@pytest.mark.parametrize("kind", ["fog", "shallow", "deep"])
+def test_scalar_lanes_in_refilled_slots(kind):
+    # more lanes than the wave's slots (2,048 an SM): every lane once, as in waves that fill them once
+    torch = pytest.importorskip("torch")
+    slots = 2048 * torch.cuda.get_device_properties(0).multi_processor_count
+    if kind == "fog":
+        scene = scenes.cornell_fog(64, 64, 1, 8)
+    else:
+        scene = scenes.mixed_scene(64, 64, 1, 8, subdivisions=1 if kind == "shallow" else 5, sphere_count=4)
+        scene.transport = abi.TRANSPORT_SCALAR
+    rs = build(scene)
+    for spp in (slots // 4096, slots // 4096 + 1, slots // 4096 + 17):
+        whole = rs.sample_scalar(renderer.RenderRequest(64, 64, sample_count=spp)).samples
+        half = spp // 2
+        parts = [rs.sample_scalar(renderer.RenderRequest(64, 64, sample_begin=b, sample_count=n)).samples
+                 for b, n in ((0, half), (half, spp - half))]
+        assert whole.tobytes() == np.concatenate(parts).tobytes()
+    rs.close()
