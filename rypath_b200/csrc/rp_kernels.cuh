@@ -30,7 +30,7 @@ RP_DEV void raygen_lane(const DeviceScene &s, const RasterCam &cam, const WavePa
         sample_wavelengths(sample_uniform(p, b.words.z), s.hero_mode, lambda, pdf);
         V3 o, d;
         primary_ray_from(s, cam, p, b, o, d);
-        u32 flags = 15u | F_ROULETTE | (kCamera << F_LTYPE_SHIFT);
+        u32 flags = 15u | F_ROULETTE;
         if (!finite3(o) || !finite3(d))
             flags = set_status(flags, 2) | F_COMPLETE;
         pool.ident(slot) = make_uint4(b.pixel, b.sample_low, b.sample_high, flags);
@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(Block, walk_blocks(Block, Stack, Stream))
         static_assert(!Count && !Resolve);
         __shared__ u32 stage[Block / 32 * 4 * kStageEntries];
         TraceRays io{s, pool, pool.queue[in], in, event, {stage + (threadIdx.x >> 5) * 4 * kStageEntries, 0}, 0};
-        walk_stream<Walker<false, Stack, false>>(s, count, event + kTraceNext, stack + threadIdx.x, Block, io);
+        walk_stream<Walker<false, Stack>>(s, count, event + kTraceNext, stack + threadIdx.x, Block, io);
         return;
     }
     const u32 *queue = pool.queue[in];
@@ -467,7 +467,6 @@ RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool
         // latest vertex (the previous event's) for MIS; what only a weighted emission reads of
         // it is loaded there
         Latest latest;
-        latest.type = (flags >> F_LTYPE_SHIFT) & 3u;
         latest.kind = (flags >> F_LKIND_SHIFT) & 3u;
         latest.mask = (flags >> F_LMASK_SHIFT) & 15u;
         latest.delta = (flags & F_LDELTA) != 0;
@@ -589,7 +588,6 @@ RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool
         // rest of its state is not written back.
         if (cnt != old_count) {
             // preceding = latest; latest = current (shaders/packet_pt_event_body.inc:453-460)
-            flags = (flags & ~(3u << F_PTYPE_SHIFT)) | (latest.type << F_PTYPE_SHIFT);
             if (!complete || nee) {
                 float4 *vertex = pool.vertex(in ^ 1, path);
                 vertex[0] = make_float4(cp.position.x, cp.position.y, cp.position.z, cbsdf.g.alpha_x);
@@ -598,8 +596,8 @@ RP_DEV void shade_path(const DeviceScene &s, const WaveParams &p, const PathPool
                 if (F == 1)
                     vertex[3] = make_float4(cbsdf.k[0], cbsdf.k[1], cbsdf.k[2], cbsdf.k[3]);
             }
-            flags &= ~((3u << F_LTYPE_SHIFT) | F_LDELTA | (3u << F_LKIND_SHIFT) | (15u << F_LMASK_SHIFT) | F_LSMOOTH);
-            flags |= (ctype << F_LTYPE_SHIFT) | (cdelta ? F_LDELTA : 0u) | ((cbsdf.kind & 3u) << F_LKIND_SHIFT) |
+            flags &= ~(F_LDELTA | (3u << F_LKIND_SHIFT) | (15u << F_LMASK_SHIFT) | F_LSMOOTH);
+            flags |= (cdelta ? F_LDELTA : 0u) | ((cbsdf.kind & 3u) << F_LKIND_SHIFT) |
                      ((cbsdf.active_mask & 15u) << F_LMASK_SHIFT) | (cbsdf.g.smooth ? F_LSMOOTH : 0u);
         }
         flags = (flags & ~(F_MASK | F_ROULETTE)) | active_mask | (roulette ? F_ROULETTE : 0u);
@@ -929,10 +927,9 @@ RP_DEV void shadow_result(const DeviceScene &s, const PathPool &pool, float *sgr
                            pool.adj_w[path]);
     }
 }
-template <bool Adjoint> struct ShadowRays {
+struct ShadowRays {
     const DeviceScene &s;
     const PathPool &pool;
-    float *sgrad;
     u32 entry;
 
     template <class W> RP_DEV bool load(u32 i, W &w) {
@@ -945,7 +942,7 @@ template <bool Adjoint> struct ShadowRays {
         if (!done)
             return;
         const u32 path = __float_as_uint(pool.sh_d[entry].w);
-        shadow_result<Adjoint>(s, pool, sgrad, pool.sh_c[entry], path, w.ok ? 0u : 3u, w.h.prim != kNone);
+        shadow_result<false>(s, pool, nullptr, pool.sh_c[entry], path, w.ok ? 0u : 3u, w.h.prim != kNone);
     }
     RP_DEV void flush() {}
 };
@@ -963,9 +960,9 @@ __global__ void __launch_bounds__(Block, walk_blocks(Block, Stack, Stream))
     const u32 count = event[kShadowCount];
     u32 nodes = 0, tris = 0, rays = 0;
     if constexpr (Stream) {
-        static_assert(!Count && !Resolve);
-        ShadowRays<Adjoint> io{s, pool, sgrad, 0};
-        walk_stream<Walker<true, Stack, false>>(s, count, event + kShadowNext, stack + threadIdx.x, Block, io);
+        static_assert(!Count && !Resolve && !Adjoint);
+        ShadowRays io{s, pool, 0};
+        walk_stream<Walker<true, Stack>>(s, count, event + kShadowNext, stack + threadIdx.x, Block, io);
     } else {
         for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
             const float4 o = pool.sh_o[i], d = pool.sh_d[i];
@@ -1183,7 +1180,6 @@ __global__ void k_count_failures(PathPool pool, u32 lanes) {
             atomicAdd(pool.counters + 3, 1u);
     }
 }
-// Every sample of a wave reduced per pixel in canonical (absolute sample, pixel) order.
 // The DrawTables of the draw blocks [first, first + blocks), for the hero transport [133, 133 +
 // blocks), and block 0: `tables` in all.
 RP_DEV u32 draw_block_of(u32 slot, u32 first, u32 blocks, u32 tables) {
@@ -1214,6 +1210,7 @@ __global__ void k_draw_tables(SobolTables sobol, unsigned short *prefix, uint4 *
     }
 }
 
+// Every sample of a wave reduced per pixel in canonical (absolute sample, pixel) order.
 __global__ void k_film(PathPool pool, u32 pixel_count, u32 samples, const double *cie, double weight, FilmClamp clamp,
                        FilmPixel *film) {
     for (u32 px = blockIdx.x * blockDim.x + threadIdx.x; px < pixel_count; px += gridDim.x * blockDim.x) {

@@ -8,7 +8,7 @@
 
 namespace rp {
 
-enum : u32 { kCamera = 0, kSurface = 1, kLight = 2, kEnvironment = 3 };
+enum : u32 { kSurface = 1, kEnvironment = 3 }; // vertex types
 
 // Path flags word (ident.w)
 enum : u32 {
@@ -16,8 +16,6 @@ enum : u32 {
     F_ROULETTE = 1u << 4,     // roulette enabled
     F_COMPLETE = 1u << 5,
     F_STATUS_SHIFT = 6,       // 3 bits
-    F_LTYPE_SHIFT = 9,        // latest vertex type, 2 bits
-    F_PTYPE_SHIFT = 11,       // preceding vertex type, 2 bits
     F_LDELTA = 1u << 13,      // latest vertex sampled a Dirac lobe
     F_LKIND_SHIFT = 14,       // latest BSDF family, 2 bits
     F_LMASK_SHIFT = 16,       // latest BSDF active mask, 4 bits
@@ -624,7 +622,7 @@ RP_DEV bool prepare_bsdf(const DeviceScene &s, const DMaterial &m, V4 lambda, u3
 
 // Compact record of the latest vertex for emission MIS (HeroPrevious, shaders/hero_pt_state.h:6-15).
 struct Latest {
-    u32 type, kind, mask;
+    u32 kind, mask;
     bool delta, smooth;
     V3 position, shading_normal;
     float alpha_x, alpha_y;

@@ -23,7 +23,7 @@ constexpr u32 kLeafLanes = 10; // lanes with leaves that start a triangle step
 
 // One ray's walk, advanced a node visit or a triangle test at a time.  Any: occlusion in
 // (0, h.t); else closest hit, minimising (t, primitive id) over (0, tmax).
-template <bool Any, int Stack, bool Proc> struct Walker {
+template <bool Any, int Stack> struct Walker {
     WalkRay r;
     WideRay wr;
     Hit h;       // closest: the best hit so far, t its limit; any: t = tmax, prim set once occluded
@@ -105,13 +105,13 @@ template <bool Any, int Stack, bool Proc> struct Walker {
         leaves &= ~(1u << k);
         u32 unused = 0;
         if constexpr (Any) {
-            if (any_leaf<false, Proc>(s, r, tmax, index, unused)) {
+            if (any_leaf<false, false>(s, r, tmax, index, unused)) {
                 h.prim = 0;
                 node = kNone;
                 leaves = 0;
             }
         } else {
-            closest_leaf<false, Proc>(s, r, tmax, h, index, unused);
+            closest_leaf<false, false>(s, r, tmax, h, index, unused);
         }
     }
 };
