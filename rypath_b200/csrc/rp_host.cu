@@ -969,6 +969,7 @@ struct rp_scene {
     u32 tree_levels = 0;     // most internal nodes on a root-to-leaf path of the LBVH
     u32 wide_levels = 0;     // levels of the compressed 8-wide traversal tree
     u32 family_mask = 0;     // BSDF families of the scene's materials
+    bool rough_dielectrics = false;
     bool resolve = false;    // hero scene with pass-through or mix-root instances
     bool dielectrics = false; // a dielectric material: the QMC samplers' depth limit
     bool scalar_full = false; // conductors, dielectrics or procedural primitives: the full scalar step kernel
@@ -1534,12 +1535,23 @@ void attach_draw_tables(rp_scene *s, WaveParams &p) {
 // Waves of so few lanes that whole paths (k_paths) beat the launches of their events: 512 lanes an
 // event, 2,048 in scenes of one BSDF family, whose warps do not diverge over the families' code.
 // One sample a pixel, whole paths against the wavefront, ms: Cornell box (one family, 9 events)
-// 0.59 / 1.10 at 6,144 lanes, 1.01 / 1.14 at 19,200, 1.75 / 1.17 at 49,152; the box with glass and
-// a conductor 1.19 / 1.18 at 6,144, 2.22 / 1.20 at 19,200; mixed scene (17 events) 1.40 / 3.12 at
-// 6,144, 2.07 / 3.53 at 19,200, 4.72 / 4.17 at 76,800.
+// 0.59 / 1.10 at 6,144 lanes, 1.01 / 1.14 at 19,200, 1.75 / 1.17 at 49,152; the box with smooth
+// glass and a conductor 1.19 / 1.18 at 6,144, 2.22 / 1.20 at 19,200.  In a closed scene with rough
+// dielectrics all three families shade and sample lights, which a warp runs one after another for
+// paths that nearly all go on, so whole paths pay only where few of a long path's events are left
+// to most: microfacet box at 1,024 lanes 0.73 / 0.57 with 4 events, 1.46 / 1.20 with 9, 2.33 / 2.11
+// with 16, 2.70 / 3.18 with 25 (4,096 and 4,624 lanes).
+// The number of families does not say how often rays meet them: the open mixed scene (17 events)
+// would gain beyond its bound of 8,704 too, 1.40 / 3.12 at 6,144, 2.07 / 3.53 at 19,200, 3.30 / 3.95
+// at 49,152, 4.72 / 4.17 at 76,800.
 bool whole_paths(const rp_scene *s, u32 lanes) {
-    const bool one_family = (s->family_mask & (s->family_mask - 1)) == 0;
-    return u64(lanes) <= u64(s->ds.max_depth + 1) * (one_family ? 2048u : 512u);
+    const u64 events = s->ds.max_depth + 1;
+    if ((s->family_mask & (s->family_mask - 1)) == 0)
+        return lanes <= 2048 * events;
+    const bool open = s->ds.environment != kNone || s->ds.img.env_image != kNone;
+    if (s->rough_dielectrics && !open)
+        return lanes <= std::max<u64>(64, 512 * (events - std::min<u64>(events, 16)));
+    return lanes <= 512 * events;
 }
 void launch_paths(rp_scene *s, const WaveParams &p, const PathPool &pool) {
     const unsigned grid = grid_for(s->sm_count, p.lanes, kPathBlock, 64);
@@ -2253,9 +2265,12 @@ rp_status rp_cuda_scene_create(const rp_scene_desc *d, int device, rp_scene **ou
                        uniform_knots(d, m.knot_begin, m.knot_count), uniform_knots(d, m.eta_begin, m.eta_count),
                        uniform_knots(d, m.k_begin, m.k_count)};
         }
-        for (const DMaterial &m : mats)
+        for (const DMaterial &m : mats) {
             if (m.scattering < 3)
                 s->family_mask |= 1u << m.scattering;
+            if (m.scattering == RP_DIELECTRIC && (m.u_roughness > 0 || m.v_roughness > 0))
+                s->rough_dielectrics = true;
+        }
         ds.materials = dupload(own, mats.data(), mats.size(), stm);
         ds.material_count = d->material_count;
         const u32 all_prims = next_prim + patch_prims + analytic_prims;

@@ -200,6 +200,20 @@ def test_the_form_that_a_wave_takes(kind, limit):
     rs.close()
 
 
+@pytest.mark.parametrize("depth,limit", [(3, 64), (15, 64), (19, 2048)])  # 512 lanes an event past the sixteenth, 64
+def test_closed_scenes_with_rough_dielectrics_take_the_wavefront_earlier(depth, limit):
+    rs = build(scenes.cornell_microfacets(64, 64, 1, depth, transport=abi.TRANSPORT_HERO))
+    whole = rs.sample(renderer.RenderRequest(64, 64))
+    assert whole.status == abi.RP_SUCCESS, whole.diagnostic
+    assert rs.timing().trace_launches > 0
+    for begin, count in ((0, 1), (1500, limit), (1500, limit + 1)):
+        part = rs.sample(renderer.RenderRequest(64, 64, pixel_begin=begin, pixel_count=count))
+        assert part.status == abi.RP_SUCCESS, part.diagnostic
+        assert (rs.timing().trace_launches > 0) == (count > limit)
+        assert_same(part.packet_samples, whole.packet_samples[begin:begin + count])
+    rs.close()
+
+
 @pytest.mark.parametrize("kind", ["fog", "shallow", "deep"])
 def test_scalar_lanes_in_refilled_slots(kind):
     # more lanes than the wave's slots (2,048 an SM): every lane once, as in waves that fill them once
