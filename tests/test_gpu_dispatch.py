@@ -232,3 +232,34 @@ def test_scalar_lanes_in_refilled_slots(kind):
                  for b, n in ((0, half), (half, spp - half))]
         assert whole.tobytes() == np.concatenate(parts).tobytes()
     rs.close()
+
+
+@pytest.mark.parametrize("transport", [abi.TRANSPORT_HERO, abi.TRANSPORT_SCALAR])
+@pytest.mark.parametrize("lanes", [1, 1024, 1025])  # the most whose statuses the host reads, and one more
+def test_the_first_failed_lane_is_reported(transport, lanes):
+    # a boundary limit of one crossing, and two panes in a row before part of the film
+    scene = scenes.cornell_pass_through(64, 64, 1, 8, invisible_light=False, mixes=False)
+    scene.transport = transport
+    second = scenes.identity_instance(scene.positions.shape[0], scene.triangles.shape[0], 2,
+                                      scene.instances[-1].material)
+    scene.positions = np.concatenate([scene.positions, scene.positions[-4:] + np.float32([0, 0, 0.1])])
+    scene.triangles = np.concatenate([scene.triangles, scene.triangles[-2:]])
+    scene.instances.append(second)
+    rs = build(scene)
+    sample = rs.sample if transport == abi.TRANSPORT_HERO else rs.sample_scalar
+
+    def run(begin):
+        res = sample(renderer.RenderRequest(64, 64, pixel_begin=begin, pixel_count=lanes, boundary_limit=1))
+        return res, (res.samples if transport == abi.TRANSPORT_SCALAR else res.packet_samples)["status"]
+
+    whole = sample(renderer.RenderRequest(64, 64, boundary_limit=1))
+    status = (whole.samples if transport == abi.TRANSPORT_SCALAR else whole.packet_samples)["status"]
+    first = int(np.flatnonzero(status)[0])
+    for begin in (first, max(0, first - lanes + 1), int(np.flatnonzero(status == 0)[0])):
+        res, got = run(begin)
+        np.testing.assert_array_equal(got, status[begin:begin + lanes])
+        failed = np.flatnonzero(got)
+        assert res.status == (abi.RP_FAILURE if len(failed) else abi.RP_SUCCESS)
+        if len(failed):
+            assert res.diagnostic.endswith(f"failed with status {got[failed[0]]} at lane {failed[0]}")
+    rs.close()
