@@ -337,12 +337,15 @@ typedef struct rp_film_request {
 } rp_film_request;
 enum { RP_FILM_FRESH = 1 };
 
-/* Kernel-level timing of the last call on a scene (CUDA events on the scene stream). */
+/* Kernel-level timing of the last call on a scene (CUDA events on the scene stream).  A hero wave of
+ * few lanes runs as whole paths in one kernel, walks included: it is one of the shade launches, and
+ * trace and shadow stay 0.  A counting run (rp_cuda_set_counting) never does, and times them apart.
+ * Of the scalar transport the walks and steps of a wave are one shade group. */
 typedef struct rp_timing {
     double total_ms;          /* whole call, device time */
     double trace_ms;          /* closest-hit traversal kernels */
     double shadow_ms;         /* any-hit traversal kernels */
-    double shade_ms;          /* shading kernels */
+    double shade_ms;          /* shading kernels; whole-path kernels; scalar walks and steps */
     double other_ms;          /* raygen, queue resets, film */
     uint64_t closest_rays, shadow_rays, kernel_launches, samples;
     uint64_t nodes_visited, triangles_tested; /* closest-hit rays; only when counting */
@@ -654,7 +657,8 @@ rp_status rp_cuda_trace_rays(struct rp_scene *scene, const float *rays, uint32_t
 /* Size of the library's file-scope device scratch array used by rp_cuda_sample_device_static.
  * Every GPU that loads this library holds this much device memory until the process exits. */
 #define RP_STATIC_SCRATCH_BYTES (64u << 20)
-/* Largest request, in lanes (pixel_count * sample_count), that fits that scratch. */
+/* Largest request, in lanes (pixel_count * sample_count), that the entry point takes; it fits that
+ * scratch, with some of it to spare. */
 #define RP_STATIC_MAX_LANES 118976u
 
 /* No counterpart in rypath.  Same work and results as rp_cuda_sample_device, for callers that

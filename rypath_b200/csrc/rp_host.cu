@@ -1356,7 +1356,6 @@ std::string validate_request(const rp_scene *s, const rp_request &r) {
     return {};
 }
 
-constexpr u32 kStreamLevels = 5;
 // The scalar step kernel: the plain one, or the full one for scenes with conductors,
 // dielectrics or procedural primitives.
 void launch_scalar_step(const rp_scene *s, unsigned grid, const WaveParams &p, const ScalarParams &q,
@@ -1367,11 +1366,13 @@ void launch_scalar_step(const rp_scene *s, unsigned grid, const WaveParams &p, c
         k_scalar_step<false><<<grid, kStepBlock, 0, s->stream>>>(s->ds, p, q, w, parity);
 }
 
-// Whether walks of this scene's tree stream (rp_walk.cuh): where rays visit about six nodes or
-// more, so that what the longest of 32 waits for outweighs the streaming's own bookkeeping: the
-// mixed scenes (7 to 11 nodes a ray) gain 2 to 3%; the fog box, of 38 triangles, lost 6 of 38 ms,
-// the demonstration scene, of 26, 2 of 10.  A tree deeper than any stack keeps the plain walks: a
-// query that runs out of entries has then tested the leaves of its last node, which may end it.
+// Whether the hero transport's walks of this scene's tree stream (rp_walk.cuh): where rays visit
+// about six nodes or more, so that what the longest of 32 waits for outweighs the streaming's own
+// bookkeeping: the mixed scenes (7 to 11 nodes a ray) gain 2 to 3%; scenes of some thirty triangles
+// (3 nodes a ray), tried when scalar walks could stream too, lost 6 of 38 and 2 of 10 ms.  A tree
+// deeper than any stack keeps the plain walks: a query that runs out of entries has then tested the
+// leaves of its last node, which may end it.
+constexpr u32 kStreamLevels = 5;
 bool use_stream(const rp_scene *s) { return s->wide_levels >= kStreamLevels && s->wide_levels <= u32(kStackDepth); }
 // The closest-hit and shadow kernels with the traversal stack the built tree needs, resolving
 // pass-through and mix-root hits when the scene has them.  Stream: the streaming form.
@@ -1675,8 +1676,8 @@ ScalarSlots scalar_slots(rp_scene *s, u32 count) {
 // the walk/step trips between two host reads of the wave's remaining lanes.  2,048 slots are
 // four for each thread of the step kernel (two blocks of 256 an SM) and two for each of the
 // walk (eight of 128), so a trip's passes over them are whole, and the state of the 303,104 paths
-// of 148 SMs (70 MB) stays in L2.  Fog box 512x512, 16 spp: 2^18 slots, whose last step pass is
-// half empty, 34.0 ms, 148 x 2048 32.5 ms.
+// of 148 SMs (79 MB with their queue entries) stays in L2.  Fog box 512x512, 16 spp: 2^18 slots,
+// whose last step pass is half empty, 34.0 ms, 148 x 2048 32.5 ms.
 constexpr u32 kScalarSlotsPerSm = 2048;
 constexpr int kScalarTripsPerCheck = 8;
 

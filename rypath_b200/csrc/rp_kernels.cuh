@@ -244,8 +244,8 @@ __global__ void __launch_bounds__(Block, walk_blocks(Block, Stack, Stream))
 // The warps of a block meet between two phases of a long straight run of code, so that a line of
 // instructions fetched for one serves them all: the shade kernels run some four thousand
 // instructions an event once each, and their warps, left to drift apart, spent up to 6.9 of 17
-// cycles an instruction waiting for instructions (0.9 so; the textured box 24.8 -> 13.4 ms of
-// shading, the Cornell box 14.0 -> 12.1).  Blocks of 256 serve better than of 128 or 512.
+// cycles an instruction waiting for instructions (0.9 so; of a pass, the two kernels' part 24.8 -> 13.4
+// ms in the textured box, 14.0 -> 12.1 in the Cornell box).  Blocks of 256 serve better than of 128 or 512.
 template <bool Sync> RP_DEV void phase() {
     if (Sync)
         __syncthreads();
